@@ -13,6 +13,8 @@
 namespace ppm {
 
 constexpr int kMaxSpots = 2;
+constexpr int kMuHints = 256;  // uniform cells of the mu axis with a stored bracket
+constexpr int kMaxSlots = 16;  // energies per NSX cell the home-cell kernel takes
 // doubles per fine phase k in DevProfile::fine: cos(2 pi k / n_fine), sin(2 pi k / n_fine), k / n_fine
 constexpr int kFineStride = 3;
 // per-profile counters: active (integrated rings), rings, dropped rings, points, clamped, active (dropped rings)
@@ -35,6 +37,7 @@ struct DevNsx {
   const float* data;   // [nT][ng][slice_stride] with slice [nE][nmu], values 10^logInuT3 * 2^scale_exp
   const double* mu;    // [nmu] strictly descending
   const double* mu_den;  // [nmu - 3][4] reciprocals of the cubic Lagrange denominators per stencil start
+  double mu_scale;     // kMuHints / (mu[0] - mu[nmu - 1])
   int scale_exp;       // power of two applied to the stored FP32 values
 };
 
@@ -55,6 +58,9 @@ struct DevGrid {
   const float* fEs;       // [n_e] fE in t_E order
   const int* cell_first;  // [span + 1]
   int maxe;               // most energies in one home cell
+  // smallest and largest fraction of the k-th energy of a home cell (in t_E order) over all cells, k < 16;
+  // 2 and -1 where no cell has k + 1 energies
+  float slot_lo[kMaxSlots], slot_hi[kMaxSlots];
 };
 
 struct DevSpot {
@@ -67,6 +73,7 @@ struct DevSpot {
   int kind;            // PPM_SPOT_*
   int i_lo, i_hi;      // HEALPix ring range that can hold active elements
   int T_clamped;       // logT outside the NSX axis
+  int job0;            // ring records: index of the spot's first ring job in its kernel group
   int nT_taps;         // 2 (linear logT) or 4 (cubic logT)
   int iT[4];
   double wT[4];
@@ -98,6 +105,43 @@ struct Tile {
   short u0, u1;
 };
 
+// Ring jobs of a spot (ring_kernel's CTAs): its rings inside the batch's window; a point source is one.
+__host__ __device__ __forceinline__ int ring_jobs(const DevSpot& s) { return s.i_hi >= s.i_lo ? s.i_hi - s.i_lo + 1 : 0; }
+
+// One chunk of a ring's active elements, with the ring's sweep and slice in the image of its job.
+struct RingRec {
+  int profile, spot, ring, job;
+  int n_act, list;  // active elements, their indices at lists[list]
+  int n_nodes;      // phase nodes of the profile
+  int flags;        // 1: phase_o is non-decreasing, 2: logT or log g outside the table
+};
+
+// Ring records of one kernel group: per job an image {P, F, Z, MU as in shared memory; bracket table; slice}.
+struct RingWork {
+  unsigned char* data;  // nullptr: the group runs from the planner's tiles
+  long long stride;     // bytes between images
+  int off_hidx, hidx_bytes, off_slice, slice_bytes;
+  RingRec* recs;
+  int4* ctr;              // per record: next phase node, slots that took the record, phase nodes, active elements;
+                          // behind the last one the count of records handed out
+  unsigned short* lists;  // element indices of the records, 16-byte aligned lists
+  int *n_recs, *list_next;
+  int rec_cap, list_cap, n_jobs, n_profiles, chunk;
+  // node sums of the first part_cap records, [record][node][energy in t_E order], part_stride floats a record,
+  // summed into the flux pool by sum_parts_kernel; further records add to the pool atomically
+  float* parts;
+  long long part_stride;
+  int part_cap;
+};
+
+// Adds the rounding error of old + v to *c (TwoSum).
+__device__ __forceinline__ void comp_error(double* c, double old, double v) {
+  const double s = old + v;
+  const double bb = s - old;
+  const double err = (old - (s - bb)) + (v - bb);
+  if (err != 0.0) atomicAdd(c, err);
+}
+
 // Adds v to *a with a compensated (TwoSum) accumulation: the atomic returns the
 // old value, so the rounding error of old + v is known exactly and is added to
 // the compensation pool *c.  *a + *c is then the sum of every value added, to
@@ -108,11 +152,7 @@ __device__ __forceinline__ void comp_add(double* a, double* c, double v) {
     atomicAdd(a, v);
     return;
   }
-  const double old = atomicAdd(a, v);
-  const double s = old + v;
-  const double bb = s - old;
-  const double err = (old - (s - bb)) + (v - bb);
-  if (err != 0.0) atomicAdd(c, err);
+  comp_error(c, atomicAdd(a, v), v);
 }
 
 struct WorkQueue {
@@ -202,7 +242,9 @@ __host__ __device__ __forceinline__ int hunt_from(const double* xx, int n, doubl
 // xx[i] <= x, or 0) by unit steps from any i in [0, n - 2]: a step or none
 // when i is the bracket of a nearby x.
 __host__ __device__ __forceinline__ int walk_bracket(const double* xx, int n, double x, int i) {
+#pragma unroll 1
   while (i > 0 && x < xx[i]) --i;
+#pragma unroll 1
   while (i < n - 2 && x >= xx[i + 1]) ++i;
   return i;
 }

@@ -280,6 +280,7 @@ void Engine::load_nsx(const ppm_nsx_desc& d) {
   X.data = data;
   X.mu = mu;
   X.mu_den = mu_den;
+  X.mu_scale = kMuHints / (d.mu[0] - d.mu[d.n_mu - 1]);
   X.scale_exp = scale_exp;
   nsx = X;
   nsx_mu.assign(d.mu, d.mu + d.n_mu);
@@ -346,6 +347,16 @@ void split_grid(const std::vector<double>& E, double inv_dE, GridSplit& o) {
     o.maxe = std::max(o.maxe, o.cell_first[r + 1]);
     o.cell_first[r + 1] += o.cell_first[r];
   }
+  for (int k = 0; k < kMaxSlots; ++k) {
+    o.slot_lo[k] = 2.0f;
+    o.slot_hi[k] = -1.0f;
+    for (int r = 0; r < o.span; ++r) {
+      const int at = o.cell_first[r] + k;
+      if (at >= o.cell_first[r + 1]) continue;
+      o.slot_lo[k] = std::min(o.slot_lo[k], o.fEs[at]);
+      o.slot_hi[k] = std::max(o.slot_hi[k], o.fEs[at]);
+    }
+  }
 }
 
 // Per-energy split of t_E = log10(E) (n_E - 1)/(logEkT_max - logEkT_min) for the loaded NSX axis.
@@ -368,6 +379,8 @@ void Engine::prepare_grid(int id) {
   g.span = sp.span;
   g.tE_lo = sp.lo;
   g.tE_hi = sp.hi;
+  std::copy(sp.slot_lo, sp.slot_lo + kMaxSlots, g.slot_lo);
+  std::copy(sp.slot_hi, sp.slot_hi + kMaxSlots, g.slot_hi);
   g.nsx_version = nsx_version;
 }
 
@@ -387,6 +400,8 @@ DevGrid Engine::dev_grid(int id) {
   d.fEs = g.dfEs;
   d.cell_first = g.dcell_first;
   d.maxe = g.maxe;
+  std::copy(g.slot_lo, g.slot_lo + kMaxSlots, d.slot_lo);
+  std::copy(g.slot_hi, g.slot_hi + kMaxSlots, d.slot_hi);
   return d;
 }
 
@@ -716,13 +731,82 @@ void Engine::batch_build(BatchImpl& B, int n, const ppm_params* ps, cudaStream_t
   B.chunk = chunk[0];
   long long cap[NV] = {0, 0, 0, 0, 0};
   int start[NV + 1] = {0, 0, 0, 0, 0, 0};
-  for (int k = 0; k < n; ++k) {
-    const int i = order[k];
-    const int v = vof[i];
-    cap[v] += tile_bound(ps[i], hp[k], chunk[v], npt[v]);
-    start[v + 1] = k + 1;
-  }
+  for (int k = 0; k < n; ++k) start[vof[order[k]] + 1] = k + 1;
   for (int v = 1; v <= NV; ++v) start[v] = std::max(start[v], start[v - 1]);
+  IntegrandShape shapes[NV];
+  RingWork rings[NV] = {};
+  int gb[NV] = {}, gne[NV] = {};
+  for (int v = 0; v < NV; ++v) {
+    const int g0 = start[v], g1 = start[v + 1];
+    if (g1 <= g0) continue;
+    int ne_max = 1, nf_max = 2, cells_max = 2, maxe_max = 0, bins_max = 0;
+    for (int k = g0; k < g1; ++k) {
+      ne_max = std::max(ne_max, hp[k].n_e);
+      nf_max = std::max(nf_max, hp[k].n_fine);
+      cells_max = std::max(cells_max, hp[k].grid.span + 1);
+      maxe_max = std::max(maxe_max, hp[k].grid.maxe);
+      bins_max = std::max(bins_max, hp[k].n_bins);
+    }
+    gb[v] = bins_max;
+    gne[v] = ne_max;
+    const bool cell = v == 0 || v == 4;
+    shapes[v] = choose_shape(cell || v == 3, v == 1, ne_max, nf_max, cells_max, maxe_max, bins_max, cell, gw[v].rings);
+    if (cell && !shapes[v].cellk) throw Error(PPM_E_STATE, "home-cell NSX kernel expected for the grid");
+    // a group whose nodes are split over several tiles a ring runs from ring records: each ring's sweep and slice
+    // are computed once (by ring_kernel) instead of by every tile.  A single profile of 408 rings, N_side 256:
+    // 1660 -> 1250 us a call (integrand 1410 -> 1000).  Groups with rings enough to fill the GPU keep the tiles: their rings
+    // have one tile each, and their images (60 KB a ring) would be read back from HBM.
+    if (cell && npt[v] > 0) {
+      const size_t limit = B.ring_limit ? B.ring_limit : std::min<size_t>(kRingBytesMax, (size_t)cfg.memory_budget / 8);
+      const size_t bytes = ring_work(shapes[v], hp.data(), order.data(), ps, g0, g1, chunk[v], rings[v]);
+      unsigned char* base = nullptr;
+      IntegrandShape rs = shapes[v];
+      if (bytes && rec_shape(rs, rings[v]) && B.ring_bytes + bytes <= limit) {
+        try {
+          base = (unsigned char*)B.mem.alloc(bytes);
+        } catch (const Error&) {  // no room: the tiles need none
+          cudaGetLastError();
+        }
+      }
+      if (base) {
+        B.ring_bytes += bytes;
+        RingWork& W = rings[v];
+        W.recs = (RingRec*)base;
+        W.ctr = (int4*)(W.recs + W.rec_cap);
+        W.lists = (unsigned short*)(base + ((sizeof(RingRec) + sizeof(int4)) * ((size_t)W.rec_cap + 1) + 255) / 256 * 256);
+        W.data = (unsigned char*)W.lists + (sizeof(unsigned short) * (size_t)W.list_cap + 255) / 256 * 256;
+        W.n_recs = B.d_ctrl + 3 * v;
+        W.list_next = B.d_ctrl + 3 * v + 1;
+        shapes[v] = rs;
+        // node sums for about one chunk a ring, as far as the memory goes (further chunks add atomically)
+        W.part_stride = ((long long)ne_max * gw[v].nodes_max + 63) / 64 * 64;
+        const size_t each = sizeof(float) * (size_t)W.part_stride, left = limit - B.ring_bytes;
+        size_t cls = 1 << 20;
+        while (cls < each * ((size_t)W.n_jobs + W.n_jobs / 4 + 8)) cls <<= 1;
+        while (cls > left && cls > 0) cls >>= 1;
+        W.part_cap = (int)std::min<size_t>(cls / each, (size_t)W.rec_cap);
+        if (W.part_cap > 0) {
+          try {
+            W.parts = (float*)B.mem.alloc(cls);
+            B.ring_bytes += cls;
+          } catch (const Error&) {
+            cudaGetLastError();
+            W.part_cap = 0;
+          }
+        }
+        int job = 0;
+        for (int k = g0; k < g1; ++k)
+          for (int s = 0; s < hp[k].n_spots; ++s) {
+            hp[k].spot[s].job0 = job;
+            job += ring_jobs(hp[k].spot[s]);
+          }
+      } else {
+        rings[v] = RingWork{};
+      }
+    }
+    if (!shapes[v].rec)
+      for (int k = g0; k < g1; ++k) cap[v] += tile_bound(ps[order[k]], hp[k], chunk[v], npt[v]);
+  }
   long long cap_total = 0;
   for (int v = 0; v < NV; ++v) cap_total += cap[v];
   if (cap_total > (1ll << 31) - 1) throw Error(PPM_E_RANGE, "batch too large for one work queue");
@@ -766,30 +850,22 @@ void Engine::batch_build(BatchImpl& B, int n, const ppm_params* ps, cudaStream_t
     q.next = B.d_ctrl + 3 * v + 1;
     q.overflow = B.d_ctrl + 3 * v + 2;
     base += cap[v];
-    int ne_max = 1, nf_max = 2, cells_max = 2, maxe_max = 0, bins_max = 0;
-    for (int k = g0; k < g1; ++k) {
-      ne_max = std::max(ne_max, hp[k].n_e);
-      nf_max = std::max(nf_max, hp[k].n_fine);
-      cells_max = std::max(cells_max, hp[k].grid.span + 1);
-      maxe_max = std::max(maxe_max, hp[k].grid.maxe);
-      bins_max = std::max(bins_max, hp[k].n_bins);
-    }
     G.args.profiles = B.d_prof + g0;
     G.args.lens = lens;
     G.args.nsx = nsx;
     G.args.flux = B.d_flux;
     G.args.comp = B.d_comp;
-    G.args.shape =
-        choose_shape(v == 0 || v == 3 || v == 4, v == 1, ne_max, nf_max, cells_max, maxe_max, bins_max,
-                     v == 0 || v == 4, gw[v].rings);
-    if ((v == 0 || v == 4) && !G.args.shape.cellk)
-      throw Error(PPM_E_STATE, "home-cell NSX kernel expected for the grid");
+    G.args.shape = shapes[v];
+    G.args.rings = rings[v];
+    G.bins_max = gb[v];
+    G.ne_max = gne[v];
     PPM_CUDA(configure_integrand_smem(G.args.shape));
     const int occ = max_active_ctas(G.args.shape);
     if (occ < 1)
       throw Error(PPM_E_RANGE, "integrand launch shape does not fit on an SM (" + std::to_string(G.args.shape.total) +
                                    " bytes of shared memory)");
-    G.grid = (int)std::min<long long>((long long)sm_count * occ, std::max(1ll, cap[v]));
+    G.grid = sm_count * occ;
+    if (!shapes[v].rec) G.grid = (int)std::min<long long>(G.grid, std::max(1ll, cap[v]));
     B.groups.push_back(G);
   }
   // fused point-source mode: one blackbody group, every spot a point source taking the phase-major walk,
@@ -843,14 +919,21 @@ void Engine::batch_enqueue(BatchImpl& B, cudaStream_t st, cudaEvent_t* events) {
     PPM_CUDA(cudaMemsetAsync(B.d_flux, 0, 2 * sizeof(double) * (size_t)std::max(1ll, B.flux_off[n]), st));
     PPM_CUDA(cudaMemsetAsync(B.d_stats, 0, B.small_bytes, st));
     for (const auto& G : B.groups)
-      PPM_CUDA(launch_plan(B.d_prof + G.g0, G.g1 - G.g0, lens, G.args.queue, G.chunk, G.npt, st));
+      PPM_CUDA(G.args.shape.rec ? launch_rings(G.args, st) : launch_plan(B.d_prof + G.g0, G.g1 - G.g0, lens, G.args.queue, G.chunk, G.npt, st));
   }
   if (events) PPM_CUDA(cudaEventRecord(events[1], st));
   {
     NvtxRange range("integrand");
-    for (const auto& G : B.groups) PPM_CUDA(launch_integrand(G.args, G.grid, st));
+    bool pool = false;  // a group's flux is in the pools
+    for (const auto& G : B.groups) {
+      PPM_CUDA(launch_integrand(G.args, G.grid, st));
+      if (G.args.shape.rec)
+        PPM_CUDA(launch_sum_parts(G.args, G.bins_max, G.ne_max, st));
+      else
+        pool = true;
+    }
     // the compensation pool's rounding errors back into the flux pool (a fused pass adds plainly)
-    if (!B.fused_points) PPM_CUDA(launch_add_comp(B.d_flux, B.d_comp, B.flux_off[n], sm_count, st));
+    if (!B.fused_points && pool) PPM_CUDA(launch_add_comp(B.d_flux, B.d_comp, B.flux_off[n], sm_count, st));
   }
   if (events) PPM_CUDA(cudaEventRecord(events[2], st));
   NvtxRange fold_range("fold");
@@ -878,7 +961,13 @@ void Engine::batch_launch_timed(BatchImpl& B, cudaStream_t st, float* ms) {
 
 int Engine::kernels_per_pass(const BatchImpl& B) const {
   if (B.fused_points) return 1 + (int)B.folds.size();          // the fused integrand, folds
-  return 2 * (int)B.groups.size() + 1 + (int)B.folds.size();  // plan + integrand per group, add_comp, folds
+  // per group the plan (or rings) and the integrand, and the sum of the node sums; add_comp for the others; folds
+  int n = (int)B.folds.size(), pool = 0;
+  for (const auto& G : B.groups) {
+    n += G.args.shape.rec ? 3 : 2;
+    pool |= G.args.shape.rec ? 0 : 1;
+  }
+  return n + pool;
 }
 
 void Engine::batch_capture(BatchImpl& B) {
@@ -1028,6 +1117,55 @@ void Engine::group_tiling(bool pooled, const GroupWork& w, int chunk_override, i
   *npt = splits <= 1 ? 0 : (w.nodes_max + splits - 1) / splits;
 }
 
+// Sizes of the ring records of profiles g0 .. g1 - 1 (fills W's sizes, not its pointers): the bytes of one block that
+// holds the records, their counters, the element lists and the images, 0 if there is nothing to hold or too much.
+size_t Engine::ring_work(const IntegrandShape& shape, const DevProfile* hp, const int* order, const ppm_params* ps, int g0,
+                         int g1, int chunk, RingWork& W) const {
+  long long recs = 0, list = 0, jobs = 0;
+  for (int k = g0; k < g1; ++k) {
+    recs += tile_bound(ps[order[k]], hp[k], chunk, 0);
+    for (int s = 0; s < hp[k].n_spots; ++s) {
+      const long long nj = ring_jobs(hp[k].spot[s]), per = 4ll * hp[k].n_side;
+      jobs += nj;
+      list += nj * (per + 8 * (2 + (per + chunk - 1) / chunk));
+    }
+  }
+  if (jobs <= 0 || recs > (1 << 24) || list > (1 << 30) || jobs > (1 << 24)) return 0;
+  auto up = [](size_t v) { return (v + 255) / 256 * 256; };
+  W.hidx_bytes = (int)((2 * ((size_t)shape.n_fine + 1) + 15) / 16 * 16);
+  W.off_hidx = shape.off_mu - shape.off_P;
+  W.off_slice = W.off_hidx + W.hidx_bytes;
+  const size_t rows = (size_t)((((shape.cpl + 1) * shape.ldS + 3) & ~3) + (shape.nE + shape.cpl + 1) * shape.ldS);
+  W.slice_bytes = (int)((rows * 4 + 15) / 16 * 16);
+  W.stride = (long long)up((size_t)W.off_slice + W.slice_bytes);
+  W.rec_cap = (int)recs;
+  W.list_cap = (int)list;
+  W.n_jobs = (int)jobs;
+  W.n_profiles = g1 - g0;
+  W.chunk = chunk;
+  const size_t bytes = up((sizeof(RingRec) + sizeof(int4)) * ((size_t)recs + 1)) + up(sizeof(unsigned short) * (size_t)list) +
+                       (size_t)W.stride * (size_t)jobs;
+  // whole powers of two, so that the blocks of a sampler's next proposals fit the cached ones
+  size_t cls = 1 << 20;
+  while (cls < bytes) cls <<= 1;
+  return cls;
+}
+
+// Turns a home-cell shape into the ring-record kernel's: one CTA per SM, as many chunk slots (an image and its
+// element list) as its shared memory holds.  False if not one fits.
+bool Engine::rec_shape(IntegrandShape& s, const RingWork& W) {
+  s.rec = 1;
+  s.nt = rec_threads(s.maxe_t) / (32 * s.cell_warps) * (32 * s.cell_warps);
+  s.rec_slot_bytes = (W.off_slice + W.slice_bytes + 2 * W.chunk + 31) / 16 * 16;
+  const int mu = (s.off_S - s.off_mu), batch = (s.nt * (kPairFloats / 2) * 4 + 15) / 16 * 16, room = 219 * 1024;
+  if (s.nt < 32 || room < mu + batch) return false;
+  s.rec_slots = std::min(kMaxRecSlots, (room - mu - batch) / s.rec_slot_bytes);
+  s.rec_off_mu = s.rec_slots * s.rec_slot_bytes;
+  s.rec_off_batch = s.rec_off_mu + mu;
+  s.total = s.rec_off_batch + batch;
+  return s.rec_slots >= 1;
+}
+
 // Work tiles the planner may push for one profile (its queue capacity).
 long long Engine::tile_bound(const ppm_params& p, const DevProfile& d, int chunk, int npt) const {
   const int nodes = p.n_bins * std::max(1, p.n_gl);
@@ -1078,7 +1216,7 @@ IntegrandShape Engine::choose_shape(bool nsx_kernel, bool bb_fp64, int ne_max, i
   // home-cell NSX kernel: cpl cells per lane (the last (cpl + 3) / cpl lanes of a warp
   // only supply slice rows), warp sets up to 512 threads
   const int span_max = cells_max - 1;
-  const int maxe_t = maxe_max <= 2 ? 2 : (maxe_max <= 4 ? 4 : (maxe_max <= 8 ? 8 : 16));
+  const int maxe_t = maxe_max <= 2 ? 2 : (maxe_max <= 4 ? maxe_max : (maxe_max <= 8 ? 8 : 16));
   if (allow_cell && nsx_kernel && tune.kernel == 0 && maxe_max >= 1 && maxe_max <= 16 && span_max <= 16 * 32 &&
       nsx.nmu < 4096 && bins_max < (1 << 20)) {
     // cells per lane: fewest estimated lane instructions per point (window rows,
@@ -1099,12 +1237,12 @@ IntegrandShape Engine::choose_shape(bool nsx_kernel, bool bb_fp64, int ne_max, i
     if (tune.cpl > 0) cpl = std::min(tune.cpl, cmax);
     const int cell_warps = (span_max + cells_per_warp(cpl) - 1) / cells_per_warp(cpl);
     if (best >= 0 && cell_warps <= 16) {
-      // default: about 256 threads (three CTAs of 80 registers per SM measured fastest)
-      int sets = std::min(16 / cell_warps, tune.sets > 0 ? tune.sets : std::max(1, 8 / cell_warps));
+      int sets = std::min(16 / cell_warps, tune.sets > 0 ? tune.sets : std::max(1, kCellThreads / 32 / cell_warps));
       IntegrandShape s;
       for (;;) {
         const int nt = 32 * cell_warps * sets;
-        s = make_shape(true, nt, 1, 1, tune.chunk, nf_max, lens.n_cp, lens.n_ca, nsx.nE, nsx.nmu, cells_max, true);
+        s = make_shape(true, nt, 1, 1, tune.chunk, nf_max, lens.n_cp, lens.n_ca, nsx.nE, nsx.nmu, cells_max, true,
+                       cpl);
         if (s.total <= 200 * 1024 || sets == 1) break;
         --sets;
       }

@@ -80,6 +80,7 @@ struct Grid {
   int maxe = 0;
   int iE_min = 0, span = 1;
   double tE_lo = 0, tE_hi = 0;
+  float slot_lo[kMaxSlots] = {}, slot_hi[kMaxSlots] = {};
   int nsx_version = -1;
 };
 
@@ -148,6 +149,7 @@ struct BatchImpl {
   FoldJob* d_jobs = nullptr;
   struct Group {
     int g0 = 0, g1 = 0, grid = 0;
+    int bins_max = 1, ne_max = 1;
     int chunk = 1024, npt = 0;  // candidate elements and phase nodes (0 = all) per tile
     KernelArgs args{};
   };
@@ -156,6 +158,8 @@ struct BatchImpl {
   };
   std::vector<Group> groups;
   std::vector<Fold> folds;
+  // device memory that ring records may take (0: the engine's default share) and what they took
+  size_t ring_limit = 0, ring_bytes = 0;
   size_t h2d_bytes = 0;
   // pinned host memory the build stages its uploads in, when given (serving: one area per stream slot, untouched
   // until the slot's batch has finished, so the copies run asynchronously); pageable copies otherwise
@@ -183,9 +187,11 @@ struct GridSplit {
   std::vector<float> fE, fEs;
   int iE_min = 0, span = 1, maxe = 0;
   double lo = 0, hi = 0;
+  float slot_lo[kMaxSlots] = {}, slot_hi[kMaxSlots] = {};  // DevGrid's fraction range of each slot
 };
 void split_grid(const std::vector<double>& E, double inv_dE, GridSplit& out);
 
+constexpr size_t kRingBytesMax = (size_t)1 << 30;  // most device memory of one batch's ring records and node sums
 // Work estimate of one kernel group of a batch (the tiling's inputs).
 constexpr int kMinNodesPerTile = 8;
 constexpr double kMinEvalsPerTile = 65536;  // (element, node, energy) evaluations per tile, at least
@@ -294,6 +300,9 @@ class Engine {
                               int bins_max = 0, bool allow_cell = true, double rings = 0);
   bool cell_kernel_takes(int grid);
   void group_tiling(bool pooled, const GroupWork& w, int chunk_override, int* chunk, int* npt) const;
+  size_t ring_work(const IntegrandShape& shape, const DevProfile* hp, const int* order, const ppm_params* ps, int g0,
+                   int g1, int chunk, RingWork& W) const;
+  static bool rec_shape(IntegrandShape& s, const RingWork& W);
   long long tile_bound(const ppm_params& p, const DevProfile& d, int chunk, int npt) const;
   void fold_tc_prepare(Resp& r);
   // error: word the kernel sets when a bounded wait runs out (nullptr = the engine's d_err)

@@ -71,7 +71,7 @@ __device__ __forceinline__ int block_compact(bool flag, int* scratch, int* total
 }
 
 struct SmemPtrs {
-  int* j;
+  unsigned short* j;  // active elements' indices in the ring (at most 4 N_side = 32768)
   double *P, *F, *Z, *MU, *mu;
   float* S;
   double* rows;
@@ -83,7 +83,7 @@ struct SmemPtrs {
 
 __device__ __forceinline__ SmemPtrs carve(unsigned char* sm, const IntegrandShape& S) {
   SmemPtrs s;
-  s.j = (int*)(sm + S.off_j);
+  s.j = (unsigned short*)(sm + S.off_j);
   s.P = (double*)(sm + S.off_P);
   s.F = (double*)(sm + S.off_F);
   s.Z = (double*)(sm + S.off_Z);
@@ -98,53 +98,15 @@ __device__ __forceinline__ SmemPtrs carve(unsigned char* sm, const IntegrandShap
   return s;
 }
 
-// Steps 1-4 for one tile.  Returns the number of active elements (0 = nothing to do).
-// On return (non-zero), P/F/Z/MU hold the filled fine-phase arrays and s_g the ring geometry.
-__device__ int tile_prologue(const KernelArgs& a, const DevProfile& p, const DevSpot& sp, const Tile& tile,
-                             const SmemPtrs& s, RingGeom& s_g, int* s_int, bool nsx) {
+// Stages the two lensing rows of each table and sweeps the fine phases: returns
+// whether the ring is dropped (fine sample 0 or n_fine - 1 invisible,
+// cpu/devarshi24st_cpu.cpp:195); if not, P/F/Z/MU hold the filled and wrapped
+// arrays.  s_g is visible to all threads; block barriers inside.
+__device__ __forceinline__ bool ring_sweep(const KernelArgs& a, const DevProfile& p, const SmemPtrs& s,
+                                           const RingGeom& s_g, int* s_int, bool nsx) {
   const int tid = threadIdx.x, nt = blockDim.x;
-  const bool point = sp.kind == 1;
   const DevLens& L = a.lens;
   if (tid == 0) {
-    double cos_t = point ? sp.cos_theta_pt : p.ring[3 * tile.ring];
-    double dOmega = point ? sp.dOmega_pt : p.dOmega_hp;
-    ring_geometry(p, L, cos_t, dOmega, nsx, s_g);
-  }
-  // compaction of active elements over the candidate range
-  int n_act = 0;
-  if (point) {
-    if (tid == 0) s.j[0] = 0;
-    n_act = 1;
-  } else {
-    const int N = p.n_side, ring = tile.ring;
-    const double c2 = p.ring[3 * ring + 1], s2 = p.ring[3 * ring + 2];
-    const int n_c = tile.j1 - tile.j0;
-    for (int k0 = 0; k0 < n_c; k0 += nt) {
-      int k = k0 + tid;
-      bool flag = false;
-      if (k < n_c) flag = in_spot(sp, c2, s2, healpix_phi(N, ring, tile.j0 + k));
-      int tot;
-      int pos = block_compact(flag, s_int, &tot);
-      if (flag) s.j[n_act + pos] = tile.j0 + k;
-      n_act += tot;
-      __syncthreads();
-    }
-  }
-  __syncthreads();
-  if (n_act == 0) return 0;
-  // counted by the tiles of the first node range only; a ring counts once, by the first of its tiles to
-  // find active elements.  In the fused point-source mode no planner has dropped the ring yet: the counting
-  // waits for the sweep's drop test below
-  auto count_ring = [&]() {
-    atomicAdd(&p.stats[0], (unsigned long long)n_act);
-    const unsigned bit = 1u << (tile.ring & 31);
-    if (!(atomicOr(&p.ring_seen[tile.spot * p.ring_words + (tile.ring >> 5)], bit) & bit))
-      atomicAdd(&p.stats[1], 1ull);
-    if (s_g.u_clamped && tile.first) atomicAdd(&p.stats[4], 1ull);
-  };
-  const bool fused = a.n_fused > 0;
-  if (tid == 0) {
-    if (tile.u0 == 0 && !fused) count_ring();
     s_int[40] = p.n_fine + 1;  // invisible min
     s_int[41] = -1;            // invisible max
   }
@@ -182,17 +144,7 @@ __device__ int tile_prologue(const KernelArgs& a, const DevProfile& p, const Dev
   }
   __syncthreads();
   const int inv_min = s_int[40], inv_max = s_int[41];
-  const bool dropped = inv_min == 0 || inv_max == nf - 1;  // cpu/devarshi24st_cpu.cpp:195
-  if (fused && tid == 0) {
-    if (!dropped) {
-      count_ring();
-    } else {  // the planner's count of a dropped ring (plan_kernel)
-      atomicAdd(&p.stats[1], 1ull);
-      atomicAdd(&p.stats[2], 1ull);
-      atomicAdd(&p.stats[5], (unsigned long long)n_act);
-    }
-  }
-  if (dropped) return 0;
+  if (inv_min == 0 || inv_max == nf - 1) return true;
   if (inv_min <= inv_max) {
     const int beg = inv_min - 1, end = inv_max + 1;
     const double p0 = s.P[beg], p1 = s.P[end], z0 = s.Z[beg], z1 = s.Z[end];
@@ -209,7 +161,117 @@ __device__ int tile_prologue(const KernelArgs& a, const DevProfile& p, const Dev
     s.MU[nf] = s.MU[0];
   }
   __syncthreads();
-  return n_act;
+  return false;
+}
+
+// Steps 1-4 for one tile.  Returns the number of active elements (0 = nothing to do).
+// On return (non-zero), P/F/Z/MU hold the filled fine-phase arrays and s_g the ring geometry.
+__device__ int tile_prologue(const KernelArgs& a, const DevProfile& p, const DevSpot& sp, const Tile& tile,
+                             const SmemPtrs& s, RingGeom& s_g, int* s_int, bool nsx) {
+  const int tid = threadIdx.x, nt = blockDim.x;
+  const bool point = sp.kind == 1;
+  const DevLens& L = a.lens;
+  if (tid == 0) {
+    double cos_t = point ? sp.cos_theta_pt : p.ring[3 * tile.ring];
+    double dOmega = point ? sp.dOmega_pt : p.dOmega_hp;
+    ring_geometry(p, L, cos_t, dOmega, nsx, s_g);
+  }
+  // compaction of active elements over the candidate range
+  int n_act = 0;
+  if (point) {
+    if (tid == 0) s.j[0] = 0;
+    n_act = 1;
+  } else {
+    const int N = p.n_side, ring = tile.ring;
+    const double c2 = p.ring[3 * ring + 1], s2 = p.ring[3 * ring + 2];
+    const int n_c = tile.j1 - tile.j0;
+    for (int k0 = 0; k0 < n_c; k0 += nt) {
+      int k = k0 + tid;
+      bool flag = false;
+      if (k < n_c) flag = in_spot(sp, c2, s2, healpix_phi(N, ring, tile.j0 + k));
+      int tot;
+      int pos = block_compact(flag, s_int, &tot);
+      if (flag) s.j[n_act + pos] = (unsigned short)(tile.j0 + k);
+      n_act += tot;
+      __syncthreads();
+    }
+  }
+  __syncthreads();
+  if (n_act == 0) return 0;
+  // counted by the tiles of the first node range only; a ring counts once, by the first of its tiles to
+  // find active elements.  In the fused point-source mode no planner has dropped the ring yet: the counting
+  // waits for the sweep's drop test below
+  auto count_ring = [&]() {
+    atomicAdd(&p.stats[0], (unsigned long long)n_act);
+    const unsigned bit = 1u << (tile.ring & 31);
+    if (!(atomicOr(&p.ring_seen[tile.spot * p.ring_words + (tile.ring >> 5)], bit) & bit))
+      atomicAdd(&p.stats[1], 1ull);
+    if (s_g.u_clamped && tile.first) atomicAdd(&p.stats[4], 1ull);
+  };
+  const bool fused = a.n_fused > 0;
+  if (tid == 0) {
+    if (tile.u0 == 0 && !fused) count_ring();
+  }
+  const bool dropped = ring_sweep(a, p, s, s_g, s_int, nsx);
+  if (fused && tid == 0) {
+    if (!dropped) {
+      count_ring();
+    } else {  // the planner's count of a dropped ring (plan_kernel)
+      atomicAdd(&p.stats[1], 1ull);
+      atomicAdd(&p.stats[2], 1ull);
+      atomicAdd(&p.stats[5], (unsigned long long)n_act);
+    }
+  }
+  return dropped ? 0 : n_act;
+}
+
+// Ring range of disk 1 in element index j: up to two [j_lo, j_hi] ranges
+// (with a one-element margin) that contain every active element.
+__device__ int candidate_ranges(const DevSpot& s, int N, int i, double c2, double s2, int jmax, int r[2][2]) {
+  const double A = s.s1 * s2, B = s.c1 * c2;
+  bool full = false;
+  double w = 0.0;
+  if (A < 1e-12) {
+    if (B > s.cos_ar1 - 1e-9)
+      full = true;
+    else
+      return 0;
+  } else {
+    const double qv = (s.cos_ar1 - B) / A;
+    if (qv > 1.0 + 1e-9) return 0;
+    if (qv <= -1.0)
+      full = true;
+    else
+      w = acos(fmin(qv, 1.0)) + 1e-7;
+    if (w >= kPi) full = true;
+  }
+  if (full) {
+    r[0][0] = 1;
+    r[0][1] = jmax;
+    return 1;
+  }
+  const int ii = i > 2 * N ? 4 * N - i : i;
+  const double sh = ii < N ? 0.5 : 0.5 * ((ii - N + 1) % 2);
+  const double dphi = kTwoPi / jmax;
+  const double jc = s.ph1 / dphi + sh, jw = w / dphi;
+  long long jlo = (long long)floor(jc - jw) - 1, jhi = (long long)ceil(jc + jw) + 1;
+  const long long len = jhi - jlo + 1;
+  if (len >= jmax) {
+    r[0][0] = 1;
+    r[0][1] = jmax;
+    return 1;
+  }
+  long long m = ((jlo - 1) % jmax + jmax) % jmax + 1;  // jlo mapped into [1, jmax]
+  if (m + len - 1 <= jmax) {
+    r[0][0] = (int)m;
+    r[0][1] = (int)(m + len - 1);
+    return 1;
+  }
+  r[0][0] = (int)m;
+  r[0][1] = jmax;
+  r[1][0] = 1;
+  r[1][1] = (int)(m + len - 1 - jmax);
+  return 2;
 }
 
 // Phase node u = bin * n_gl + GL point (u = bin when n_gl = 0): its bin, its
@@ -242,34 +304,6 @@ __device__ __forceinline__ double node_point(const DevProfile& p, const SmemPtrs
   if (patch < s.P[0]) patch += 1.;
   double af;
   const int i = vhunt(s.P, p.n_fine + 1, patch, af);
-  const double flux = (1 - af) * s.F[i] + af * s.F[i + 1];
-  if (flux == 0) return 0.0;
-  z = (1 - af) * s.Z[i] + af * s.Z[i + 1];
-  mu = (1 - af) * s.MU[i] + af * s.MU[i + 1];
-  return flux;
-}
-
-// node_point with the tile's bracket table hidx (hidx[k] = vhunt's bracket of
-// phase_o[0] + k / n_fine): on a non-decreasing phase_o (mono) the bracket of
-// the patch phase is walked to from its table entry, a step or none, and is
-// vhunt's bracket exactly; the fraction and the lerps are node_point's.
-__device__ __forceinline__ double node_point_tab(const DevProfile& p, const SmemPtrs& s, const RingPhi& rp, bool point,
-                                                 int jj, double ppt, bool mono, double& z, double& mu) {
-  const double phi = point ? 0.0 : rp.dphi * (s.j[jj] - rp.jofs);
-  const double phase_shift = phi / kTwoPi;
-  const double xph = ppt + phase_shift + 1.;
-  double patch = xph - floor(xph);
-  if (patch < s.P[0]) patch += 1.;
-  const int n = p.n_fine + 1;
-  double af;
-  int i;
-  if (mono) {
-    const int k = clampi((int)((patch - s.P[0]) * p.n_fine), 0, p.n_fine);
-    i = walk_bracket(s.P, n, patch, s.hidx[k]);
-    af = (patch - s.P[i]) / (s.P[i + 1] - s.P[i]);
-  } else {
-    i = vhunt(s.P, n, patch, af);
-  }
   const double flux = (1 - af) * s.F[i] + af * s.F[i + 1];
   if (flux == 0) return 0.0;
   z = (1 - af) * s.Z[i] + af * s.Z[i + 1];
@@ -662,11 +696,6 @@ __global__ void __launch_bounds__(MINB == 1 ? 512 : 320, MINB) integrand_nsx_ker
 // Lagrange stencil clamped at the table ends, cpu/nsx.hpp:187-225, written
 // as Newton differences in the cell fraction); outside the logEkT axis the
 // edge value is held (cpu/hunt.hpp:98-121 clamps the coordinate).
-__device__ __forceinline__ float slice_dot(const float* S, int ldS, int k, int imu, float4 w) {
-  const float* row = S + k * ldS + imu;
-  return fmaf(w.w, row[3], fmaf(w.z, row[2], fmaf(w.y, row[1], w.x * row[0])));
-}
-
 // Lanes of a warp that only supply slice rows to their neighbours (no home
 // cells): a lane needs rows up to C + 3 past its first, i.e. own rows of the
 // next (C + 3) / C lanes.
@@ -675,49 +704,9 @@ __host__ __device__ constexpr int halo_lanes() {
   return (C + 3) / C;
 }
 
-// Slice rows seen by one lane for one point record.  The lane owns C
-// consecutive cells starting at cell g (= G0 + first cell of the lane) and
-// needs the cubics of cells g .. g + C, i.e. rows g - 1 .. g + C + 2 of the
-// mu-contracted slice: window h[j] = row g - 1 + j, j = 0 .. C + 3.  The lane
-// contracts rows j < C itself; row j >= C is own row j mod C of lane
-// lane + j / C (the last halo_lanes<C>() lanes of the warp own no cells).
-// Sx points at slice row 0 of a slice with rows -2 .. nE + 1: rows -1 and nE
-// hold the cubic extrapolations of the first and last four rows, so that the
-// centred stencil of cell 0 (rows -1..2) and of cell nE - 2 (rows nE - 3..nE)
-// is the same cubic as the end-clamped stencil (rows 0..3, rows nE - 4..nE - 1);
-// rows -2 and nE + 1 repeat rows 0 and nE - 1, and window rows are clamped to
-// -2 .. nE + 1, so cells past either end see the end value H[0] / H[nE - 1].
-template <int C>
-__device__ __forceinline__ void lane_window(const float* Sx, int ldS, int nE, int g, int imu, float4 w,
-                                            float (&h)[C + 4]) {
-#pragma unroll
-  for (int j = 0; j < C; ++j) h[j] = slice_dot(Sx, ldS, min(max(g - 1 + j, -2), nE + 1), imu, w);
-#pragma unroll
-  for (int j = C; j < C + 4; ++j) h[j] = __shfl_down_sync(0xffffffffu, h[j % C], j / C);
-}
-
-// Cubics of the C + 1 cells whose stencils are window rows i .. i + 3 (the
-// cell between rows i + 1 and i + 2), in the cell fraction t: the Newton form
-// about row i + 1 rewritten as q0 + t (q1 + t (q2 + t q3)), from forward
-// differences shared by neighbouring cells.
-template <int C>
-__device__ __forceinline__ void window_cubics(const float (&h)[C + 4], float4 (&Q)[C + 1]) {
-  float d1[C + 3], d2[C + 2], d3[C + 1];
-#pragma unroll
-  for (int j = 0; j < C + 3; ++j) d1[j] = h[j + 1] - h[j];
-#pragma unroll
-  for (int j = 0; j < C + 2; ++j) d2[j] = d1[j + 1] - d1[j];
-#pragma unroll
-  for (int j = 0; j < C + 1; ++j) d3[j] = d2[j + 1] - d2[j];
-#pragma unroll
-  for (int i = 0; i <= C; ++i) {
-    const float c3 = d3[i] * (1.f / 6.f);
-    Q[i] = make_float4(h[i + 1], d1[i] + 0.5f * d2[i] - c3, 0.5f * d2[i], c3);
-  }
-}
-
-// Packed FP32 pairs (add / fma .f32x2, one instruction for two lanes of
-// arithmetic): two energy slots of one cell share the cubics' coefficients.
+// Packed FP32 pairs (.f32x2: one instruction for two lanes of arithmetic, each
+// rounded as the scalar instruction rounds).  The home-cell kernel packs two
+// point records: lo = record A, hi = record B.
 typedef unsigned long long f32x2;
 __device__ __forceinline__ f32x2 pk(float lo, float hi) {
   f32x2 r;
@@ -737,31 +726,656 @@ __device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
   asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
   return d;
 }
+__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) {
+  f32x2 d;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
 
+// Groups of the energy slots of a cell whose side of the carry is known together (at most `most`: pair_slots has a
+// variant for each, and a kernel whose warps run apart keeps its code small for the instruction cache).
+__host__ __device__ constexpr int slot_groups(int maxe, int most) {
+  return maxe <= most ? maxe : (maxe == 3 ? 3 : most);
+}
+
+// Cubic q.x + t (q.y + t (q.z + t q.w)) of one cell for both records of a pair.
+struct Cubic2 {
+  f32x2 x, y, z, w;
+};
+__device__ __forceinline__ f32x2 cubic_at(const Cubic2& q, f32x2 t) {
+  return fma2(fma2(fma2(q.w, t, q.z), t, q.y), t, q.x);
+}
+
+// Slice rows seen by one lane for a pair of point records.  The lane owns C
+// consecutive cells starting at cell g (= G0 + first cell of the lane) and
+// needs the cubics of cells g .. g + C, i.e. rows g - 1 .. g + C + 2 of the
+// mu-contracted slice: window h[j] = row g - 1 + j, j = 0 .. C + 3.  The lane
+// contracts rows j < C itself; row j >= C is own row j mod C of lane
+// lane + j / C (the last halo_lanes<C>() lanes of the warp own no cells).
+// ra / rb: row g - 1, column imu of each record.
+template <int C>
+__device__ __forceinline__ void pair_window(const float* ra, const float* rb, int ldS, f32x2 w0, f32x2 w1, f32x2 w2,
+                                            f32x2 w3, f32x2 (&h)[C + 4]) {
+#pragma unroll
+  for (int j = 0; j < C; ++j, ra += ldS, rb += ldS)
+    h[j] = fma2(w3, pk(ra[3], rb[3]), fma2(w2, pk(ra[2], rb[2]), fma2(w1, pk(ra[1], rb[1]), mul2(w0, pk(ra[0], rb[0])))));
+#pragma unroll
+  for (int j = C; j < C + 4; ++j) h[j] = __shfl_down_sync(0xffffffffu, h[j % C], j / C);
+}
+
+// Cubics of the C + 1 cells whose stencils are window rows i .. i + 3 (the
+// cell between rows i + 1 and i + 2), in the cell fraction t: the Newton form
+// about row i + 1 rewritten as q0 + t (q1 + t (q2 + t q3)), from forward
+// differences shared by neighbouring cells.
+template <int C>
+__device__ __forceinline__ void window_cubics(const f32x2 (&h)[C + 4], Cubic2 (&Q)[C + 1]) {
+  const f32x2 half = pk(0.5f, 0.5f), sixth = pk(1.f / 6.f, 1.f / 6.f), msixth = pk(-1.f / 6.f, -1.f / 6.f);
+  f32x2 d1[C + 3], d2[C + 2], d3[C + 1];
+#pragma unroll
+  for (int j = 0; j < C + 3; ++j) d1[j] = sub2(h[j + 1], h[j]);
+#pragma unroll
+  for (int j = 0; j < C + 2; ++j) d2[j] = sub2(d1[j + 1], d1[j]);
+#pragma unroll
+  for (int j = 0; j < C + 1; ++j) d3[j] = sub2(d2[j + 1], d2[j]);
+#pragma unroll
+  for (int i = 0; i <= C; ++i) {
+    Q[i].x = h[i + 1];
+    Q[i].z = mul2(half, d2[i]);
+    Q[i].w = mul2(d3[i], sixth);
+#ifdef PPM_YB
+    Q[i].y = fma2(d3[i], msixth, fma2(half, d2[i], d1[i]));
+#else
+    Q[i].y = sub2(fma2(half, d2[i], d1[i]), Q[i].w);
+#endif
+  }
+}
+
+// Cubics of cells lo .. lo + 2 (either record) become the constant x; cell `mid`
+// takes the x of a neighbouring cell.  ga / gb: the lane's first cell.
+template <int C>
+__device__ __forceinline__ void hold_cells(Cubic2 (&Q)[C + 1], int ga, int gb, int lo, int mid) {
+  auto hold = [](f32x2& v, bool a, bool b) {
+    float va, vb;
+    upk(v, va, vb);
+    v = pk(a ? 0.f : va, b ? 0.f : vb);
+  };
+#pragma unroll
+  for (int i = 0; i <= C; ++i) {
+    const bool a = (unsigned)(ga + i - lo) <= 2u, b = (unsigned)(gb + i - lo) <= 2u;
+    float na, nb, xa, xb;
+    upk(i < C ? Q[i + 1].x : Q[i > 0 ? i - 1 : 0].x, na, nb);
+    upk(Q[i].x, xa, xb);
+    Q[i].x = pk(ga + i == mid ? na : xa, gb + i == mid ? nb : xb);
+    hold(Q[i].y, a, b);
+    hold(Q[i].z, a, b);
+    hold(Q[i].w, a, b);
+  }
+}
+
+// Adds one pair of records to a lane's energies.  The split coordinate of an
+// energy is t = fE + fP; its cell is the home cell below 1 and the next one, at
+// t - 1, above.  KG says which case each group of slots is in, for every cell
+// and both records: groups below KG lie below 1, groups above KG at or above 1,
+// and group KG is decided slot by slot (both cubics, the result selected);
+// KG = -1 decides every slot and sets negative intensities to 0 if sg.  MG slots per group.
+template <int MAXE, int C, int MG, int KG>
+__device__ __forceinline__ void pair_slots(const Cubic2 (&Q)[C + 1], const float (&fE)[C][MAXE], float fPa, float fPb,
+                                           float ca, float cb, bool has_b, bool sg, float (&acc)[C][MAXE]) {
+  const f32x2 m1 = pk(-1.f, -1.f);
+#pragma unroll
+  for (int i = 0; i < C; ++i) {
+#pragma unroll
+    for (int k = 0; k < MAXE; ++k) {
+      const int kg = k / MG;
+      const float ta = fE[i][k] + fPa, tb = fE[i][k] + fPb;
+      const f32x2 t0 = pk(ta, tb);
+      float va, vb;
+      if (KG >= 0 && kg < KG) {
+        upk(cubic_at(Q[i], t0), va, vb);
+      } else if (KG >= 0 && kg > KG) {
+        upk(cubic_at(Q[i + 1], add2(t0, m1)), va, vb);
+      } else {
+        float a0, b0, a1, b1;
+        upk(cubic_at(Q[i], t0), a0, b0);
+        upk(cubic_at(Q[i + 1], add2(t0, m1)), a1, b1);
+        va = ta >= 1.f ? a1 : a0;
+        vb = tb >= 1.f ? b1 : b0;
+      }
+      if (KG < 0) {
+        va = sg && !(va >= 0.f) ? 0.f : va;
+        vb = sg && !(vb >= 0.f) ? 0.f : vb;
+      }
+      float s = fmaf(ca, va, acc[i][k]);
+      if (has_b) s = fmaf(cb, vb, s);
+      acc[i][k] = s;
+    }
+  }
+}
+
+// One chunk of a ring's active elements as the deposit needs it, in shared memory
+// (read at every step of 32 points: global loads there cost their latency).
+struct ChunkCtx {
+  double dphi, jofs, l10kT, tE_lo, tE_hi, out_scale;
+  long long flux_off;
+  const int *perm, *cell_first;
+  const float* fEs;
+  const double* invE;
+  unsigned long long* stats;
+  float* part;             // the chunk's node sums (stored plainly), or nullptr: added to the flux pool
+  int n_act, n_nodes, u_ofs, n_fine, n_e, span, iE_min, mode;
+  int mono, held;          // phase_o non-decreasing; logT or log g outside the table (points count as clamped)
+  int profile, spot, rec;
+  float glo[4], ghi[4];    // smallest and largest energy fraction of each slot group
+};
+
+// Fills a context (one thread); MAXE slots a cell.
+template <int MAXE, int MOST>
+__device__ __forceinline__ void fill_ctx(ChunkCtx& c, const DevProfile& p, const DevSpot& sp, int ring, int n_act, bool mono,
+                                         bool held) {
+  constexpr int NG = slot_groups(MAXE, MOST), MG = MAXE / NG;
+  const RingPhi rp = sp.kind == 1 ? RingPhi{0.0, 0.0} : healpix_ring_phi(p.n_side, ring);
+  c.dphi = rp.dphi;
+  c.jofs = rp.jofs;
+  c.l10kT = sp.l10kT;
+  c.tE_lo = p.grid.tE_lo;
+  c.tE_hi = p.grid.tE_hi;
+  c.out_scale = sp.out_scale;
+  c.flux_off = p.flux_off;
+  c.perm = p.grid.perm;
+  c.cell_first = p.grid.cell_first;
+  c.fEs = p.grid.fEs;
+  c.invE = p.grid.invE;
+  c.stats = p.stats;
+  c.part = nullptr;
+  c.n_act = n_act;
+  c.n_nodes = p.n_bins * max(p.n_gl, 1);
+  c.u_ofs = 0;
+  c.n_fine = p.n_fine;
+  c.n_e = p.n_e;
+  c.span = p.grid.span;
+  c.iE_min = p.grid.iE_min;
+  c.mode = p.interp;
+  c.mono = mono;
+  c.held = held;
+  for (int g = 0; g < NG; ++g) {
+    float lo = 2.f, hi = -1.f;
+    for (int k = g * MG; k < (g + 1) * MG; ++k) {
+      lo = fminf(lo, p.grid.slot_lo[k]);
+      hi = fmaxf(hi, p.grid.slot_hi[k]);
+    }
+    c.glo[g] = lo;
+    c.ghi[g] = hi;
+  }
+}
+
+// A chunk's tables in shared memory.  Sx: slice row 0.
+struct ChunkBufs {
+  const unsigned short* j;
+  const double *P, *F, *Z, *MU;
+  const unsigned short* hidx;
+  const float* Sx;
+};
+
+// A phase node taken by a warp set: its number, bin, phase and weight.
+struct Node {
+  int node, bin;
+  double ppt, wgl;
+};
+
+// (out of line: the deposit's code is kept small for the instruction cache)
+__device__ __noinline__ int vhunt_call(const double* xx, int n, double x, double& a) { return vhunt(xx, n, x, a); }
+
+// Active element jj of the chunk at phase ppt: patch phase, hunt and lerps in
+// FP64 (cpu/devarshi24st_cpu.cpp:220-229).  Returns flux/I (0 = skip).  hidx[k]
+// is vhunt's bracket of phase_o[0] + k / n_fine: on a non-decreasing phase_o
+// (mono) the bracket of the patch phase is walked to from its table entry, a
+// step or none, and is vhunt's bracket exactly.
+__device__ __forceinline__ double node_point_tab(const ChunkCtx& c, const ChunkBufs& b, int jj, double ppt, double& z,
+                                                 double& mu) {
+  const double phi = c.dphi * (b.j[jj] - c.jofs);
+  const double phase_shift = phi / kTwoPi;
+  // fmod(x, 1) of x = ppt + phase_shift + 1 in [1, 3): x - floor(x) is the same exact value
+  const double xph = ppt + phase_shift + 1.;
+  double patch = xph - floor(xph);
+  if (patch < b.P[0]) patch += 1.;
+  const int n = c.n_fine + 1;
+  double af;
+  int i;
+  if (c.mono) {
+    const int k = clampi((int)((patch - b.P[0]) * c.n_fine), 0, c.n_fine);
+    i = walk_bracket(b.P, n, patch, b.hidx[k]);
+    af = (patch - b.P[i]) / (b.P[i + 1] - b.P[i]);
+  } else {
+    i = vhunt_call(b.P, n, patch, af);
+  }
+  const double flux = (1 - af) * b.F[i] + af * b.F[i + 1];
+  if (flux == 0) return 0.0;
+  z = (1 - af) * b.Z[i] + af * b.Z[i + 1];
+  mu = (1 - af) * b.MU[i] + af * b.MU[i + 1];
+  return flux;
+}
+
+// vhunt's bracket on the descending mu axis (cpu/hunt.hpp:14-66), walked to from
+// the bracket stored for the value's uniform cell (kMuHints of them, behind the
+// axis and the reciprocal denominators).
+__device__ __forceinline__ int mu_bracket(const double* mu_s, int nmu, double scale, double x, double& a) {
+  const unsigned short* hint = (const unsigned short*)(mu_s + 5 * nmu);
+  int i = hint[clampi((int)((mu_s[0] - x) * scale), 0, kMuHints - 1)];
+#pragma unroll 1
+  while (i > 0 && !(x < mu_s[i])) --i;
+#pragma unroll 1
+  while (i < nmu - 2 && x < mu_s[i + 1]) ++i;
+  a = (x - mu_s[i]) / (mu_s[i + 1] - mu_s[i]);
+  return i;
+}
+
+// Loads the mu axis, its reciprocal denominators and brackets (all threads).
+__device__ __forceinline__ void load_mu(const DevNsx& X, double* mu_s) {
+  const int tid = threadIdx.x, nt = blockDim.x, nmu = X.nmu;
+  for (int k = tid; k < nmu; k += nt) mu_s[k] = X.mu[k];
+  for (int k = tid; k < 4 * (nmu - 3); k += nt) mu_s[nmu + k] = X.mu_den[k];
+  unsigned short* hint = (unsigned short*)(mu_s + 5 * nmu);
+  for (int k = tid; k < kMuHints; k += nt) {
+    double a_unused;
+    hint[k] = (unsigned short)vhunt(X.mu, nmu, X.mu[0] - k / X.mu_scale, a_unused);
+  }
+}
+
+// Where a thread stands: its warp set, its lane's first home cell, the set's record space.
+template <int C>
+struct SetPlace {
+  static constexpr int kOwners = 32 - halo_lanes<C>();  // lanes with home cells
+  int lane, warp, set, ST, st, r0;                      // ST: threads of a set, st: this thread's index in it
+  float* srec;
+  __device__ __forceinline__ SetPlace(const IntegrandShape& S, float* rec) {
+    const int tid = threadIdx.x;
+    lane = tid & 31;
+    warp = tid >> 5;
+    set = warp / S.cell_warps;
+    ST = 32 * S.cell_warps;
+    st = tid - set * ST;
+    r0 = ((warp - set * S.cell_warps) * kOwners + lane) * C;
+    srec = rec + (kPairFloats / 2) * set * ST;
+  }
+};
+
+// The lane's energy fractions: per home cell, MAXE energy slots.
+template <int MAXE, int C>
+__device__ __forceinline__ void lane_fractions(const ChunkCtx& c, const SetPlace<C>& w, float (&fE)[C][MAXE]) {
+#pragma unroll
+  for (int i = 0; i < C; ++i) {
+    const int rc = w.r0 + i;
+    const bool own = w.lane < SetPlace<C>::kOwners && rc < c.span;
+    const int e0 = own ? c.cell_first[rc] : 0;
+    const int cnt = own ? min(c.cell_first[rc + 1] - e0, MAXE) : 0;
+#pragma unroll
+    for (int k = 0; k < MAXE; ++k) fE[i][k] = k < cnt ? c.fEs[e0 + k] : 0.f;
+  }
+}
+
+// The deposit of one phase node of a chunk by one warp set.  The set walks the
+// elements jj = 0 .. n_act - 1 in order, 32 x cell_warps at a time: every
+// thread evaluates one point (FP64), the visible points are compacted in order
+// into the set's records, and every lane adds each record to its energies' FP32
+// partial sums; at the end the sums are stored or flushed with compensated FP64
+// atomics.  A node's sums thus depend on the chunk's elements and the node only,
+// not on which set or CTA takes it or what else is in the batch.  wcnt: per-warp
+// counts of a set of several warps; n_vis, n_clamped: the warp's visible and
+// clamped points are added.
+template <int MAXE, int C, int MOST>
+__device__ __forceinline__ void deposit_node(const KernelArgs& a, const ChunkCtx& c, const ChunkBufs& b, const Node& nd,
+                                             const double* mu_s, const SetPlace<C>& w, const float (&fE)[C][MAXE],
+                                             int* wcnt, unsigned& n_vis, unsigned& n_clamped) {
+  const IntegrandShape& S = a.shape;
+  const DevNsx& X = a.nsx;
+  const int nE = X.nE, nmu = X.nmu, ldS = S.ldS;
+  const int lane = w.lane, warp = w.warp, set = w.set, ST = w.ST, st = w.st, r0 = w.r0;
+  constexpr int kOwners = SetPlace<C>::kOwners;
+  // point records in pairs, kPairFloats floats each: {c}, {fP}, {w0}..{w3}, {row base}, {16 G0 + slot-group mask},
+  // {imu}, every field as (record A, record B)
+  float* srec = w.srec;
+  constexpr int NG = slot_groups(MAXE, MOST), MG = MAXE / NG;  // slot groups, slots per group
+  const float* Sx = b.Sx;
+  // the lane's first row, past a record's row base (no cell needs rows past G0 + span + 2)
+  const char* const Sl = (const char*)(Sx + min(r0, c.span + 3) * ldS);
+  const int mode = c.mode, n_act = c.n_act, n_e = c.n_e;
+  const double* den = mu_s + nmu;  // [nmu - 3][4] reciprocal Lagrange denominators
+  float acc[C][MAXE];
+#pragma unroll
+  for (int i = 0; i < C; ++i)
+#pragma unroll
+    for (int k = 0; k < MAXE; ++k) acc[i][k] = 0.f;
+#pragma unroll 1
+  for (int jb = 0; jb < n_act; jb += ST) {
+    // every thread evaluates one element at the node (FP64); the visible
+    // ones are compacted, in element order, into the set's records
+    bool vis = false, clamped = false;
+    float cw = 0.f, fP = 0.f;
+    int G0 = 0, imu = 0;
+    float w4[4] = {0.f, 0.f, 0.f, 0.f};
+    const int jj = jb + st;
+    if (jj < n_act) {
+      double z = 0, mu = 0;
+      const double flux = node_point_tab(c, b, jj, nd.ppt, z, mu);
+      if (flux != 0.0) {
+        vis = true;
+        if (mu < mu_s[nmu - 1]) mu = mu_s[nmu - 1];
+        cw = (float)(flux * nd.wgl);
+        const double tP = (log10(z) - c.l10kT - X.E_min) * X.inv_dE;
+        const double fl = floor(tP);
+        fP = (float)(tP - fl);
+        if (fP >= 1.f) fP = 0.99999994f;
+        G0 = c.iE_min + (int)fl;
+        clamped = (c.tE_lo + tP < 0.0) || (c.tE_hi + tP > (double)(nE - 1)) || c.held;
+        // mu weights (cpu/nsx.hpp:173-321)
+        double am;
+        const int im = mu_bracket(mu_s, nmu, X.mu_scale, mu, am);
+        const bool linear_mu = (mode == 4) || ((mode == 2 || mode == 3) && im >= nmu - 5);
+        int start;
+        if (linear_mu) {
+          start = min(im, nmu - 4);
+          const int o = im - start;
+#pragma unroll
+          for (int k = 0; k < 4; ++k) w4[k] = k == o ? (float)(1 - am) : (k == o + 1 ? (float)am : 0.f);
+        } else {
+          start = clampi(im - 1, 0, nmu - 4);
+          const double x0 = mu_s[start], x1 = mu_s[start + 1], x2 = mu_s[start + 2], x3 = mu_s[start + 3];
+          const double* rd = den + 4 * start;
+          w4[0] = (float)((mu - x1) * (mu - x2) * (mu - x3) * rd[0]);
+          w4[1] = (float)((mu - x0) * (mu - x2) * (mu - x3) * rd[1]);
+          w4[2] = (float)((mu - x0) * (mu - x1) * (mu - x3) * rd[2]);
+          w4[3] = (float)((mu - x0) * (mu - x1) * (mu - x2) * rd[3]);
+        }
+        imu = start;
+      }
+    }
+    const unsigned bal = __ballot_sync(0xffffffffu, vis);
+    const unsigned bal_clamped = __ballot_sync(0xffffffffu, clamped);
+    n_vis += __popc(bal);
+    n_clamped += __popc(bal_clamped);
+    int nv, slot;
+    if (S.cell_warps == 1) {
+      nv = __popc(bal);
+      slot = __popc(bal & lanemask_lt());
+    } else {
+      const int w = st >> 5;
+      if (lane == 0) wcnt[warp] = __popc(bal);
+      set_sync(set, ST);
+      int before = 0;
+      nv = 0;
+      for (int k = 0; k < S.cell_warps; ++k) {
+        const int cw = wcnt[set * S.cell_warps + k];
+        before += k < w ? cw : 0;
+        nv += cw;
+      }
+      slot = before + __popc(bal & lanemask_lt());
+    }
+    if (vis) {
+      // which slot group holds the energies whose cell is decided slot by slot: bit k is set where every
+      // slot of the groups below k lies below the carry and every slot of the groups above k past it
+      unsigned mask = 0;
+#pragma unroll
+      for (int k = 0; k < NG; ++k) {
+        bool ok = true;
+#pragma unroll
+        for (int j = 0; j < NG; ++j) ok = ok && (j == k || (j < k ? c.ghi[j] + fP < 1.f : c.glo[j] + fP >= 1.f));
+        mask |= ok ? 1u << k : 0u;
+      }
+      G0 = max(-(1 << 16), min(G0, 1 << 16));  // far past either end: the same held value
+      auto put = [&](int at, float cc) {
+        float* r = srec + (at >> 1) * kPairFloats + (at & 1);
+        r[0] = cc;
+        r[2] = fP;
+        r[4] = w4[0];
+        r[6] = w4[1];
+        r[8] = w4[2];
+        r[10] = w4[3];
+        r[12] = __int_as_float(4 * ((G0 - 1) * ldS + imu));
+        r[14] = __int_as_float(G0 * 16 + (int)mask);
+        r[16] = __int_as_float(imu);
+      };
+      put(slot, cw);
+      if (slot == nv - 1 && !(slot & 1)) put(slot + 1, 0.f);  // fills the last pair (its sums are skipped)
+    }
+    // whether a record of this step may reach past a table end (rows G0 - 1 .. G0 + span + C + 1 are read,
+    // cells G0 .. G0 + span are in use); the same for every lane: the warp's votes, or both ends for sets of
+    // several warps
+    bool step_hi = true, step_lo = true;
+    if (S.cell_warps == 1) {
+      step_hi = __any_sync(0xffffffffu, vis && G0 + c.span >= nE - (C > 1 ? C : 1));
+      step_lo = __any_sync(0xffffffffu, vis && G0 <= -1);
+    }
+    set_sync(set, ST);
+    const int nrec = __reduce_max_sync(0xffffffffu, nv);
+    const int flags = (step_hi ? 16 : 0) | (step_lo ? 32 : 0) | (mode == 4 ? 64 : 0) | (mode == 1 ? 128 : 0);
+    const int variants = mode == 1 ? 0 : 15;
+#pragma unroll 1
+    for (int q = 0; q < nrec; q += 2) {
+      const float* r = srec + (q >> 1) * kPairFloats;
+      const float4 rc = *(const float4*)r;
+      const int4 rg = *(const int4*)(r + 12);
+      const ulonglong2 w01 = *(const ulonglong2*)(r + 4), w23 = *(const ulonglong2*)(r + 8);
+      // what the pair needs, as one vote (uniform over the warp, so that the branches below need no divergence
+      // bookkeeping): bits 0..3 slot-group variants that serve both records, 4 and 5 rows past the high or low
+      // end, 6 linear in energy, 7 negative intensities become 0
+      const unsigned um = __ballot_sync(0xffffffffu, (((rg.z & rg.w & variants) | flags) >> (lane & 7)) & 1) & 255u;
+      f32x2 h[C + 4];
+      const float *ra = (const float*)(Sl + rg.x), *rb = (const float*)(Sl + rg.y);
+      if (um & 0x30u) {
+        // rows past either end repeat (C of them are stored past rows -1 and nE): the lane's first row is
+        // clamped so that all C rows exist
+        const int2 im = *(const int2*)(r + 16);
+        ra = Sx + min(max((rg.z >> 4) + r0 - 1, -1 - C), nE + 1) * ldS + im.x;
+        rb = Sx + min(max((rg.w >> 4) + r0 - 1, -1 - C), nE + 1) * ldS + im.y;
+      }
+      pair_window<C>(ra, rb, ldS, w01.x, w01.y, w23.x, w23.y, h);
+      Cubic2 Q[C + 1];
+      window_cubics<C>(h, Q);
+      if (um & 0xf0u) {
+        if (um & 0x40u) {
+#pragma unroll
+          for (int i = 0; i <= C; ++i) Q[i] = Cubic2{h[i + 1], sub2(h[i + 2], h[i + 1]), pk(0.f, 0.f), pk(0.f, 0.f)};
+        }
+        // cells past an end hold the end value.  A cell four or more rows past
+        // an end reads four equal rows, so its cubic is that constant already;
+        // the three cells next to each end become constants here.  Their value
+        // is the x of a cubic (the x of cell k is row k): of the cell itself,
+        // except for cell nE and cell -1, whose rows are the extrapolated ones;
+        // they take the x of a neighbouring cell, row nE + 1 or nE - 1 (both
+        // hold H[nE - 1]), row 0 or row -2 (H[0]).
+        if (um & 0x10u) hold_cells<C>(Q, (rg.z >> 4) + r0, (rg.w >> 4) + r0, nE - 1, nE);
+        if (um & 0x20u) hold_cells<C>(Q, (rg.z >> 4) + r0, (rg.w >> 4) + r0, -3, -1);
+      }
+      const bool has_b = q + 1 < nrec;
+      if (um & 1u)
+        pair_slots<MAXE, C, MG, 0>(Q, fE, rc.z, rc.w, rc.x, rc.y, has_b, (um & 0x80u) != 0, acc);
+      else if (um & 2u)
+        pair_slots<MAXE, C, MG, 1>(Q, fE, rc.z, rc.w, rc.x, rc.y, has_b, (um & 0x80u) != 0, acc);
+      else if (NG > 2 && (um & 4u))
+        pair_slots<MAXE, C, MG, (NG > 2 ? 2 : 0)>(Q, fE, rc.z, rc.w, rc.x, rc.y, has_b, (um & 0x80u) != 0, acc);
+      else if (NG > 3 && (um & 8u))
+        pair_slots<MAXE, C, MG, (NG > 3 ? 3 : 0)>(Q, fE, rc.z, rc.w, rc.x, rc.y, has_b, (um & 0x80u) != 0, acc);
+      else
+        pair_slots<MAXE, C, MG, -1>(Q, fE, rc.z, rc.w, rc.x, rc.y, has_b, (um & 0x80u) != 0, acc);
+    }
+    set_sync(set, ST);  // the records are rewritten by the next step
+  }
+  // the node's partial sums into the flux pool
+  const int bin = nd.bin;
+  double* flux_base = a.flux + c.flux_off;
+  double* comp_base = a.comp ? a.comp + c.flux_off : nullptr;
+  const double out_scale = c.out_scale;
+  // through the set's record space, so that consecutive threads add to consecutive energies (one 32-byte sector
+  // serves four atomics) and kFlush atomics of a thread are in flight at once
+  constexpr int kFlush = 5;
+  const int cap = (kPairFloats / 2) * ST;
+  for (int base = 0; base < n_e; base += cap) {
+#pragma unroll
+    for (int i = 0; i < C; ++i) {
+      const int rc = r0 + i;
+      const bool own = lane < kOwners && rc < c.span;
+      const int e0 = own ? c.cell_first[rc] : 0;
+      const int cnt = own ? min(c.cell_first[rc + 1] - e0, MAXE) : 0;
+#pragma unroll
+      for (int k = 0; k < MAXE; ++k)
+        if (k < cnt && (unsigned)(e0 + k - base) < (unsigned)cap) srec[e0 + k - base] = acc[i][k];
+    }
+    set_sync(set, ST);
+    const int lim = min(cap, n_e - base);
+    if (c.part) {
+      float* out = c.part + (size_t)nd.node * n_e + base;
+      for (int q = st; q < lim; q += ST) out[q] = srec[q];
+      set_sync(set, ST);
+      continue;
+    }
+    for (int q0 = st; q0 < lim; q0 += kFlush * ST) {
+      double v[kFlush], old[kFlush];
+      int o[kFlush];
+#pragma unroll
+      for (int u = 0; u < kFlush; ++u) {
+        const int q = q0 + u * ST;
+        v[u] = 0.0;
+        o[u] = -1;
+        if (q < lim && srec[q] != 0.f) {
+          const int e = c.perm[base + q];
+          o[u] = bin * n_e + e;
+          v[u] = (double)srec[q] * out_scale * c.invE[e];
+        }
+      }
+      if (comp_base) {
+#pragma unroll
+        for (int u = 0; u < kFlush; ++u)
+          if (o[u] >= 0) old[u] = atomicAdd(flux_base + o[u], v[u]);
+#pragma unroll
+        for (int u = 0; u < kFlush; ++u)
+          if (o[u] >= 0) comp_error(comp_base + o[u], old[u], v[u]);
+      } else {
+#pragma unroll
+        for (int u = 0; u < kFlush; ++u)
+          if (o[u] >= 0) atomicAdd(flux_base + o[u], v[u]);
+      }
+    }
+    set_sync(set, ST);
+  }
+}
+
+// (logT, logg) taps of the slice at one ring's gravity: weights and table offsets (one thread).
+__device__ __forceinline__ int nsx_taps(const DevNsx& X, const DevProfile& p, const DevSpot& sp, double lg, float* tapw,
+                                        int* tapo) {
+  const bool cubic = (p.interp == 0 || p.interp == 1 || p.interp == 2);
+  double ag;
+  int ig = uhunt(lg, X.g_min, X.g_max, X.ng, ag);
+  double wg[4];
+  int ig0, ngt;
+  if (cubic) {
+    ig0 = clampi(ig - 1, 0, X.ng - 4);
+    cubic_lagrange(wg, lg, uhunt_at(X.g_min, X.g_max, X.ng, ig0), uhunt_at(X.g_min, X.g_max, X.ng, ig0 + 1),
+                   uhunt_at(X.g_min, X.g_max, X.ng, ig0 + 2), uhunt_at(X.g_min, X.g_max, X.ng, ig0 + 3));
+    ngt = 4;
+  } else {
+    ig0 = ig;
+    wg[0] = 1 - ag;
+    wg[1] = ag;
+    ngt = 2;
+  }
+  int n = 0;
+  for (int jt = 0; jt < sp.nT_taps; ++jt)
+    for (int jg = 0; jg < ngt; ++jg) {
+      tapw[n] = (float)(sp.wT[jt] * wg[jg]);
+      tapo[n] = (sp.iT[jt] * X.ng + ig0 + jg) * X.slice_stride;
+      ++n;
+    }
+  return n;
+}
+
+// The home-cell kernels' slice image: rows 0..nE-1 start 16-byte aligned after
+// room for rows -1 - C .. -1; rows nE .. nE + C follow them.
+__host__ __device__ __forceinline__ int slice_row0(int ldS, int C) { return ((C + 1) * ldS + 3) & ~3; }
+
+// Reduces the NSX table into S[E][mu] (row stride ldS, Sx = row 0, in shared or
+// global memory); all threads of the block, block barriers inside.
+__device__ __forceinline__ void build_slice(const DevNsx& X, int ldS, int C, const float* tapw, const int* tapo, int ntap,
+                                            float* Sx) {
+  const int tid = threadIdx.x, nt = blockDim.x, nE = X.nE, nmu = X.nmu;
+  const int n_el = nE * nmu;
+  if (ldS == nmu) {
+    const int n4 = (n_el + 3) >> 2;
+    float4* S4 = (float4*)Sx;
+    for (int k = tid; k < n4; k += nt) {
+      float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int q = 0; q < ntap; ++q) {
+        const float4 v = __ldg((const float4*)(X.data + tapo[q]) + k);
+        const float w = tapw[q];
+        acc.x = fmaf(w, v.x, acc.x);
+        acc.y = fmaf(w, v.y, acc.y);
+        acc.z = fmaf(w, v.z, acc.z);
+        acc.w = fmaf(w, v.w, acc.w);
+      }
+      S4[k] = acc;
+    }
+  } else {
+    for (int k = tid; k < n_el; k += nt) {
+      float acc = 0.f;
+      for (int q = 0; q < ntap; ++q) acc = fmaf(tapw[q], __ldg(X.data + tapo[q] + k), acc);
+      const int row = k / nmu;
+      Sx[row * ldS + (k - row * nmu)] = acc;
+    }
+  }
+  __syncthreads();
+  // rows -1 and nE: the cubic through the first (last) four rows, one row
+  // further out; the C rows past them: copies of rows 0 and nE - 1
+  for (int k = tid; k < 2 * nmu; k += nt) {
+    const int top = k >= nmu, m = top ? k - nmu : k;
+    const float* a = Sx + (top ? (nE - 1) * ldS : 0) + m;
+    const int st = top ? -ldS : ldS;
+    Sx[(top ? nE : -1) * ldS + m] = fmaf(4.f, a[0], fmaf(-6.f, a[st], fmaf(4.f, a[2 * st], -a[3 * st])));
+    for (int j = 1; j <= C; ++j) Sx[(top ? nE + j : -1 - j) * ldS + m] = a[0];
+  }
+  __syncthreads();
+}
+
+// The bracket table of phase_o for node_point_tab (hidx in shared or global
+// memory), used where phase_o is non-decreasing: returns whether it is (a block
+// barrier).
+__device__ __forceinline__ bool phase_table(const double* P, int n_fine, unsigned short* hidx) {
+  const int tid = threadIdx.x, nt = blockDim.x;
+  bool ok = true;
+  for (int k = tid; k < n_fine; k += nt) ok &= P[k + 1] >= P[k];
+  for (int k = tid; k <= n_fine; k += nt) {
+    double a_unused;
+    hidx[k] = (unsigned short)vhunt(P, n_fine + 1, P[0] + (double)k / n_fine, a_unused);
+  }
+  return __syncthreads_and(ok) != 0;
+}
+
+// Home-cell kernel over the planner's tiles: every tile computes its ring's
+// sweep and slice itself; its phase nodes u in [u0, u1) go to the warp sets one
+// at a time through a shared counter.  For batches with rings enough to fill the
+// GPU, and for ppm_profile_noalloc.
 template <int MAXE, int C, int NTMAX, int MINB>
 __global__ void __launch_bounds__(NTMAX, MINB) integrand_nsx_cell_kernel(const KernelArgs a) {
   extern __shared__ __align__(16) unsigned char sm[];
-  const IntegrandShape& S = a.shape;
-  const SmemPtrs s = carve(sm, S);
+  const SmemPtrs s = carve(sm, a.shape);
   __shared__ RingGeom s_g;
   __shared__ int s_int[48];
   __shared__ int s_tile;
   __shared__ float s_tapw[16];
   __shared__ int s_tapo[16];
   __shared__ int s_ntap;
-  __shared__ int s_node[16], s_bin[16];          // node taken by each warp set, its bin
-  __shared__ double s_ppt[16], s_wgl[16];        // the node's phase and GL weight
-  __shared__ int s_wcnt[16];                     // visible points per warp (sets of several warps)
-  __shared__ unsigned s_nvis[16], s_nclamp[16];  // per warp: visible and clamped points of the tile
-  const int tid = threadIdx.x, nt = blockDim.x;
+  __shared__ ChunkCtx s_ctx;
+  __shared__ Node s_node[16];
+  __shared__ int s_next[16], s_wcnt[16];
+  const int tid = threadIdx.x;
   const DevNsx& X = a.nsx;
-  const int nE = X.nE, nmu = X.nmu, ldS = S.ldS;
-  const int lane = tid & 31, warp = tid >> 5;
-  const int set = warp / S.cell_warps, n_sets = (nt >> 5) / S.cell_warps;
-  constexpr int kOwners = 32 - halo_lanes<C>();        // lanes with home cells
-  const int wc = (warp - set * S.cell_warps) * kOwners * C;  // first cell of the warp
-  const int r0 = wc + C * lane;                              // first of the lane's C home cells
-  float4* rec = (float4*)s.batch;  // [nt][2]: {c, fP, imu, G0}, {mu weights}; set k uses [32 cell_warps k, ..)
+  const int ldS = a.shape.ldS;
+  float* const Sx = s.S + slice_row0(ldS, C);
+  const SetPlace<C> w(a.shape, (float*)s.batch);
+  load_mu(X, s.mu);  // (visible after the barriers of the first tile)
 
   for (;;) {
     __syncthreads();
@@ -772,321 +1386,375 @@ __global__ void __launch_bounds__(NTMAX, MINB) integrand_nsx_cell_kernel(const K
     const Tile tile = a.queue.tiles[t];
     const DevProfile& p = a.profiles[tile.profile];
     const DevSpot& sp = p.spot[tile.spot];
-    const bool point = sp.kind == 1;
     const int n_act = tile_prologue(a, p, sp, tile, s, s_g, s_int, true);
     if (n_act == 0) continue;
-    const RingPhi rp = point ? RingPhi{0.0, 0.0} : healpix_ring_phi(p.n_side, tile.ring);
-
-    // ---- (logT, logg) pre-reduction of the NSX table into S[E][mu] (row stride ldS)
     if (tid == 0) {
-      const bool cubic = (p.interp == 0 || p.interp == 1 || p.interp == 2);
-      double lg = s_g.logg, ag;
-      s_int[45] = (lg < X.g_min || lg > X.g_max) ? 1 : 0;
-      s_int[44] = 0;
       s_int[46] = tile.u0;  // next phase node of the deposit
-      int ig = uhunt(lg, X.g_min, X.g_max, X.ng, ag);
-      double wg[4];
-      int ig0, ngt;
-      if (cubic) {
-        ig0 = clampi(ig - 1, 0, X.ng - 4);
-        cubic_lagrange(wg, lg, uhunt_at(X.g_min, X.g_max, X.ng, ig0), uhunt_at(X.g_min, X.g_max, X.ng, ig0 + 1),
-                       uhunt_at(X.g_min, X.g_max, X.ng, ig0 + 2), uhunt_at(X.g_min, X.g_max, X.ng, ig0 + 3));
-        ngt = 4;
-      } else {
-        ig0 = ig;
-        wg[0] = 1 - ag;
-        wg[1] = ag;
-        ngt = 2;
-      }
-      int n = 0;
-      for (int jt = 0; jt < sp.nT_taps; ++jt)
-        for (int jg = 0; jg < ngt; ++jg) {
-          s_tapw[n] = (float)(sp.wT[jt] * wg[jg]);
-          s_tapo[n] = (sp.iT[jt] * X.ng + ig0 + jg) * X.slice_stride;
-          ++n;
-        }
-      s_ntap = n;
+      s_ntap = nsx_taps(X, p, sp, s_g.logg, s_tapw, s_tapo);
     }
-    for (int k = tid; k < nmu; k += nt) s.mu[k] = X.mu[k];
-    for (int k = tid; k < 4 * (nmu - 3); k += nt) s.mu[nmu + k] = X.mu_den[k];
-    // the tile's phase_o bracket table for node_point_tab, used where phase_o is non-decreasing
-    bool mono_ok = true;
-    {
-      const int n_fp = p.n_fine + 1;
-      for (int k = tid; k < p.n_fine; k += nt) mono_ok &= s.P[k + 1] >= s.P[k];
-      for (int k = tid; k <= p.n_fine; k += nt) {
-        double a_unused;
-        s.hidx[k] = (unsigned short)vhunt(s.P, n_fp, s.P[0] + (double)k / p.n_fine, a_unused);
-      }
-    }
-    const bool mono = __syncthreads_and(mono_ok) != 0;
-    // slice rows 0..nE-1 start 16-byte aligned after room for rows -2, -1; rows nE, nE + 1 follow them
-    float* const Sx = s.S + ((2 * ldS + 3) & ~3);
-    {
-      const int ntap = s_ntap, n_el = nE * nmu;
-      if (ldS == nmu) {
-        const int n4 = (n_el + 3) >> 2;
-        float4* S4 = (float4*)Sx;
-        for (int k = tid; k < n4; k += nt) {
-          float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-          for (int q = 0; q < ntap; ++q) {
-            const float4 v = __ldg((const float4*)(X.data + s_tapo[q]) + k);
-            const float w = s_tapw[q];
-            acc.x = fmaf(w, v.x, acc.x);
-            acc.y = fmaf(w, v.y, acc.y);
-            acc.z = fmaf(w, v.z, acc.z);
-            acc.w = fmaf(w, v.w, acc.w);
-          }
-          S4[k] = acc;
-        }
-      } else {
-        for (int k = tid; k < n_el; k += nt) {
-          float acc = 0.f;
-          for (int q = 0; q < ntap; ++q) acc = fmaf(s_tapw[q], __ldg(X.data + s_tapo[q] + k), acc);
-          const int row = k / nmu;
-          Sx[row * ldS + (k - row * nmu)] = acc;
-        }
-      }
-    }
-    __syncthreads();
-    // rows -1 and nE: the cubic through the first (last) four rows, one row
-    // further out; rows -2 and nE + 1: copies of rows 0 and nE - 1
-    for (int k = tid; k < 2 * nmu; k += nt) {
-      const int top = k >= nmu, m = top ? k - nmu : k;
-      const float* a = Sx + (top ? (nE - 1) * ldS : 0) + m;
-      const int st = top ? -ldS : ldS;
-      Sx[(top ? nE : -1) * ldS + m] = fmaf(4.f, a[0], fmaf(-6.f, a[st], fmaf(4.f, a[2 * st], -a[3 * st])));
-      Sx[(top ? nE + 1 : -2) * ldS + m] = a[0];
-    }
-    __syncthreads();
-
-    // ---- deposit.  The tile's phase nodes u in [u0, u1) (u = bin * n_gl + GL
-    // point) go to the warp sets one at a time through a shared counter.  A set
-    // walks its node's elements jj = 0 .. n_act - 1 in order, 32 x cell_warps
-    // at a time: every thread evaluates one point (FP64), the visible points are
-    // compacted in order into the set's records, and every lane adds each record
-    // to its energies' FP32 partial sums; at the end of the node the sums are
-    // flushed with compensated FP64 atomics.  A node's sums thus depend on the
-    // tile's elements and the node only, not on the tile's node range, the sets
-    // or what else is in the batch.
-    const DevGrid& G = p.grid;
-    const int n_e = G.n_e;
-    // per home cell i of the lane: MAXE energy slots in pairs (fractions, partial sums); the cells' energy
-    // ranges (cell_first) are read again at each flush, out of the record loop's registers
-    f32x2 fE2[C][MAXE / 2], acc2[C][MAXE / 2];
-#pragma unroll
-    for (int i = 0; i < C; ++i) {
-      const int rc = r0 + i;
-      const bool own = lane < kOwners && rc < G.span;
-      const int e0 = own ? G.cell_first[rc] : 0;
-      const int cnt = own ? min(G.cell_first[rc + 1] - e0, MAXE) : 0;
-#pragma unroll
-      for (int k = 0; k < MAXE / 2; ++k) {
-        fE2[i][k] = pk(2 * k < cnt ? G.fEs[e0 + 2 * k] : 0.f, 2 * k + 1 < cnt ? G.fEs[e0 + 2 * k + 1] : 0.f);
-        acc2[i][k] = pk(0.f, 0.f);
-      }
-    }
-    const int mode = p.interp;
-    const bool cubicE = mode != 4;
-    const bool sg = mode == 1;
-    const int ST = 32 * S.cell_warps;  // threads of a set
-    const int st = tid - set * ST;     // this thread's index in its set
-    const bool lane_cells = lane < kOwners && r0 < G.span;  // the lane owns cells of the grid
-    float4* srec = rec + 2 * set * ST;  // the set's records
-    if (lane == 0) {
-      s_nvis[warp] = 0;
-      s_nclamp[warp] = 0;
-    }
-
-    const double* den = s.mu + nmu;  // [nmu - 3][4] reciprocal Lagrange denominators
+    const bool mono = phase_table(s.P, p.n_fine, s.hidx);
+    if (tid == 0)
+      fill_ctx<MAXE, 4>(s_ctx, p, sp, tile.ring, n_act, mono, sp.T_clamped || s_g.logg < X.g_min || s_g.logg > X.g_max);
+    build_slice(X, ldS, C, s_tapw, s_tapo, s_ntap, Sx);
+    const ChunkBufs bufs{s.j, s.P, s.F, s.Z, s.MU, s.hidx, Sx};
+    float fE[C][MAXE];
+    lane_fractions<MAXE, C>(s_ctx, w, fE);
+    unsigned n_vis = 0, n_clamped = 0;
     for (;;) {
-      // the set's next node: its index, bin, phase and weight, published in shared memory (kept out of the
-      // registers of the record loop below)
-      if (st == 0) {
+      if (w.st == 0) {
         const int u = atomicAdd(&s_int[46], 1);
-        s_node[set] = u;
+        s_next[w.set] = u;
         if (u < tile.u1) {
-          int bin;
-          double ppt, wgl;
-          node_phase(p, u, bin, ppt, wgl);
-          s_bin[set] = bin;
-          s_ppt[set] = ppt;
-          s_wgl[set] = wgl;
+          Node& nd = s_node[w.set];
+          nd.node = u;
+          node_phase(p, u, nd.bin, nd.ppt, nd.wgl);
         }
       }
-      set_sync(set, ST);
-      if (s_node[set] >= tile.u1) break;
-      for (int jb = 0; jb < n_act; jb += ST) {
-        // every thread evaluates one element at the node (FP64); the visible
-        // ones are compacted, in element order, into the set's records
-        bool vis = false, clamped = false;
-        float c = 0.f, fP = 0.f;
-        int G0 = 0, imu = 0;
-        float w4[4] = {0.f, 0.f, 0.f, 0.f};
-        const int jj = jb + st;
-        if (jj < n_act) {
-          double z = 0, mu = 0;
-          const double flux = node_point_tab(p, s, rp, point, jj, s_ppt[set], mono, z, mu);
-          if (flux != 0.0) {
-            vis = true;
-            if (mu < s.mu[nmu - 1]) mu = s.mu[nmu - 1];
-            c = (float)(flux * s_wgl[set]);
-            const double tP = (log10(z) - sp.l10kT - X.E_min) * X.inv_dE;
-            const double fl = floor(tP);
-            fP = (float)(tP - fl);
-            if (fP >= 1.f) fP = 0.99999994f;
-            G0 = G.iE_min + (int)fl;
-            clamped = (G.tE_lo + tP < 0.0) || (G.tE_hi + tP > (double)(nE - 1)) || sp.T_clamped || s_int[45];
-            // mu weights (cpu/nsx.hpp:173-321)
-            double am;
-            const int im = vhunt(s.mu, nmu, mu, am);
-            const bool linear_mu = (mode == 4) || ((mode == 2 || mode == 3) && im >= nmu - 5);
-            int start;
-            if (linear_mu) {
-              start = min(im, nmu - 4);
-              const int o = im - start;
-#pragma unroll
-              for (int k = 0; k < 4; ++k) w4[k] = k == o ? (float)(1 - am) : (k == o + 1 ? (float)am : 0.f);
-            } else {
-              start = clampi(im - 1, 0, nmu - 4);
-              const double x0 = s.mu[start], x1 = s.mu[start + 1], x2 = s.mu[start + 2], x3 = s.mu[start + 3];
-              const double* rd = den + 4 * start;
-              w4[0] = (float)((mu - x1) * (mu - x2) * (mu - x3) * rd[0]);
-              w4[1] = (float)((mu - x0) * (mu - x2) * (mu - x3) * rd[1]);
-              w4[2] = (float)((mu - x0) * (mu - x1) * (mu - x3) * rd[2]);
-              w4[3] = (float)((mu - x0) * (mu - x1) * (mu - x2) * rd[3]);
-            }
-            imu = start;
-          }
-        }
-        const unsigned bal = __ballot_sync(0xffffffffu, vis);
-        const unsigned bal_clamped = __ballot_sync(0xffffffffu, clamped);
-        if (lane == 0) {
-          s_nvis[warp] += __popc(bal);
-          s_nclamp[warp] += __popc(bal_clamped);
-        }
-        int nv, slot;
-        if (S.cell_warps == 1) {
-          nv = __popc(bal);
-          slot = __popc(bal & lanemask_lt());
+      set_sync(w.set, w.ST);
+      if (s_next[w.set] >= tile.u1) break;
+      deposit_node<MAXE, C, 4>(a, s_ctx, bufs, s_node[w.set], s.mu, w, fE, s_wcnt, n_vis, n_clamped);
+    }
+    if (w.lane == 0) {
+      if (n_vis) atomicAdd(&p.stats[3], (unsigned long long)n_vis);
+      if (n_clamped) atomicAdd(&p.stats[4], (unsigned long long)n_clamped);
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Ring records: the home-cell path of batches with few rings (single profiles,
+// small batches), whose nodes have to be spread over many CTAs.  ring_kernel
+// does each ring's planning, sweep and slice once and leaves them in global
+// memory (L2); integrand_nsx_rec_kernel's CTAs load a ring's record and take its
+// phase nodes one at a time from the chunk's counter in global memory.
+
+// One CTA per (profile, spot, ring).
+__global__ void __launch_bounds__(256) ring_kernel(const KernelArgs a) {
+  extern __shared__ __align__(16) unsigned char sm[];
+  const IntegrandShape& S = a.shape;
+  const RingWork& W = a.rings;
+  const SmemPtrs s = carve(sm, S);
+  __shared__ RingGeom s_g;
+  __shared__ int s_int[48];
+  __shared__ int s_job[3];
+  __shared__ int s_range[2][2], s_nr;
+  __shared__ float s_tapw[16];
+  __shared__ int s_tapo[16];
+  __shared__ int s_ntap;
+  const int tid = threadIdx.x, nt = blockDim.x;
+  const int job = blockIdx.x;
+  if (job == 0 && tid == 0) W.ctr[W.rec_cap] = make_int4(0, 0, 0, 0);
+  for (int t = tid; t < W.n_profiles * kMaxSpots; t += nt) {
+    const DevProfile& q = a.profiles[t / kMaxSpots];
+    const int si = t % kMaxSpots;
+    if (si >= q.n_spots) continue;
+    const int at = job - q.spot[si].job0, n = ring_jobs(q.spot[si]);
+    if (at >= 0 && at < n) {
+      s_job[0] = t / kMaxSpots;
+      s_job[1] = si;
+      s_job[2] = q.spot[si].kind == 1 ? 0 : q.spot[si].i_lo + at;
+    }
+  }
+  __syncthreads();
+  const DevProfile& p = a.profiles[s_job[0]];
+  const DevSpot& sp = p.spot[s_job[1]];
+  const int ring = s_job[2];
+  const bool point = sp.kind == 1;
+  const DevLens& L = a.lens;
+  const double z = point ? sp.cos_theta_pt : p.ring[3 * ring];
+  const double c2 = point ? 0.0 : p.ring[3 * ring + 1], s2 = point ? 0.0 : p.ring[3 * ring + 2];
+  if (tid == 0) {
+    ring_geometry(p, L, z, point ? sp.dOmega_pt : p.dOmega_hp, true, s_g);
+    s_ntap = nsx_taps(a.nsx, p, sp, s_g.logg, s_tapw, s_tapo);
+  }
+  if (tid == 32) {
+    int r[2][2] = {{0, 0}, {0, 0}};
+    s_nr = point ? 1 : candidate_ranges(sp, p.n_side, ring, c2, s2, healpix_jmax(p.n_side, ring), r);
+    for (int k = 0; k < 2; ++k) {
+      s_range[k][0] = r[k][0];
+      s_range[k][1] = r[k][1];
+    }
+  }
+  __syncthreads();
+  const int nr = s_nr;
+  if (nr == 0) return;
+  const bool dropped = ring_sweep(a, p, s, s_g, s_int, true);
+  if (dropped) {  // counted, with its elements, only if it holds active elements (as plan_kernel)
+    int na = 0;
+    if (point) {
+      na = tid == 0 ? 1 : 0;
+    } else {
+      for (int k = 0; k < nr; ++k)
+        for (int j = s_range[k][0] + tid; j <= s_range[k][1]; j += nt)
+          na += in_spot(sp, c2, s2, healpix_phi(p.n_side, ring, j)) ? 1 : 0;
+    }
+    na = __reduce_add_sync(0xffffffffu, na);
+    if (tid == 0) s_int[42] = 0;
+    __syncthreads();
+    if ((tid & 31) == 0 && na) atomicAdd(&s_int[42], na);
+    __syncthreads();
+    if (tid == 0 && s_int[42]) {
+      atomicAdd(&p.stats[1], 1ull);
+      atomicAdd(&p.stats[2], 1ull);
+      atomicAdd(&p.stats[5], (unsigned long long)s_int[42]);
+      if (s_g.u_clamped && !point) atomicAdd(&p.stats[4], 1ull);
+    }
+    return;
+  }
+  // the ring's image: the sweep as it lies in shared memory, the bracket table, the slice
+  unsigned char* const img = W.data + (size_t)job * W.stride;
+  const bool mono = phase_table(s.P, p.n_fine, (unsigned short*)(img + W.off_hidx));
+  // active elements, one record per chunk of candidates
+  int n_ring = 0;
+  bool first = true;
+  for (int k = 0; k < nr; ++k) {
+    const int j_end = point ? 1 : s_range[k][1] + 1;
+    for (int j0 = point ? 0 : s_range[k][0]; j0 < j_end; j0 += W.chunk, first = false) {
+      const int n_c = min(W.chunk, j_end - j0);
+      int n_act = 0;
+      for (int k0 = 0; k0 < n_c; k0 += nt) {
+        const int c = k0 + tid;
+        const bool flag = c < n_c && (point || in_spot(sp, c2, s2, healpix_phi(p.n_side, ring, j0 + c)));
+        int tot;
+        const int pos = block_compact(flag, s_int, &tot);
+        if (flag) s.j[n_act + pos] = (unsigned short)(j0 + c);
+        n_act += tot;
+        __syncthreads();
+      }
+      if (n_act == 0) continue;
+      n_ring += n_act;
+      if (tid == 0) {
+        const int at = atomicAdd(W.n_recs, 1), lo = atomicAdd(W.list_next, (n_act + 7) & ~7);
+        s_int[43] = lo;
+        const bool held = sp.T_clamped || s_g.logg < a.nsx.g_min || s_g.logg > a.nsx.g_max;
+        if (at < W.rec_cap && lo + n_act <= W.list_cap) {
+          W.recs[at] = RingRec{s_job[0], s_job[1], ring, job, n_act, lo, p.n_bins * max(p.n_gl, 1),
+                               (mono ? 1 : 0) | (held ? 2 : 0)};
+          W.ctr[at] = make_int4(0, 0, p.n_bins * max(p.n_gl, 1), n_act);
         } else {
-          const int w = st >> 5;
-          if (lane == 0) s_wcnt[warp] = __popc(bal);
-          set_sync(set, ST);
-          int before = 0;
-          nv = 0;
-          for (int k = 0; k < S.cell_warps; ++k) {
-            const int cw = s_wcnt[set * S.cell_warps + k];
-            before += k < w ? cw : 0;
-            nv += cw;
-          }
-          slot = before + __popc(bal & lanemask_lt());
+          s_int[43] = -1;
+          atomicOr(a.queue.overflow, 1);
         }
-        if (vis) {
-          srec[2 * slot] = make_float4(c, fP, __int_as_float(imu), __int_as_float(G0));
-          srec[2 * slot + 1] = make_float4(w4[0], w4[1], w4[2], w4[3]);
-        }
-        // whether a record of this step may use a cell next to the high or the low end of the table (cells
-        // G0 .. G0 + span are in use); the same for every lane: the warp's votes, or both ends for sets of
-        // several warps
-        bool step_hi = true, step_lo = true;
-        if (S.cell_warps == 1) {
-          step_hi = __any_sync(0xffffffffu, vis && G0 + G.span >= nE - 1 && G0 <= nE + 1);
-          step_lo = __any_sync(0xffffffffu, vis && G0 <= -1 && G0 + G.span >= -3);
-        }
-        set_sync(set, ST);
-        for (int b = 0; b < nv; ++b) {
-          const float4 rA = srec[2 * b], wA = srec[2 * b + 1];
-          const int g = __float_as_int(rA.w) + r0;  // first home cell of the lane for this point
-          float h[C + 4];
-          lane_window<C>(Sx, ldS, nE, g, __float_as_int(rA.z), wA, h);
-          float4 Q[C + 1];
-          if (cubicE) {
-            window_cubics<C>(h, Q);
-          } else {
-#pragma unroll
-            for (int i = 0; i <= C; ++i) Q[i] = make_float4(h[i + 1], h[i + 2] - h[i + 1], 0.f, 0.f);
-          }
-          // cells past an end hold the end value.  A cell four or more rows past
-          // an end reads four equal clamped rows, so its cubic is that constant
-          // already; the three cells next to each end become constants here.
-          // Their value is the x of a cubic (the x of cell k is row k): of the
-          // cell itself, except for cell nE and cell -1, whose rows are the
-          // extrapolated ones; they take the x of a neighbouring cell, row
-          // nE + 1 or nE - 1 (both hold H[nE - 1]), row 0 or row -2 (H[0]).
-          if (step_hi && __any_sync(0xffffffffu, lane_cells && g + C >= nE - 1 && g <= nE + 1)) {
-#pragma unroll
-            for (int i = 0; i <= C; ++i) {
-              const int gi = g + i;
-              const float nb = i < C ? Q[i + 1].x : Q[i > 0 ? i - 1 : 0].x;
-              if ((unsigned)(gi - (nE - 1)) <= 2u) Q[i] = make_float4(gi == nE ? nb : Q[i].x, 0.f, 0.f, 0.f);
+        if (s_g.u_clamped && first) atomicAdd(&p.stats[4], 1ull);
+      }
+      __syncthreads();
+      const int lo = s_int[43];
+      if (lo >= 0)
+        for (int c = tid; c < n_act; c += nt) W.lists[lo + c] = s.j[c];
+      __syncthreads();
+    }
+  }
+  if (n_ring == 0) return;
+  if (tid == 0) {
+    atomicAdd(&p.stats[0], (unsigned long long)n_ring);
+    atomicAdd(&p.stats[1], 1ull);
+  }
+  const int n16 = (S.off_mu - S.off_P) >> 4;
+  for (int k = tid; k < n16; k += nt) ((float4*)img)[k] = ((const float4*)(sm + S.off_P))[k];
+  build_slice(a.nsx, S.ldS, S.cpl, s_tapw, s_tapo, s_ntap, (float*)(img + W.off_slice) + slice_row0(S.ldS, S.cpl));
+}
+
+// 16-byte asynchronous copy from global to shared memory.
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+
+// State of a chunk slot: the warp sets inside it (low bits) and its flags.
+constexpr unsigned kSlotDrain = 1u << 16;    // its chunk has no nodes left to take
+constexpr unsigned kSlotLoading = 1u << 17;  // one set is loading its next chunk
+constexpr unsigned kSlotDead = 1u << 18;     // no chunk left to load
+
+// One CTA per SM with up to four chunk slots: the warp sets take nodes from any
+// loaded chunk; the last set to leave a drained slot loads its next chunk (the
+// one with the most work left per slot on it) while the others go on with the
+// other slots, so that nobody waits for a chunk's slowest node.
+template <int MAXE, int C, int NTMAX>
+__global__ void __launch_bounds__(NTMAX, 1) integrand_nsx_rec_kernel(const KernelArgs a) {
+  extern __shared__ __align__(16) unsigned char sm[];
+  const IntegrandShape& S = a.shape;
+  const RingWork& W = a.rings;
+  constexpr int kSets = NTMAX / 32;
+  __shared__ ChunkCtx s_ctx[kMaxRecSlots];
+  __shared__ unsigned s_word[kMaxRecSlots];
+  __shared__ Node s_node[kSets];
+  __shared__ int s_got[kSets], s_wcnt[kSets];
+  __shared__ unsigned long long s_best[kSets];
+  const int tid = threadIdx.x, nt = blockDim.x;
+  const DevNsx& X = a.nsx;
+  const int n_recs = min(*W.n_recs, W.rec_cap);
+  if (n_recs == 0) return;
+  const int NS = S.rec_slots;
+  double* const mu_s = (double*)(sm + S.rec_off_mu);
+  load_mu(X, mu_s);
+  if (tid < NS) {
+    s_word[tid] = kSlotDrain;
+    s_ctx[tid].rec = -1;
+  }
+  __syncthreads();
+  const SetPlace<C> w(S, (float*)(sm + S.rec_off_batch));
+  const int per_slot = max(1, nt / w.ST / NS);  // warp sets per slot
+  const int a16 = (S.off_F - S.off_P) / 8;      // doubles between the sweep's arrays
+  volatile unsigned* const word = s_word;
+
+  // leader of a set: leaves slot sl; true if the set has become the loader of the drained slot
+  auto leave = [&](int sl) {
+    return atomicSub(&s_word[sl], 1u) == (kSlotDrain | 1u) && atomicCAS(&s_word[sl], kSlotDrain, kSlotLoading) == kSlotDrain;
+  };
+  constexpr int kExit = -1;  // s_got: a slot to work in, kExit, or -2 - slot to load
+  float fE[C][MAXE];
+  unsigned n_vis = 0, n_clamped = 0;
+  int cur_rec = -1, cur_slot = -1, profile = -1;
+  bool claimed = false;  // (leader) the slot just left is this set's to load
+  for (;;) {
+    if (w.st == 0) {
+      int got = kExit;
+      if (claimed) {
+        got = -2 - cur_slot;
+        claimed = false;
+      } else {
+        // bounded: a set that finds nothing for a second leaves, the others finish the work
+        for (int spin = 0; spin < (1 << 21); ++spin) {
+          bool live = false;
+          for (int k = 0; k < NS && got == kExit; ++k) {
+            const int sl = (max(cur_slot, w.set % NS) + k) % NS;
+            const unsigned v = word[sl];
+            if (v & kSlotDead) continue;
+            live = true;
+            if (v == kSlotDrain) {
+              if (atomicCAS(&s_word[sl], kSlotDrain, kSlotLoading) == kSlotDrain) got = -2 - sl;
+              continue;
             }
-          }
-          if (step_lo && __any_sync(0xffffffffu, lane_cells && g <= -1 && g + C >= -3)) {
-#pragma unroll
-            for (int i = 0; i <= C; ++i) {
-              const int gi = g + i;
-              const float nb = i < C ? Q[i + 1].x : Q[i > 0 ? i - 1 : 0].x;
-              if ((unsigned)(gi + 3) <= 2u) Q[i] = make_float4(gi == -1 ? nb : Q[i].x, 0.f, 0.f, 0.f);
-            }
-          }
-          const f32x2 cw2 = pk(rA.x, rA.x), fP2 = pk(rA.y, rA.y), m1 = pk(-1.f, -1.f);
-#pragma unroll
-          for (int i = 0; i < C; ++i) {
-            const f32x2 ax = pk(Q[i].x, Q[i].x), ay = pk(Q[i].y, Q[i].y), az = pk(Q[i].z, Q[i].z), aw = pk(Q[i].w, Q[i].w);
-            const f32x2 bx = pk(Q[i + 1].x, Q[i + 1].x), by = pk(Q[i + 1].y, Q[i + 1].y), bz = pk(Q[i + 1].z, Q[i + 1].z),
-                        bw = pk(Q[i + 1].w, Q[i + 1].w);
-#pragma unroll
-            for (int k = 0; k < MAXE / 2; ++k) {
-              // split coordinate t = fE + fP: cell i below 1, cell i + 1 at t - 1
-              // above; both cubics are evaluated and the result selected
-              const f32x2 t0 = add2(fE2[i][k], fP2), t1 = add2(t0, m1);
-              const f32x2 v0 = fma2(fma2(fma2(aw, t0, az), t0, ay), t0, ax);
-              const f32x2 v1 = fma2(fma2(fma2(bw, t1, bz), t1, by), t1, bx);
-              float ta, tb, a0, b0, a1, b1;
-              upk(t0, ta, tb);
-              upk(v0, a0, b0);
-              upk(v1, a1, b1);
-              float va = ta >= 1.f ? a1 : a0, vb = tb >= 1.f ? b1 : b0;
-              if (sg) {
-                va = fmaxf(va, 0.f);
-                vb = fmaxf(vb, 0.f);
+            if (v & (kSlotDrain | kSlotLoading)) continue;
+            if (!(atomicAdd(&s_word[sl], 1u) & (kSlotDrain | kSlotLoading | kSlotDead))) {
+              __threadfence_block();
+              const ChunkCtx& c = s_ctx[sl];
+              const int u = atomicAdd(&W.ctr[c.rec].x, 1);
+              if (u < c.n_nodes) {
+                const int v2 = u + c.u_ofs < c.n_nodes ? u + c.u_ofs : u + c.u_ofs - c.n_nodes;
+                Node& nd = s_node[w.set];
+                nd.node = v2;
+                node_phase(a.profiles[c.profile], v2, nd.bin, nd.ppt, nd.wgl);
+                got = sl;
+                continue;
               }
-              acc2[i][k] = fma2(cw2, pk(va, vb), acc2[i][k]);
+              atomicOr(&s_word[sl], kSlotDrain);
             }
+            if (leave(sl)) got = -2 - sl;
           }
-        }
-        set_sync(set, ST);  // the records are rewritten by the next step
-      }
-      // the node's partial sums into the flux pool
-      const int bin = s_bin[set];
-      double* flux_base = a.flux + p.flux_off;
-      double* comp_base = a.comp ? a.comp + p.flux_off : nullptr;
-      const double out_scale = sp.out_scale;
-#pragma unroll
-      for (int i = 0; i < C; ++i) {
-        const int rc = r0 + i;
-        const bool own = lane < kOwners && rc < G.span;
-        const int e0 = own ? G.cell_first[rc] : 0;
-        const int cnt = own ? min(G.cell_first[rc + 1] - e0, MAXE) : 0;
-#pragma unroll
-        for (int k = 0; k < MAXE; ++k) {
-          float lo, hi;
-          upk(acc2[i][k / 2], lo, hi);
-          const float v = (k & 1) ? hi : lo;
-          if (k < cnt && v != 0.f) {
-            const int e = G.perm[e0 + k];
-            const size_t o = (size_t)bin * n_e + e;
-            comp_add(flux_base + o, comp_base ? comp_base + o : nullptr, (double)v * out_scale * G.invE[e]);
-          }
-          if (k & 1) acc2[i][k / 2] = pk(0.f, 0.f);
+          if (got != kExit || !live) break;
+          __nanosleep(500);
         }
       }
+      s_got[w.set] = got;
     }
-    if (lane == 0) {
-      if (s_nvis[warp]) atomicAdd(&p.stats[3], (unsigned long long)s_nvis[warp]);
-      if (s_nclamp[warp]) atomicAdd(&p.stats[4], (unsigned long long)s_nclamp[warp]);
+    set_sync(w.set, w.ST);
+    const int got = s_got[w.set];
+    if (got == kExit) break;
+    if (got < kExit) {
+      const int sl = -2 - got;
+      int r = -1;
+      for (;;) {
+        if (s_ctx[sl].rec < 0) {  // the slot's first chunk
+          r = (int)((blockIdx.x + (unsigned)sl * gridDim.x) % (unsigned)n_recs);
+          if (w.st == 0) atomicAdd(&W.ctr[r].y, 1);
+          set_sync(w.set, w.ST);
+          break;
+        }
+        // chunks that nobody has yet, in order
+        if (w.st == 0) {
+          s_best[w.set] = 0;
+          const int nx = NS * (int)gridDim.x < n_recs ? NS * (int)gridDim.x + atomicAdd(&W.ctr[W.rec_cap].x, 1) : n_recs;
+          s_got[w.set] = nx < n_recs ? nx : -1;
+          if (nx < n_recs) atomicAdd(&W.ctr[nx].y, 1);
+        }
+        set_sync(w.set, w.ST);
+        r = s_got[w.set];
+        if (r >= 0) break;
+        // then the one with the most work left per slot on it
+        unsigned long long best = 0;
+#pragma unroll 4
+        for (int q = w.st; q < n_recs; q += w.ST) {
+          const int4 t = __ldcg(W.ctr + q);
+          const int left = t.z - t.x;
+          // (scattered a little, so that slots that look at the same time choose differently)
+          const float jitter = 0.5f + (float)(((unsigned)q * 2654435761u + blockIdx.x * 40503u) >> 24) * (1.f / 512.f);
+          const float score = (float)left * (float)t.w / (float)(t.y + 1) * jitter;
+          const unsigned long long key = ((unsigned long long)__float_as_uint(score) << 32) | (unsigned)q;
+          // a chunk whose slots' sets will take the remaining nodes at once is left to them
+          best = left > per_slot * t.y / 2 && key > best ? key : best;
+        }
+        if (best) atomicMax(&s_best[w.set], best);
+        set_sync(w.set, w.ST);
+        if (s_best[w.set] == 0) break;
+        r = (int)(unsigned)s_best[w.set];
+        if (w.st == 0) {
+          const int y = atomicAdd(&W.ctr[r].y, 1);
+          s_got[w.set] = W.recs[r].n_nodes - __ldcg(&W.ctr[r].x) > per_slot * y / 2 ? 1 : 0;
+        }
+        set_sync(w.set, w.ST);
+        const bool ok = s_got[w.set] != 0;
+        set_sync(w.set, w.ST);
+        if (ok) break;
+        r = -1;
+      }
+      if (r < 0) {
+        if (w.st == 0) atomicXor(&s_word[sl], kSlotLoading | kSlotDead);
+        continue;
+      }
+      const RingRec q = W.recs[r];
+      unsigned char* const dst = sm + (size_t)sl * S.rec_slot_bytes;
+      const unsigned char* const img = W.data + (size_t)q.job * W.stride;
+      const int n16 = (W.off_slice + W.slice_bytes) >> 4;
+      for (int k = w.st; k < n16; k += w.ST) cp_async16(dst + 16 * k, img + 16 * k);
+      for (int k = w.st; k < ((q.n_act + 7) >> 3); k += w.ST)
+        cp_async16(dst + 16 * (n16 + k), W.lists + q.list + 8 * k);
+      if (w.st == 0) {
+        const DevProfile& p = a.profiles[q.profile];
+        ChunkCtx& c = s_ctx[sl];
+        fill_ctx<MAXE, 2>(c, p, p.spot[q.spot], q.ring, q.n_act, (q.flags & 1) != 0, (q.flags & 2) != 0);
+        c.u_ofs = (int)((unsigned)q.job * 40503u % (unsigned)q.n_nodes);
+        c.part = r < W.part_cap ? W.parts + (size_t)r * W.part_stride : nullptr;
+        c.profile = q.profile;
+        c.spot = q.spot;
+        c.rec = r;
+      }
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      __threadfence_block();
+      set_sync(w.set, w.ST);
+      if (w.st == 0) {
+        __threadfence_block();
+        atomicAnd(&s_word[sl], ~kSlotLoading);
+      }
+      continue;
     }
+    // a node of the chunk in slot `got`
+    __threadfence_block();
+    cur_slot = got;
+    const ChunkCtx& c = s_ctx[got];
+    if (c.rec != cur_rec) {
+      cur_rec = c.rec;
+      if (w.lane == 0 && profile >= 0 && profile != c.profile) {
+        if (n_vis) atomicAdd(&a.profiles[profile].stats[3], (unsigned long long)n_vis);
+        if (n_clamped) atomicAdd(&a.profiles[profile].stats[4], (unsigned long long)n_clamped);
+        n_vis = n_clamped = 0;
+      }
+      profile = c.profile;
+      lane_fractions<MAXE, C>(c, w, fE);
+    }
+    const unsigned char* const base = sm + (size_t)got * S.rec_slot_bytes;
+    const double* P = (const double*)base;
+    const ChunkBufs bufs{(const unsigned short*)(base + W.off_slice + W.slice_bytes), P, P + a16, P + 2 * a16, P + 3 * a16,
+                         (const unsigned short*)(base + W.off_hidx),
+                         (const float*)(base + W.off_slice) + slice_row0(S.ldS, C)};
+    deposit_node<MAXE, C, 2>(a, c, bufs, s_node[w.set], mu_s, w, fE, s_wcnt, n_vis, n_clamped);
+    __threadfence_block();
+    set_sync(w.set, w.ST);
+    if (w.st == 0) claimed = leave(got);
+  }
+  if (w.lane == 0 && profile >= 0) {
+    if (n_vis) atomicAdd(&a.profiles[profile].stats[3], (unsigned long long)n_vis);
+    if (n_clamped) atomicAdd(&a.profiles[profile].stats[4], (unsigned long long)n_clamped);
   }
 }
 
@@ -1468,55 +2136,6 @@ __global__ void __launch_bounds__(512, 2) integrand_bb_kernel(const KernelArgs a
 }
 
 // ---------------------------------------------------------------------------
-// Ring range of disk 1 in element index j: up to two [j_lo, j_hi] ranges
-// (with a one-element margin) that contain every active element.
-__device__ int candidate_ranges(const DevSpot& s, int N, int i, double c2, double s2, int jmax, int r[2][2]) {
-  const double A = s.s1 * s2, B = s.c1 * c2;
-  bool full = false;
-  double w = 0.0;
-  if (A < 1e-12) {
-    if (B > s.cos_ar1 - 1e-9)
-      full = true;
-    else
-      return 0;
-  } else {
-    const double qv = (s.cos_ar1 - B) / A;
-    if (qv > 1.0 + 1e-9) return 0;
-    if (qv <= -1.0)
-      full = true;
-    else
-      w = acos(fmin(qv, 1.0)) + 1e-7;
-    if (w >= kPi) full = true;
-  }
-  if (full) {
-    r[0][0] = 1;
-    r[0][1] = jmax;
-    return 1;
-  }
-  const int ii = i > 2 * N ? 4 * N - i : i;
-  const double sh = ii < N ? 0.5 : 0.5 * ((ii - N + 1) % 2);
-  const double dphi = kTwoPi / jmax;
-  const double jc = s.ph1 / dphi + sh, jw = w / dphi;
-  long long jlo = (long long)floor(jc - jw) - 1, jhi = (long long)ceil(jc + jw) + 1;
-  const long long len = jhi - jlo + 1;
-  if (len >= jmax) {
-    r[0][0] = 1;
-    r[0][1] = jmax;
-    return 1;
-  }
-  long long m = ((jlo - 1) % jmax + jmax) % jmax + 1;  // jlo mapped into [1, jmax]
-  if (m + len - 1 <= jmax) {
-    r[0][0] = (int)m;
-    r[0][1] = (int)(m + len - 1);
-    return 1;
-  }
-  r[0][0] = (int)m;
-  r[0][1] = jmax;
-  r[1][0] = 1;
-  r[1][1] = (int)(m + len - 1 - jmax);
-  return 2;
-}
-
 // Whether the ring is skipped because fine sample 0 or n_fine-1 is invisible
 // (cpu/devarshi24st_cpu.cpp:195), evaluated with the sweep's own arithmetic.
 __device__ bool ring_dropped(const DevProfile& p, const DevLens& L, const RingGeom& g, bool nsx) {
@@ -1641,7 +2260,7 @@ __global__ void fold_simt_kernel(const FoldJob* jobs, const double* rsp, int n_c
 
 // ---------------------------------------------------------------------------
 IntegrandShape make_shape(bool nsx, int nt, int ne_t, int pb, int max_cand, int n_fine, int n_cp, int n_ca, int nE,
-                          int nmu, int cells, bool cellk) {
+                          int nmu, int cells, bool cellk, int cpl) {
   IntegrandShape s{};
   s.nsx = nsx;
   s.cellk = (nsx && cellk) ? 1 : 0;
@@ -1658,7 +2277,7 @@ IntegrandShape make_shape(bool nsx, int nt, int ne_t, int pb, int max_cand, int 
   auto al = [](long v) { return (int)((v + 15) / 16 * 16); };
   int off = 0;
   s.off_j = off;
-  off += al((long)max_cand * 4);
+  off += al((long)max_cand * 2);
   const long nf1 = n_fine + 1;
   s.off_P = off;
   off += al(nf1 * 8);
@@ -1669,24 +2288,25 @@ IntegrandShape make_shape(bool nsx, int nt, int ne_t, int pb, int max_cand, int 
   s.off_MU = off;
   off += al(nf1 * 8);
   s.off_mu = off;
-  off += nsx ? al((long)nmu * 8 * 5) : 0;
+  off += nsx ? al((long)nmu * 8 * 5 + (s.cellk ? 2 * kMuHints : 0)) : 0;
   s.off_S = off;
   const int rows = al((long)(4 * n_cp + 2 * n_ca) * 8);
   if (s.cellk) {
     // home-cell kernel: odd row stride; the lensing rows (used only by the
-    // sweep, before the slice is built) share the slice's space; 32-byte point records
+    // sweep, before the slice is built) share the slice's space; 80 bytes per pair of point records
     s.ldS = nmu | 1;
-    // rows -2 .. nE + 1, row 0 16-byte aligned
-    const int slice = al(((long)((2 * s.ldS + 3) & ~3) + (long)(nE + 2) * s.ldS) * 4);
+    // rows -1 - cpl .. nE + cpl, row 0 16-byte aligned
+    const int slice = al(((long)(((cpl + 1) * s.ldS + 3) & ~3) + (long)(nE + cpl + 1) * s.ldS) * 4);
     s.off_rows = off;
     off += slice > rows ? slice : rows;
     s.off_union = off;
     s.off_batch = off;
     s.off_Q = off;
-    off += al((long)nt * 32);
+    off += al((long)nt * (kPairFloats / 2) * 4);
     s.off_hidx = off;
     off += al((long)nf1 * 2);
     s.total = off;
+    s.ring_bytes = s.off_rows + rows;
     return s;
   }
   s.ldS = nmu;
@@ -1705,25 +2325,22 @@ IntegrandShape make_shape(bool nsx, int nt, int ne_t, int pb, int max_cand, int 
 }
 
 namespace {
+// home-cell kernels: (energy slots per cell, cells per lane) as compiled, two register budgets each: two CTAs per
+// SM (96 registers, nothing of the record loop spilled) up to kCellThreads threads, one up to 512
+#define PPM_CELL_SHAPES(X) X(2, 1) X(2, 2) X(2, 3) X(3, 1) X(3, 2) X(3, 3) X(4, 1) X(4, 2) X(4, 3) X(8, 1) X(8, 2) X(16, 1)
+
 void* kernel_for(const IntegrandShape& s, int precision) {
   if (s.nsx && s.cellk) {
-    // register budget: two CTAs per SM (80 registers) up to 384 threads, else one
-    const bool two = s.minb >= 2 && s.nt <= 384;
-    if (s.maxe_t == 2) {
-      if (s.cpl >= 3) return two ? (void*)integrand_nsx_cell_kernel<2, 3, 384, 2> : (void*)integrand_nsx_cell_kernel<2, 3, 512, 1>;
-      if (s.cpl == 2) return two ? (void*)integrand_nsx_cell_kernel<2, 2, 384, 2> : (void*)integrand_nsx_cell_kernel<2, 2, 512, 1>;
-      return two ? (void*)integrand_nsx_cell_kernel<2, 1, 384, 2> : (void*)integrand_nsx_cell_kernel<2, 1, 512, 1>;
-    }
-    if (s.maxe_t == 4) {
-      if (s.cpl >= 3) return two ? (void*)integrand_nsx_cell_kernel<4, 3, 384, 2> : (void*)integrand_nsx_cell_kernel<4, 3, 512, 1>;
-      if (s.cpl == 2) return two ? (void*)integrand_nsx_cell_kernel<4, 2, 384, 2> : (void*)integrand_nsx_cell_kernel<4, 2, 512, 1>;
-      return two ? (void*)integrand_nsx_cell_kernel<4, 1, 384, 2> : (void*)integrand_nsx_cell_kernel<4, 1, 512, 1>;
-    }
-    if (s.maxe_t == 8) {
-      if (s.cpl >= 2) return two ? (void*)integrand_nsx_cell_kernel<8, 2, 384, 2> : (void*)integrand_nsx_cell_kernel<8, 2, 512, 1>;
-      return two ? (void*)integrand_nsx_cell_kernel<8, 1, 384, 2> : (void*)integrand_nsx_cell_kernel<8, 1, 512, 1>;
-    }
-    return (void*)integrand_nsx_cell_kernel<16, 1, 512, 1>;
+    const bool two = s.minb >= 2 && s.nt <= kCellThreads;
+#define PPM_CELL(E, C)                                                                                            \
+  if (s.maxe_t == E && s.cpl == C) {                                                                              \
+    if (s.rec)                                                                                                    \
+      return (void*)integrand_nsx_rec_kernel<E, C, rec_threads(E)>;                                               \
+    return two ? (void*)integrand_nsx_cell_kernel<E, C, kCellThreads, 2> : (void*)integrand_nsx_cell_kernel<E, C, 512, 1>; \
+  }
+    PPM_CELL_SHAPES(PPM_CELL)
+#undef PPM_CELL
+    return nullptr;
   }
   if (s.nsx) {
     const bool two = s.minb >= 2;
@@ -1769,20 +2386,16 @@ cudaError_t once_per_device(int slot, cudaError_t (*set_up)()) {
 namespace {
 // every integrand variant gets the largest dynamic shared-memory allowance of the current device
 cudaError_t set_integrand_smem() {
-  void* fns[] = {(void*)integrand_nsx_cell_kernel<2, 1, 512, 1>, (void*)integrand_nsx_cell_kernel<2, 1, 384, 2>,
-                 (void*)integrand_nsx_cell_kernel<2, 2, 512, 1>, (void*)integrand_nsx_cell_kernel<2, 2, 384, 2>,
-                 (void*)integrand_nsx_cell_kernel<2, 3, 512, 1>, (void*)integrand_nsx_cell_kernel<2, 3, 384, 2>,
-                 (void*)integrand_nsx_cell_kernel<4, 1, 512, 1>, (void*)integrand_nsx_cell_kernel<4, 1, 384, 2>,
-                 (void*)integrand_nsx_cell_kernel<4, 2, 512, 1>, (void*)integrand_nsx_cell_kernel<4, 2, 384, 2>,
-                 (void*)integrand_nsx_cell_kernel<4, 3, 512, 1>, (void*)integrand_nsx_cell_kernel<4, 3, 384, 2>,
-                 (void*)integrand_nsx_cell_kernel<8, 1, 512, 1>, (void*)integrand_nsx_cell_kernel<8, 1, 384, 2>,
-                 (void*)integrand_nsx_cell_kernel<8, 2, 512, 1>, (void*)integrand_nsx_cell_kernel<8, 2, 384, 2>,
-                 (void*)integrand_nsx_cell_kernel<16, 1, 512, 1>,
+#define PPM_CELL(E, C)                                                                            \
+  (void*)integrand_nsx_cell_kernel<E, C, 512, 1>, (void*)integrand_nsx_cell_kernel<E, C, kCellThreads, 2>, \
+      (void*)integrand_nsx_rec_kernel<E, C, rec_threads(E)>,
+  void* fns[] = {PPM_CELL_SHAPES(PPM_CELL)(void*) ring_kernel,
                  (void*)integrand_nsx_kernel<1, 1>, (void*)integrand_nsx_kernel<1, 2>,
                  (void*)integrand_nsx_kernel<2, 1>, (void*)integrand_nsx_kernel<2, 2>, (void*)integrand_nsx_kernel<4, 1>,
                  (void*)integrand_bb_kernel<double, 1>, (void*)integrand_bb_kernel<double, 2>,
                  (void*)integrand_bb_kernel<double, 4>, (void*)integrand_bb_kernel<float, 1>,
                  (void*)integrand_bb_kernel<float, 2>, (void*)integrand_bb_kernel<float, 4>};
+#undef PPM_CELL
   int dev = 0, optin = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
@@ -1830,6 +2443,79 @@ cudaError_t launch_add_comp(double* flux, const double* comp, long long n, int s
   if (n <= 0) return cudaSuccess;
   const long long blocks = std::min<long long>((n + 255) / 256, (long long)sm_count * 8);
   add_comp_kernel<<<(unsigned)blocks, 256, 0, st>>>(flux, comp, n);
+  return cudaGetLastError();
+}
+
+namespace {
+constexpr int kSumQ = 128, kSumSegs = 8, kSumRecs = 1024;
+
+__device__ __forceinline__ void dd_add(double& s, double& c, double x) {
+  // (intrinsics: x is a product, which must not be contracted into the sum)
+  const double t = __dadd_rn(s, x), bb = __dsub_rn(t, s);
+  c = __dadd_rn(c, __dadd_rn(__dsub_rn(s, __dsub_rn(t, bb)), __dsub_rn(x, bb)));
+  s = t;
+}
+
+// The flux of one (profile, bin) from its chunks' node sums: grid (bins, energy tiles of kSumQ, profiles), kSumSegs
+// threads an energy, each over every kSumSegs-th chunk.  Double-double sums: the exact sum to about 1e-32, in any
+// order of the records, as the pool's compensated atomics give it; what the atomics added is included.  Bound by the
+// read of the node sums (4 bytes per node and energy, from L2 for a single profile).
+__global__ void __launch_bounds__(kSumQ * kSumSegs) sum_parts_kernel(const KernelArgs a) {
+  const RingWork& W = a.rings;
+  const DevProfile& p = a.profiles[blockIdx.z];
+  const int bin = blockIdx.x, n_e = p.n_e;
+  const int ql = threadIdx.x % kSumQ, seg = threadIdx.x / kSumQ, q = blockIdx.y * kSumQ + ql;
+  if (bin >= p.n_bins || blockIdx.y * kSumQ >= n_e) return;
+  __shared__ int s_rec[kSumRecs], s_n;
+  __shared__ double s_s[kSumSegs][kSumQ], s_c[kSumSegs][kSumQ];
+  const int n_recs = min(*W.n_recs, min(W.rec_cap, W.part_cap));
+  const int e = q < n_e ? p.grid.perm[q] : 0;
+  const double invE = q < n_e ? p.grid.invE[e] : 0.0;
+  const int n_gl = max(p.n_gl, 1);
+  double s = 0.0, c = 0.0;
+  for (int r0 = 0; r0 < n_recs; r0 += kSumRecs) {
+    __syncthreads();
+    if (threadIdx.x == 0) s_n = 0;
+    __syncthreads();
+    const int r = r0 + (int)threadIdx.x;
+    if (r < n_recs && W.recs[r].profile == (int)blockIdx.z) s_rec[atomicAdd(&s_n, 1)] = r | W.recs[r].spot << 30;
+    __syncthreads();
+    const int n = s_n;
+    if (q < n_e)
+      for (int g = 0; g < n_gl; ++g) {
+        const float* src = W.parts + ((size_t)bin * n_gl + g) * n_e + q;
+#pragma unroll 4
+        for (int k = seg; k < n; k += kSumSegs) {
+          const float v = __ldcg(src + (size_t)(s_rec[k] & 0x3fffffff) * W.part_stride);
+          dd_add(s, c, __dmul_rn(__dmul_rn((double)v, p.spot[s_rec[k] >> 30].out_scale), invE));
+        }
+      }
+  }
+  s_s[seg][ql] = s;
+  s_c[seg][ql] = c;
+  __syncthreads();
+  if (seg == 0 && q < n_e) {
+    for (int k = 1; k < kSumSegs; ++k) {
+      dd_add(s, c, s_s[k][ql]);
+      c += s_c[k][ql];
+    }
+    const size_t o = (size_t)p.flux_off + (size_t)bin * n_e + e;
+    dd_add(s, c, a.flux[o]);
+    c += a.comp[o];
+    a.comp[o] = 0.0;
+    a.flux[o] = s + c;
+  }
+}
+}  // namespace
+
+cudaError_t launch_sum_parts(const KernelArgs& a, int bins_max, int ne_max, cudaStream_t st) {
+  sum_parts_kernel<<<dim3(bins_max, (ne_max + kSumQ - 1) / kSumQ, a.rings.n_profiles), kSumQ * kSumSegs, 0, st>>>(a);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_rings(const KernelArgs& a, cudaStream_t st) {
+  if (a.rings.n_jobs <= 0) return cudaSuccess;
+  ring_kernel<<<a.rings.n_jobs, 256, a.shape.ring_bytes, st>>>(a);
   return cudaGetLastError();
 }
 

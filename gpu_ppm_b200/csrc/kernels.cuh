@@ -29,17 +29,31 @@ struct IntegrandShape {
   int ldS;        // floats between the slice rows in shared memory (odd: conflict-free column reads)
   // offsets in bytes
   int off_j, off_P, off_F, off_Z, off_MU, off_mu, off_S, off_union, off_rows, off_batch, off_Q, total;
+  int rec;        // home-cell kernel: 1 = from ring records (integrand_nsx_rec_kernel)
+  // its chunk slots per CTA, their bytes and the offsets behind them
+  int rec_slots, rec_slot_bytes, rec_off_mu, rec_off_batch;
+  int ring_bytes; // dynamic shared memory of ring_kernel
   int off_hidx;   // home-cell kernel: the tile's phase_o bracket table ([n_fine + 1] uint16), 0 elsewhere
 };
 
 IntegrandShape make_shape(bool nsx, int nt, int ne_t, int pb, int max_cand, int n_fine, int n_cp, int n_ca, int nE,
-                          int nmu, int cells, bool cellk = false);
+                          int nmu, int cells, bool cellk = false, int cpl = 1);
+
+constexpr int kMaxRecSlots = 4;
+// Home-cell kernel over tiles: two CTAs of this many threads per SM.  The record loop is bound by the FMA pipe and the
+// register file's ports, not by the number of warps: 96 profiles of the batching prior took 64.4 ms with 24 warps per SM
+// at 80 registers, 59.5 ms with 20 at 96, 65.2 ms with 16 at 128.
+constexpr int kCellThreads = 320;
+constexpr int kPairFloats = 20;  // home-cell kernels: floats per pair of point records (80 bytes: 2-way bank conflicts)
+// threads of integrand_nsx_rec_kernel's CTA, one per SM: 80 registers a thread, 128 where a cell has many slots
+__host__ __device__ constexpr int rec_threads(int maxe_t) { return maxe_t <= 4 ? 640 : 512; }
 
 struct KernelArgs {
   const DevProfile* profiles;
   DevLens lens;
   DevNsx nsx;
   WorkQueue queue;
+  RingWork rings;
   double* flux;  // pool
   double* comp;  // compensation pool of the flux pool's atomic additions (nullptr: plain additions)
   IntegrandShape shape;
@@ -53,6 +67,10 @@ cudaError_t launch_plan(const DevProfile* profiles, int n_profiles, const DevLen
                         int nodes_per_tile, cudaStream_t st);
 // flux[i] += comp[i], i < n
 cudaError_t launch_add_comp(double* flux, const double* comp, long long n, int sm_count, cudaStream_t st);
+// ring records of a group (a.rings): plan, sweep and slice of every ring
+cudaError_t launch_rings(const KernelArgs& a, cudaStream_t st);
+// the group's flux from the records' node sums and the pools (whose compensation it clears)
+cudaError_t launch_sum_parts(const KernelArgs& a, int bins_max, int ne_max, cudaStream_t st);
 cudaError_t launch_integrand(const KernelArgs& a, int grid, cudaStream_t st);
 // counts[c][b] = alpha * sum_E rsp[c][E] * flux[b][E] for each listed profile, FP64 or FP32 SIMT
 struct FoldJob {

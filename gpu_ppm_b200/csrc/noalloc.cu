@@ -73,12 +73,12 @@ ScratchHead scratch_head() {
   off += up256(sizeof(DevProfile));
   h.stats = off;
   off += up256(sizeof(unsigned long long) * kStats);
+  // one 256-byte block: 16 queue control words, 4 status words, the fold job
+  static_assert(sizeof(int) * 16 <= 64 && sizeof(int) * 4 <= 64 && sizeof(FoldJob) <= 128, "words overlap");
   h.ctrl = off;
-  off += up256(sizeof(int) * 16);
-  h.status = off;
-  off += up256(sizeof(int) * 4);
-  h.job = off;
-  off += up256(sizeof(FoldJob));
+  h.status = off + 64;
+  h.job = off + 128;
+  off += 256;
   h.end = off;
   return h;
 }
@@ -155,6 +155,8 @@ void Engine::profile_noalloc(const ppm_params& p, double* flux_d, double* counts
     g.tE_lo = split.lo;
     g.tE_hi = split.hi;
     g.maxe = split.maxe;
+    std::copy(split.slot_lo, split.slot_lo + kMaxSlots, g.slot_lo);
+    std::copy(split.slot_hi, split.slot_hi + kMaxSlots, g.slot_hi);
   } else {
     split.rE.assign(n_e, 0);
     split.fE.assign(n_e, 0.0f);

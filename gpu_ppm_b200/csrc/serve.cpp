@@ -87,6 +87,7 @@ struct Server {
     HostBuffer stage;                  // device-to-host staging of this batch, from the pool
     int slot = 0;
     size_t bytes = 0;
+    size_t ring_limit = 1;             // spare budget that the batch's ring records may take
     std::atomic<bool> finished{false};
     Server* server = nullptr;
     int* ctrl = nullptr;                 // pinned copy of the queue control words
@@ -318,6 +319,7 @@ struct Server {
       f->slot = free_slot;
       f->bytes = bytes;
       f->reqs = std::move(take_reqs);
+      f->ring_limit = std::max<size_t>(1, std::min<size_t>(kRingBytesMax, (budget - in_use) / 2));
       f->trace.t_admit = since_start_us(Clock::now());
       f->trace.n_requests = (int32_t)f->reqs.size();
       f->trace.stream_slot = free_slot;
@@ -341,6 +343,8 @@ struct Server {
         fail(f->reqs, err);
         continue;
       }
+      f->bytes += f->B->ring_bytes;  // in flight with the batch, returned with it (retire)
+      in_use += f->B->ring_bytes;
       inflight.push_back(std::move(f));
     }
   }
@@ -353,6 +357,7 @@ struct Server {
     f.B.reset(new BatchImpl());
     BatchImpl& B = *f.B;
     B.mem.stream = slot.stream;
+    B.ring_limit = f.ring_limit;
     B.h_upload = slot.upload.ptr;
     B.h_upload_cap = slot.upload.cap;
     {
