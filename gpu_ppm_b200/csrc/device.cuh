@@ -124,12 +124,14 @@ struct RingWork {
   RingRec* recs;
   int4* ctr;              // per record: next phase node, slots that took the record, phase nodes, active elements;
                           // behind the last one the count of records handed out
-  unsigned short* lists;  // element indices of the records, 16-byte aligned lists
+  unsigned char* lists;   // the records' elements, 16-byte aligned lists: indices in the ring (uint16, NSX) or phase
+                          // shifts phi / 2 pi (double, blackbody)
+  int elem_bytes;
   int *n_recs, *list_next;
   int rec_cap, list_cap, n_jobs, n_profiles, chunk;
   // node sums of the first part_cap records, [record][node][energy in t_E order], part_stride floats a record,
   // summed into the flux pool by sum_parts_kernel; further records add to the pool atomically
-  float* parts;
+  void* parts;           // float (NSX) or double (blackbody); part_stride in units of 4 bytes
   long long part_stride;
   int part_cap;
 };

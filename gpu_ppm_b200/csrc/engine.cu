@@ -733,6 +733,15 @@ void Engine::batch_build(BatchImpl& B, int n, const ppm_params* ps, cudaStream_t
   int start[NV + 1] = {0, 0, 0, 0, 0, 0};
   for (int k = 0; k < n; ++k) start[vof[order[k]] + 1] = k + 1;
   for (int v = 1; v <= NV; ++v) start[v] = std::max(start[v], start[v - 1]);
+  // every spot a point source taking the phase-major walk, at most two flux additions per (bin, energy): the fused
+  // point-source mode below
+  bool points_only = true;
+  for (int i = 0; i < n && points_only; ++i) {
+    const ppm_params& q = ps[i];
+    bool points = vof[i] == vof[0] && (vof[i] == 1 || vof[i] == 2) && q.n_spots >= 1;
+    for (int k = 0; k < q.n_spots; ++k) points &= q.spots[k].kind == PPM_SPOT_POINT;
+    points_only = points && (long long)grids[q.energy_grid].E.size() <= 4 && q.n_spots * std::max(1, q.n_gl) <= 2;
+  }
   IntegrandShape shapes[NV];
   RingWork rings[NV] = {};
   int gb[NV] = {}, gne[NV] = {};
@@ -756,7 +765,13 @@ void Engine::batch_build(BatchImpl& B, int n, const ppm_params* ps, cudaStream_t
     // are computed once (by ring_kernel) instead of by every tile.  A single profile of 408 rings, N_side 256:
     // 1660 -> 1250 us a call (integrand 1410 -> 1000).  Groups with rings enough to fill the GPU keep the tiles: their rings
     // have one tile each, and their images (60 KB a ring) would be read back from HBM.
-    if (cell && npt[v] > 0) {
+    // Blackbody groups run from ring records too.  Light curves (few energies) do so between about 200 and 592 rings
+    // on 148 SMs only: the tiles' phase-major walk evaluates a point in fewer instructions, and loses where its rings
+    // come to little more than a round of its CTAs (one energy: 302 rings 234 -> 184 us a call, 474 rings 367 -> 231;
+    // 190 rings would take 149 -> 183 us, 683 rings 335 -> 410).
+    const bool bb_rec = (v == 1 || v == 2) && !points_only &&
+                        (ne_max > 4 || (gw[v].rings > 1.35 * sm_count && gw[v].rings < 4ll * sm_count));
+    if ((cell && npt[v] > 0) || bb_rec) {
       const size_t limit = B.ring_limit ? B.ring_limit : std::min<size_t>(kRingBytesMax, (size_t)cfg.memory_budget / 8);
       const size_t bytes = ring_work(shapes[v], hp.data(), order.data(), ps, g0, g1, chunk[v], rings[v]);
       unsigned char* base = nullptr;
@@ -773,21 +788,22 @@ void Engine::batch_build(BatchImpl& B, int n, const ppm_params* ps, cudaStream_t
         RingWork& W = rings[v];
         W.recs = (RingRec*)base;
         W.ctr = (int4*)(W.recs + W.rec_cap);
-        W.lists = (unsigned short*)(base + ((sizeof(RingRec) + sizeof(int4)) * ((size_t)W.rec_cap + 1) + 255) / 256 * 256);
-        W.data = (unsigned char*)W.lists + (sizeof(unsigned short) * (size_t)W.list_cap + 255) / 256 * 256;
+        W.lists = (unsigned char*)(base + ((sizeof(RingRec) + sizeof(int4)) * ((size_t)W.rec_cap + 1) + 255) / 256 * 256);
+        W.data = W.lists + ((size_t)W.elem_bytes * (size_t)W.list_cap + 255) / 256 * 256;
         W.n_recs = B.d_ctrl + 3 * v;
         W.list_next = B.d_ctrl + 3 * v + 1;
         shapes[v] = rs;
-        // node sums for about one chunk a ring, as far as the memory goes (further chunks add atomically)
-        W.part_stride = ((long long)ne_max * gw[v].nodes_max + 63) / 64 * 64;
+        // node sums for two chunks a ring (a spot across azimuth 0 has two), as far as the memory goes (further chunks
+        // add atomically)
+        W.part_stride = ((long long)ne_max * gw[v].nodes_max * (cell ? 1 : 2) + 63) / 64 * 64;
         const size_t each = sizeof(float) * (size_t)W.part_stride, left = limit - B.ring_bytes;
         size_t cls = 1 << 20;
-        while (cls < each * ((size_t)W.n_jobs + W.n_jobs / 4 + 8)) cls <<= 1;
+        while (cls < each * std::min<size_t>(2 * (size_t)W.n_jobs + 8, (size_t)W.rec_cap)) cls <<= 1;
         while (cls > left && cls > 0) cls >>= 1;
         W.part_cap = (int)std::min<size_t>(cls / each, (size_t)W.rec_cap);
         if (W.part_cap > 0) {
           try {
-            W.parts = (float*)B.mem.alloc(cls);
+            W.parts = B.mem.alloc(cls);
             B.ring_bytes += cls;
           } catch (const Error&) {
             cudaGetLastError();
@@ -870,13 +886,7 @@ void Engine::batch_build(BatchImpl& B, int n, const ppm_params* ps, cudaStream_t
   }
   // fused point-source mode: one blackbody group, every spot a point source taking the phase-major walk,
   // at most two flux additions per (bin, energy), so that plain additions give the compensated sum's bits
-  B.fused_points = B.groups.size() == 1 && (vof[0] == 1 || vof[0] == 2);
-  for (int i = 0; i < n && B.fused_points; ++i) {
-    const ppm_params& q = ps[i];
-    bool points = q.n_spots >= 1;
-    for (int k = 0; k < q.n_spots; ++k) points &= q.spots[k].kind == PPM_SPOT_POINT;
-    B.fused_points = points && (long long)grids[q.energy_grid].E.size() <= 4 && q.n_spots * std::max(1, q.n_gl) <= 2;
-  }
+  B.fused_points = points_only;
   if (B.fused_points) {
     BatchImpl::Group& G = B.groups[0];
     G.args.n_fused = n;
@@ -1132,18 +1142,19 @@ size_t Engine::ring_work(const IntegrandShape& shape, const DevProfile* hp, cons
   }
   if (jobs <= 0 || recs > (1 << 24) || list > (1 << 30) || jobs > (1 << 24)) return 0;
   auto up = [](size_t v) { return (v + 255) / 256 * 256; };
+  W.elem_bytes = shape.nsx ? 2 : 8;
   W.hidx_bytes = (int)((2 * ((size_t)shape.n_fine + 1) + 15) / 16 * 16);
   W.off_hidx = shape.off_mu - shape.off_P;
   W.off_slice = W.off_hidx + W.hidx_bytes;
   const size_t rows = (size_t)((((shape.cpl + 1) * shape.ldS + 3) & ~3) + (shape.nE + shape.cpl + 1) * shape.ldS);
-  W.slice_bytes = (int)((rows * 4 + 15) / 16 * 16);
+  W.slice_bytes = shape.nsx ? (int)((rows * 4 + 15) / 16 * 16) : 0;
   W.stride = (long long)up((size_t)W.off_slice + W.slice_bytes);
   W.rec_cap = (int)recs;
   W.list_cap = (int)list;
   W.n_jobs = (int)jobs;
   W.n_profiles = g1 - g0;
   W.chunk = chunk;
-  const size_t bytes = up((sizeof(RingRec) + sizeof(int4)) * ((size_t)recs + 1)) + up(sizeof(unsigned short) * (size_t)list) +
+  const size_t bytes = up((sizeof(RingRec) + sizeof(int4)) * ((size_t)recs + 1)) + up((size_t)W.elem_bytes * (size_t)list) +
                        (size_t)W.stride * (size_t)jobs;
   // whole powers of two, so that the blocks of a sampler's next proposals fit the cached ones
   size_t cls = 1 << 20;
@@ -1155,9 +1166,12 @@ size_t Engine::ring_work(const IntegrandShape& shape, const DevProfile* hp, cons
 // element list) as its shared memory holds.  False if not one fits.
 bool Engine::rec_shape(IntegrandShape& s, const RingWork& W) {
   s.rec = 1;
-  s.nt = rec_threads(s.maxe_t) / (32 * s.cell_warps) * (32 * s.cell_warps);
-  s.rec_slot_bytes = (W.off_slice + W.slice_bytes + 2 * W.chunk + 31) / 16 * 16;
-  const int mu = (s.off_S - s.off_mu), batch = (s.nt * (kPairFloats / 2) * 4 + 15) / 16 * 16, room = 219 * 1024;
+  if (!s.nsx) s.cell_warps = 1;
+  s.nt = s.nsx ? rec_threads(s.maxe_t) / (32 * s.cell_warps) * (32 * s.cell_warps) : kBbRecThreads;
+  s.rec_slot_bytes = (W.off_slice + W.slice_bytes + W.elem_bytes * W.chunk + 31) / 16 * 16;
+  const int mu = (s.off_S - s.off_mu), room = 219 * 1024;
+  // the sets' records: pairs of point records, or 32 (flux, z) a warp
+  const int batch = s.nsx ? (s.nt * (kPairFloats / 2) * 4 + 15) / 16 * 16 : s.nt * 16;
   if (s.nt < 32 || room < mu + batch) return false;
   s.rec_slots = std::min(kMaxRecSlots, (room - mu - batch) / s.rec_slot_bytes);
   s.rec_off_mu = s.rec_slots * s.rec_slot_bytes;

@@ -40,6 +40,7 @@ namespace {
 constexpr double kPi = 3.14159265358979323846;
 constexpr double kTwoPi = 2. * kPi;
 constexpr int kSlotBytes = 48;  // bytes per batch point (SoA)
+constexpr int kBbPass = 128;        // blackbody from ring records: energies per pass
 constexpr int kPhaseMajorMaxE = 4;  // blackbody grids of at most this many energies take the phase-major walk
 
 __device__ __forceinline__ unsigned lanemask_lt() {
@@ -275,21 +276,22 @@ __device__ int candidate_ranges(const DevSpot& s, int N, int i, double c2, doubl
 }
 
 // Phase node u = bin * n_gl + GL point (u = bin when n_gl = 0): its bin, its
-// phase ppt and GL weight (cpu/devarshi24st_cpu.cpp:214-219).
-__device__ __forceinline__ void node_phase(const DevProfile& p, int u, int& bin, double& ppt, double& wgl) {
-  const int n_gl = p.n_gl;
+// phase ppt and GL weight (cpu/devarshi24st_cpu.cpp:214-219).  width: 1. / n_bins.
+__device__ __forceinline__ void node_phase(int n_gl, double width, int u, int& bin, double& ppt, double& wgl) {
   if (n_gl > 0) {
     bin = u / n_gl;
     const int g = u - bin * n_gl;
-    const double width = 1. / p.n_bins;
     const double lb = bin * width, ub = (bin + 1) * width;
     ppt = 0.5 * (lb + ub + c_gl_nodes[n_gl * (n_gl - 1) / 2 + g] * (ub - lb));
     wgl = 0.5 * 1. * c_gl_weights[n_gl * (n_gl - 1) / 2 + g];
   } else {
     bin = u;
-    ppt = bin * (1.0 / p.n_bins);
+    ppt = bin * width;
     wgl = 1.0;
   }
+}
+__device__ __forceinline__ void node_phase(const DevProfile& p, int u, int& bin, double& ppt, double& wgl) {
+  node_phase(p.n_gl, 1. / p.n_bins, u, bin, ppt, wgl);
 }
 
 // Active element jj of the tile at phase ppt: patch phase, hunt and lerps in
@@ -860,16 +862,21 @@ __device__ __forceinline__ void pair_slots(const Cubic2 (&Q)[C + 1], const float
 // One chunk of a ring's active elements as the deposit needs it, in shared memory
 // (read at every step of 32 points: global loads there cost their latency).
 struct ChunkCtx {
-  double dphi, jofs, l10kT, tE_lo, tE_hi, out_scale;
+  double dphi, jofs, l10kT, tE_lo, tE_hi, out_scale, width;  // width: 1 / n_bins
   long long flux_off;
   const int *perm, *cell_first;
   const float* fEs;
   const double* invE;
   unsigned long long* stats;
   float* part;             // the chunk's node sums (stored plainly), or nullptr: added to the flux pool
-  int n_act, n_nodes, u_ofs, n_fine, n_e, span, iE_min, mode;
+  int n_act, n_nodes, u_ofs, n_gl, n_fine, n_e, span, iE_min, mode;
   int mono, held;          // phase_o non-decreasing; logT or log g outside the table (points count as clamped)
   int profile, spot, rec;
+  int take;                // nodes a set takes at a time (ring records)
+  // blackbody: temperature, energies; tasks of per_pass energies, u_mod nodes each; lanes that own energies
+  double kT;
+  const double* E;
+  int per_pass, u_mod, lanes_log;
   float glo[4], ghi[4];    // smallest and largest energy fraction of each slot group
 };
 
@@ -882,6 +889,8 @@ __device__ __forceinline__ void fill_ctx(ChunkCtx& c, const DevProfile& p, const
   c.dphi = rp.dphi;
   c.jofs = rp.jofs;
   c.l10kT = sp.l10kT;
+  c.width = 1. / p.n_bins;
+  c.n_gl = p.n_gl;
   c.tE_lo = p.grid.tE_lo;
   c.tE_hi = p.grid.tE_hi;
   c.out_scale = sp.out_scale;
@@ -927,37 +936,52 @@ struct Node {
   double ppt, wgl;
 };
 
+// walk_bracket from a bracket that is right or at most two too low for almost every x (the table's: phase_o's widths
+// differ from 1 / n_fine by the delays' few per cent): two steps without a branch, the walk where a lane needs it.  All lanes of a warp call it.  lo, hi: xx at the bracket's ends.
+__device__ __forceinline__ int near_bracket(const double* xx, int n, double x, int i, double& lo, double& hi) {
+  i += x >= xx[i + 1] && i < n - 2 ? 1 : 0;
+  i += x >= xx[i + 1] && i < n - 2 ? 1 : 0;
+  lo = xx[i];
+  hi = xx[i + 1];
+  if (__any_sync(0xffffffffu, (x < lo && i > 0) || (x >= hi && i < n - 2))) {
+    i = walk_bracket(xx, n, x, i);
+    lo = xx[i];
+    hi = xx[i + 1];
+  }
+  return i;
+}
+
 // (out of line: the deposit's code is kept small for the instruction cache)
 __device__ __noinline__ int vhunt_call(const double* xx, int n, double x, double& a) { return vhunt(xx, n, x, a); }
 
-// Active element jj of the chunk at phase ppt: patch phase, hunt and lerps in
-// FP64 (cpu/devarshi24st_cpu.cpp:220-229).  Returns flux/I (0 = skip).  hidx[k]
-// is vhunt's bracket of phase_o[0] + k / n_fine: on a non-decreasing phase_o
-// (mono) the bracket of the patch phase is walked to from its table entry, a
-// step or none, and is vhunt's bracket exactly.
+// Element jj of the chunk at phase ppt: patch phase, hunt and lerps in FP64
+// (cpu/devarshi24st_cpu.cpp:220-229).  Returns flux/I (0 = skip; z and mu are then
+// not meant).  hidx[k] is vhunt's bracket of phase_o[0] + k / n_fine: on a
+// non-decreasing phase_o (mono) the bracket of the patch phase is next to its table
+// entry and is vhunt's bracket exactly.  All lanes of a warp call it (jj past the
+// last element: the last one's values).
 __device__ __forceinline__ double node_point_tab(const ChunkCtx& c, const ChunkBufs& b, int jj, double ppt, double& z,
                                                  double& mu) {
-  const double phi = c.dphi * (b.j[jj] - c.jofs);
+  const double phi = c.dphi * (b.j[min(jj, c.n_act - 1)] - c.jofs);
   const double phase_shift = phi / kTwoPi;
   // fmod(x, 1) of x = ppt + phase_shift + 1 in [1, 3): x - floor(x) is the same exact value
   const double xph = ppt + phase_shift + 1.;
   double patch = xph - floor(xph);
-  if (patch < b.P[0]) patch += 1.;
+  patch = patch < b.P[0] ? patch + 1. : patch;
   const int n = c.n_fine + 1;
   double af;
   int i;
   if (c.mono) {
     const int k = clampi((int)((patch - b.P[0]) * c.n_fine), 0, c.n_fine);
-    i = walk_bracket(b.P, n, patch, b.hidx[k]);
-    af = (patch - b.P[i]) / (b.P[i + 1] - b.P[i]);
+    double lo, hi;
+    i = near_bracket(b.P, n, patch, b.hidx[k], lo, hi);
+    af = (patch - lo) / (hi - lo);
   } else {
     i = vhunt_call(b.P, n, patch, af);
   }
-  const double flux = (1 - af) * b.F[i] + af * b.F[i + 1];
-  if (flux == 0) return 0.0;
   z = (1 - af) * b.Z[i] + af * b.Z[i + 1];
   mu = (1 - af) * b.MU[i] + af * b.MU[i + 1];
-  return flux;
+  return (1 - af) * b.F[i] + af * b.F[i + 1];
 }
 
 // vhunt's bracket on the descending mu axis (cpu/hunt.hpp:14-66), walked to from
@@ -1059,10 +1083,10 @@ __device__ __forceinline__ void deposit_node(const KernelArgs& a, const ChunkCtx
     int G0 = 0, imu = 0;
     float w4[4] = {0.f, 0.f, 0.f, 0.f};
     const int jj = jb + st;
-    if (jj < n_act) {
+    {
       double z = 0, mu = 0;
       const double flux = node_point_tab(c, b, jj, nd.ppt, z, mu);
-      if (flux != 0.0) {
+      if (jj < n_act && flux != 0.0) {
         vis = true;
         if (mu < mu_s[nmu - 1]) mu = mu_s[nmu - 1];
         cw = (float)(flux * nd.wgl);
@@ -1341,16 +1365,16 @@ __device__ __forceinline__ void build_slice(const DevNsx& X, int ldS, int C, con
 
 // The bracket table of phase_o for node_point_tab (hidx in shared or global
 // memory), used where phase_o is non-decreasing: returns whether it is (a block
-// barrier).
+// barrier; the table is complete after the next one).  walk_bracket gives vhunt's
+// bracket there, a step or two from entry k.
 __device__ __forceinline__ bool phase_table(const double* P, int n_fine, unsigned short* hidx) {
   const int tid = threadIdx.x, nt = blockDim.x;
   bool ok = true;
   for (int k = tid; k < n_fine; k += nt) ok &= P[k + 1] >= P[k];
-  for (int k = tid; k <= n_fine; k += nt) {
-    double a_unused;
-    hidx[k] = (unsigned short)vhunt(P, n_fine + 1, P[0] + (double)k / n_fine, a_unused);
-  }
-  return __syncthreads_and(ok) != 0;
+  if (__syncthreads_and(ok) == 0) return false;
+  for (int k = tid; k <= n_fine; k += nt)
+    hidx[k] = (unsigned short)walk_bracket(P, n_fine + 1, P[0] + (double)k / n_fine, min(k, n_fine - 1));
+  return true;
 }
 
 // Home-cell kernel over the planner's tiles: every tile computes its ring's
@@ -1429,6 +1453,7 @@ __global__ void __launch_bounds__(NTMAX, MINB) integrand_nsx_cell_kernel(const K
 // phase nodes one at a time from the chunk's counter in global memory.
 
 // One CTA per (profile, spot, ring).
+template <bool NSX>
 __global__ void __launch_bounds__(256) ring_kernel(const KernelArgs a) {
   extern __shared__ __align__(16) unsigned char sm[];
   const IntegrandShape& S = a.shape;
@@ -1464,8 +1489,7 @@ __global__ void __launch_bounds__(256) ring_kernel(const KernelArgs a) {
   const double z = point ? sp.cos_theta_pt : p.ring[3 * ring];
   const double c2 = point ? 0.0 : p.ring[3 * ring + 1], s2 = point ? 0.0 : p.ring[3 * ring + 2];
   if (tid == 0) {
-    ring_geometry(p, L, z, point ? sp.dOmega_pt : p.dOmega_hp, true, s_g);
-    s_ntap = nsx_taps(a.nsx, p, sp, s_g.logg, s_tapw, s_tapo);
+    ring_geometry(p, L, z, point ? sp.dOmega_pt : p.dOmega_hp, NSX, s_g);
   }
   if (tid == 32) {
     int r[2][2] = {{0, 0}, {0, 0}};
@@ -1478,32 +1502,16 @@ __global__ void __launch_bounds__(256) ring_kernel(const KernelArgs a) {
   __syncthreads();
   const int nr = s_nr;
   if (nr == 0) return;
-  const bool dropped = ring_sweep(a, p, s, s_g, s_int, true);
-  if (dropped) {  // counted, with its elements, only if it holds active elements (as plan_kernel)
-    int na = 0;
-    if (point) {
-      na = tid == 0 ? 1 : 0;
-    } else {
-      for (int k = 0; k < nr; ++k)
-        for (int j = s_range[k][0] + tid; j <= s_range[k][1]; j += nt)
-          na += in_spot(sp, c2, s2, healpix_phi(p.n_side, ring, j)) ? 1 : 0;
-    }
-    na = __reduce_add_sync(0xffffffffu, na);
-    if (tid == 0) s_int[42] = 0;
-    __syncthreads();
-    if ((tid & 31) == 0 && na) atomicAdd(&s_int[42], na);
-    __syncthreads();
-    if (tid == 0 && s_int[42]) {
-      atomicAdd(&p.stats[1], 1ull);
-      atomicAdd(&p.stats[2], 1ull);
-      atomicAdd(&p.stats[5], (unsigned long long)s_int[42]);
-      if (s_g.u_clamped && !point) atomicAdd(&p.stats[4], 1ull);
-    }
-    return;
-  }
+  const bool dropped = ring_sweep(a, p, s, s_g, s_int, NSX);
+  if (NSX && tid == nt - 1) s_ntap = nsx_taps(a.nsx, p, sp, s_g.logg, s_tapw, s_tapo);
   // the ring's image: the sweep as it lies in shared memory, the bracket table, the slice
   unsigned char* const img = W.data + (size_t)job * W.stride;
-  const bool mono = phase_table(s.P, p.n_fine, (unsigned short*)(img + W.off_hidx));
+  const bool mono = !dropped && phase_table(s.P, p.n_fine, (unsigned short*)(img + W.off_hidx));
+  if (!NSX && !dropped) {  // MU is not needed: reciprocal widths of the phase_o intervals in its place
+    __syncthreads();
+    for (int k = tid; k < p.n_fine; k += nt) s.MU[k] = 1.0 / (s.P[k + 1] - s.P[k]);
+  }
+  const RingPhi rp = point ? RingPhi{0.0, 0.0} : healpix_ring_phi(p.n_side, ring);
   // active elements, one record per chunk of candidates
   int n_ring = 0;
   bool first = true;
@@ -1521,16 +1529,17 @@ __global__ void __launch_bounds__(256) ring_kernel(const KernelArgs a) {
         n_act += tot;
         __syncthreads();
       }
-      if (n_act == 0) continue;
       n_ring += n_act;
+      if (n_act == 0 || dropped) continue;
       if (tid == 0) {
         const int at = atomicAdd(W.n_recs, 1), lo = atomicAdd(W.list_next, (n_act + 7) & ~7);
         s_int[43] = lo;
-        const bool held = sp.T_clamped || s_g.logg < a.nsx.g_min || s_g.logg > a.nsx.g_max;
+        const bool held = NSX && (sp.T_clamped || s_g.logg < a.nsx.g_min || s_g.logg > a.nsx.g_max);
+        const int tasks = p.n_bins * max(p.n_gl, 1) * (NSX ? 1 : (p.n_e + kBbPass - 1) / kBbPass);
         if (at < W.rec_cap && lo + n_act <= W.list_cap) {
-          W.recs[at] = RingRec{s_job[0], s_job[1], ring, job, n_act, lo, p.n_bins * max(p.n_gl, 1),
+          W.recs[at] = RingRec{s_job[0], s_job[1], ring, job, n_act, lo, tasks,
                                (mono ? 1 : 0) | (held ? 2 : 0)};
-          W.ctr[at] = make_int4(0, 0, p.n_bins * max(p.n_gl, 1), n_act);
+          W.ctr[at] = make_int4(0, 0, tasks, n_act);
         } else {
           s_int[43] = -1;
           atomicOr(a.queue.overflow, 1);
@@ -1540,18 +1549,29 @@ __global__ void __launch_bounds__(256) ring_kernel(const KernelArgs a) {
       __syncthreads();
       const int lo = s_int[43];
       if (lo >= 0)
-        for (int c = tid; c < n_act; c += nt) W.lists[lo + c] = s.j[c];
+        for (int c = tid; c < n_act; c += nt) {
+          if (NSX)
+            ((unsigned short*)W.lists)[lo + c] = s.j[c];
+          else  // the element's phase shift phi / 2 pi
+            ((double*)W.lists)[lo + c] = (point ? 0.0 : rp.dphi * (s.j[c] - rp.jofs)) / kTwoPi;
+        }
       __syncthreads();
     }
   }
   if (n_ring == 0) return;
-  if (tid == 0) {
-    atomicAdd(&p.stats[0], (unsigned long long)n_ring);
+  if (tid == 0) {  // a dropped ring is counted, with its elements, only if it holds active elements (as plan_kernel)
+    atomicAdd(&p.stats[dropped ? 5 : 0], (unsigned long long)n_ring);
     atomicAdd(&p.stats[1], 1ull);
+    if (dropped) {
+      atomicAdd(&p.stats[2], 1ull);
+      if (s_g.u_clamped && !point) atomicAdd(&p.stats[4], 1ull);
+    }
   }
+  if (dropped) return;
   const int n16 = (S.off_mu - S.off_P) >> 4;
   for (int k = tid; k < n16; k += nt) ((float4*)img)[k] = ((const float4*)(sm + S.off_P))[k];
-  build_slice(a.nsx, S.ldS, S.cpl, s_tapw, s_tapo, s_ntap, (float*)(img + W.off_slice) + slice_row0(S.ldS, S.cpl));
+  if (NSX)
+    build_slice(a.nsx, S.ldS, S.cpl, s_tapw, s_tapo, s_ntap, (float*)(img + W.off_slice) + slice_row0(S.ldS, S.cpl));
 }
 
 // 16-byte asynchronous copy from global to shared memory.
@@ -1569,30 +1589,26 @@ constexpr unsigned kSlotDead = 1u << 18;     // no chunk left to load
 // loaded chunk; the last set to leave a drained slot loads its next chunk (the
 // one with the most work left per slot on it) while the others go on with the
 // other slots, so that nobody waits for a chunk's slowest node.
-template <int MAXE, int C, int NTMAX>
-__global__ void __launch_bounds__(NTMAX, 1) integrand_nsx_rec_kernel(const KernelArgs a) {
-  extern __shared__ __align__(16) unsigned char sm[];
+// Work is what a set does with the nodes it took (fill: a loaded chunk's context;
+// enter: the set comes to another chunk; nodes: the nodes [u, u + take)).
+template <int NTMAX, class Work>
+__device__ __forceinline__ void rec_loop(const KernelArgs& a, unsigned char* sm, Work& w) {
   const IntegrandShape& S = a.shape;
   const RingWork& W = a.rings;
   constexpr int kSets = NTMAX / 32;
   __shared__ ChunkCtx s_ctx[kMaxRecSlots];
   __shared__ unsigned s_word[kMaxRecSlots];
-  __shared__ Node s_node[kSets];
-  __shared__ int s_got[kSets], s_wcnt[kSets];
+  __shared__ int s_got[kSets], s_u[kSets];
   __shared__ unsigned long long s_best[kSets];
   const int tid = threadIdx.x, nt = blockDim.x;
-  const DevNsx& X = a.nsx;
   const int n_recs = min(*W.n_recs, W.rec_cap);
   if (n_recs == 0) return;
   const int NS = S.rec_slots;
-  double* const mu_s = (double*)(sm + S.rec_off_mu);
-  load_mu(X, mu_s);
   if (tid < NS) {
     s_word[tid] = kSlotDrain;
     s_ctx[tid].rec = -1;
   }
   __syncthreads();
-  const SetPlace<C> w(S, (float*)(sm + S.rec_off_batch));
   const int per_slot = max(1, nt / w.ST / NS);  // warp sets per slot
   const int a16 = (S.off_F - S.off_P) / 8;      // doubles between the sweep's arrays
   volatile unsigned* const word = s_word;
@@ -1602,9 +1618,7 @@ __global__ void __launch_bounds__(NTMAX, 1) integrand_nsx_rec_kernel(const Kerne
     return atomicSub(&s_word[sl], 1u) == (kSlotDrain | 1u) && atomicCAS(&s_word[sl], kSlotDrain, kSlotLoading) == kSlotDrain;
   };
   constexpr int kExit = -1;  // s_got: a slot to work in, kExit, or -2 - slot to load
-  float fE[C][MAXE];
-  unsigned n_vis = 0, n_clamped = 0;
-  int cur_rec = -1, cur_slot = -1, profile = -1;
+  int cur_rec = -1, cur_slot = -1, profile = -1, pref = w.set % NS;
   bool claimed = false;  // (leader) the slot just left is this set's to load
   for (;;) {
     if (w.st == 0) {
@@ -1617,7 +1631,8 @@ __global__ void __launch_bounds__(NTMAX, 1) integrand_nsx_rec_kernel(const Kerne
         for (int spin = 0; spin < (1 << 21); ++spin) {
           bool live = false;
           for (int k = 0; k < NS && got == kExit; ++k) {
-            const int sl = (max(cur_slot, w.set % NS) + k) % NS;
+            int sl = pref + k;
+            sl -= sl >= NS ? NS : 0;
             const unsigned v = word[sl];
             if (v & kSlotDead) continue;
             live = true;
@@ -1629,12 +1644,9 @@ __global__ void __launch_bounds__(NTMAX, 1) integrand_nsx_rec_kernel(const Kerne
             if (!(atomicAdd(&s_word[sl], 1u) & (kSlotDrain | kSlotLoading | kSlotDead))) {
               __threadfence_block();
               const ChunkCtx& c = s_ctx[sl];
-              const int u = atomicAdd(&W.ctr[c.rec].x, 1);
+              const int u = atomicAdd(&W.ctr[c.rec].x, c.take);
               if (u < c.n_nodes) {
-                const int v2 = u + c.u_ofs < c.n_nodes ? u + c.u_ofs : u + c.u_ofs - c.n_nodes;
-                Node& nd = s_node[w.set];
-                nd.node = v2;
-                node_phase(a.profiles[c.profile], v2, nd.bin, nd.ppt, nd.wgl);
+                s_u[w.set] = u;
                 got = sl;
                 continue;
               }
@@ -1707,14 +1719,15 @@ __global__ void __launch_bounds__(NTMAX, 1) integrand_nsx_rec_kernel(const Kerne
       const unsigned char* const img = W.data + (size_t)q.job * W.stride;
       const int n16 = (W.off_slice + W.slice_bytes) >> 4;
       for (int k = w.st; k < n16; k += w.ST) cp_async16(dst + 16 * k, img + 16 * k);
-      for (int k = w.st; k < ((q.n_act + 7) >> 3); k += w.ST)
-        cp_async16(dst + 16 * (n16 + k), W.lists + q.list + 8 * k);
+      const int l16 = (q.n_act * W.elem_bytes + 15) >> 4;
+      for (int k = w.st; k < l16; k += w.ST) cp_async16(dst + 16 * (n16 + k), W.lists + (size_t)q.list * W.elem_bytes + 16 * k);
       if (w.st == 0) {
         const DevProfile& p = a.profiles[q.profile];
         ChunkCtx& c = s_ctx[sl];
-        fill_ctx<MAXE, 2>(c, p, p.spot[q.spot], q.ring, q.n_act, (q.flags & 1) != 0, (q.flags & 2) != 0);
-        c.u_ofs = (int)((unsigned)q.job * 40503u % (unsigned)q.n_nodes);
-        c.part = r < W.part_cap ? W.parts + (size_t)r * W.part_stride : nullptr;
+        w.fill(c, p, p.spot[q.spot], q);
+        // nodes are taken from a chunk's own first one on: chunks that run at the same time add to different bins
+        c.u_ofs = (int)((unsigned)q.job * 40503u % (unsigned)c.u_mod);
+        c.part = r < W.part_cap ? (float*)W.parts + (size_t)r * W.part_stride : nullptr;
         c.profile = q.profile;
         c.spot = q.spot;
         c.rec = r;
@@ -1730,32 +1743,319 @@ __global__ void __launch_bounds__(NTMAX, 1) integrand_nsx_rec_kernel(const Kerne
     }
     // a node of the chunk in slot `got`
     __threadfence_block();
-    cur_slot = got;
+    cur_slot = pref = got;
     const ChunkCtx& c = s_ctx[got];
     if (c.rec != cur_rec) {
       cur_rec = c.rec;
-      if (w.lane == 0 && profile >= 0 && profile != c.profile) {
-        if (n_vis) atomicAdd(&a.profiles[profile].stats[3], (unsigned long long)n_vis);
-        if (n_clamped) atomicAdd(&a.profiles[profile].stats[4], (unsigned long long)n_clamped);
-        n_vis = n_clamped = 0;
-      }
+      if (profile != c.profile) w.count(profile);
       profile = c.profile;
-      lane_fractions<MAXE, C>(c, w, fE);
+      w.enter(c);
     }
     const unsigned char* const base = sm + (size_t)got * S.rec_slot_bytes;
     const double* P = (const double*)base;
     const ChunkBufs bufs{(const unsigned short*)(base + W.off_slice + W.slice_bytes), P, P + a16, P + 2 * a16, P + 3 * a16,
                          (const unsigned short*)(base + W.off_hidx),
-                         (const float*)(base + W.off_slice) + slice_row0(S.ldS, C)};
-    deposit_node<MAXE, C, 2>(a, c, bufs, s_node[w.set], mu_s, w, fE, s_wcnt, n_vis, n_clamped);
+                         (const float*)(base + W.off_slice) + slice_row0(S.ldS, S.cpl)};
+    w.nodes(c, bufs, s_u[w.set]);
     __threadfence_block();
     set_sync(w.set, w.ST);
     if (w.st == 0) claimed = leave(got);
   }
-  if (w.lane == 0 && profile >= 0) {
-    if (n_vis) atomicAdd(&a.profiles[profile].stats[3], (unsigned long long)n_vis);
-    if (n_clamped) atomicAdd(&a.profiles[profile].stats[4], (unsigned long long)n_clamped);
+  w.count(profile);
+}
+
+// Work of the home-cell NSX kernel: one node at a time.
+template <int MAXE, int C, int NTMAX>
+struct NsxWork : SetPlace<C> {
+  const KernelArgs& a;
+  const double* mu_s;
+  Node* s_node;
+  int* wcnt;
+  float fE[C][MAXE];
+  unsigned n_vis = 0, n_clamped = 0;
+  __device__ __forceinline__ NsxWork(const KernelArgs& args, unsigned char* sm, Node* nodes_, int* wcnt_)
+      : SetPlace<C>(args.shape, (float*)(sm + args.shape.rec_off_batch)), a(args),
+        mu_s((const double*)(sm + args.shape.rec_off_mu)), s_node(nodes_), wcnt(wcnt_) {}
+  __device__ __forceinline__ void fill(ChunkCtx& c, const DevProfile& p, const DevSpot& sp, const RingRec& q) {
+    fill_ctx<MAXE, 2>(c, p, sp, q.ring, q.n_act, (q.flags & 1) != 0, (q.flags & 2) != 0);
+    c.take = 1;
+    c.u_mod = c.n_nodes;
   }
+  __device__ __forceinline__ void enter(const ChunkCtx& c) { lane_fractions<MAXE, C>(c, *this, fE); }
+  __device__ __forceinline__ void nodes(const ChunkCtx& c, const ChunkBufs& b, int u) {
+    Node& nd = s_node[this->set];
+    if (this->st == 0) {
+      nd.node = u + c.u_ofs < c.n_nodes ? u + c.u_ofs : u + c.u_ofs - c.n_nodes;
+      node_phase(c.n_gl, c.width, nd.node, nd.bin, nd.ppt, nd.wgl);
+    }
+    set_sync(this->set, this->ST);
+    deposit_node<MAXE, C, 2>(a, c, b, nd, mu_s, *this, fE, wcnt, n_vis, n_clamped);
+  }
+  __device__ __forceinline__ void count(int profile) {  // the warp's counters to the profile it leaves
+    if (this->lane == 0 && profile >= 0) {
+      if (n_vis) atomicAdd(&a.profiles[profile].stats[3], (unsigned long long)n_vis);
+      if (n_clamped) atomicAdd(&a.profiles[profile].stats[4], (unsigned long long)n_clamped);
+    }
+    n_vis = n_clamped = 0;
+  }
+};
+
+template <int MAXE, int C, int NTMAX>
+__global__ void __launch_bounds__(NTMAX, 1) integrand_nsx_rec_kernel(const KernelArgs a) {
+  extern __shared__ __align__(16) unsigned char sm[];
+  __shared__ Node s_node[NTMAX / 32];
+  __shared__ int s_wcnt[NTMAX / 32];
+  load_mu(a.nsx, (double*)(sm + a.shape.rec_off_mu));
+  NsxWork<MAXE, C, NTMAX> w(a, sm, s_node, s_wcnt);
+  rec_loop<NTMAX>(a, sm, w);
+}
+
+// ---------------------------------------------------------------------------
+// Blackbody integrand from ring records.  A warp takes `take` phase nodes of a
+// chunk at a time and walks a node's elements 32 at a time, a point per lane.
+// Few energies (at most kPhaseMajorMaxE): the lane evaluates its point at each.
+// More: the visible points are compacted into the warp's records and the lanes
+// own the energies (c.lanes of them, up to four each; the lane groups take the
+// records in turn), kBbPass energies a pass, each pass a task of its own.  The
+// sums are FP64 in every arithmetic; a node's are combined over the lanes and
+// stored.  Bound by the FP64 pipe (about 60 operations a point and energy).
+// FP32 arithmetic keeps the form of the tile kernel's path for the grid's size.
+template <typename Real>
+struct BbWork {
+  const KernelArgs& a;
+  int lane, set, st;
+  static constexpr int ST = 32;
+  double2* rec;
+  unsigned n_vis = 0;
+  __device__ __forceinline__ BbWork(const KernelArgs& args, unsigned char* sm) : a(args) {
+    lane = st = threadIdx.x & 31;
+    set = threadIdx.x >> 5;
+    rec = (double2*)(sm + args.shape.rec_off_batch) + 32 * set;
+  }
+  __device__ __forceinline__ void fill(ChunkCtx& c, const DevProfile& p, const DevSpot& sp, const RingRec& q) {
+    fill_ctx<1, 1>(c, p, sp, q.ring, q.n_act, (q.flags & 1) != 0, false);
+    c.kT = sp.kT;
+    c.E = p.grid.E;
+    const int passes = (p.n_e + kBbPass - 1) / kBbPass;
+    c.per_pass = (p.n_e + passes - 1) / passes;
+    c.u_mod = c.n_nodes;
+    c.n_nodes *= passes;  // as ring_kernel counted the chunk's tasks
+    // nodes per take: about 2048 points, but takes for every warp several times over
+    const long long tasks = (long long)min(*a.rings.n_recs, a.rings.rec_cap) * c.n_nodes;
+    c.take = (int)max(1ll, min(min((long long)c.u_mod / 8, 2048ll / max(q.n_act, 8)), tasks / (gridDim.x * (blockDim.x / 8))));
+    int ll = 0;
+    if (c.per_pass > kPhaseMajorMaxE)
+      while (ll < 5 && (1 << ll) < c.per_pass) ++ll;
+    c.lanes_log = ll;
+  }
+  // few energies: nodes at a time, this lane's node among them and its (first) element
+  int m = 1, sub = 0, jl = 0;
+  __device__ __forceinline__ void enter(const ChunkCtx& c) {
+    m = c.n_act <= 16 ? 32 / c.n_act : 1;
+    sub = m > 1 ? lane / c.n_act : 0;
+    jl = lane - sub * c.n_act;
+    if (m == 1) jl = lane;
+  }
+  __device__ __forceinline__ void count(int profile) {
+    n_vis = __reduce_add_sync(0xffffffffu, n_vis);
+    if (lane == 0 && profile >= 0 && n_vis) atomicAdd(&a.profiles[profile].stats[3], (unsigned long long)n_vis);
+    n_vis = 0;
+  }
+  // Ibb without its constant, times the point's flux (cpu/unit.hpp:28-31).
+  static __device__ __forceinline__ double planck(Real cb, Real zb, Real E, Real kT, Real inv_kT, bool divide) {
+    const Real Ee = E * zb;
+    return (double)(cb * (Ee * Ee * Ee / expm1(std::is_same<Real, float>::value && divide ? Ee / kT : Ee * inv_kT)));
+  }
+  // The same of two points.  Where x = E / kT > 1 for every lane's, e^x - 1 loses nothing to cancellation (two
+  // roundings, as expm1 has) and is cheaper; hidden points have c = 0 and z = 1.  In one block, so that the two
+  // evaluations overlap and share their constants.  All lanes call it.
+  static __device__ __forceinline__ double planck_pair(double ca, double za, double cb, double zb, double E, double inv_kT) {
+    const double ea = E * za, eb = E * zb, xa = ea * inv_kT, xb = eb * inv_kT;
+    if (__all_sync(0xffffffffu, xa > 1.0 && xb > 1.0)) {
+      const double ya = exp(xa) - 1.0, yb = exp(xb) - 1.0;
+      return ca * (ea * ea * ea / ya) + cb * (eb * eb * eb / yb);
+    }
+    return ca * (ea * ea * ea / expm1(xa)) + cb * (eb * eb * eb / expm1(xb));
+  }
+  // The bracket and fraction of element jj's patch phase (node_point_tab, with the element's phase shift and the
+  // reciprocal interval widths from the ring's image).  All lanes call it.
+  static __device__ __forceinline__ int bracket(const ChunkCtx& c, const ChunkBufs& b, int jj, double ppt, double& af) {
+    const double xph = ppt + ((const double*)b.j)[min(jj, c.n_act - 1)] + 1.;
+    // x - floor(x) for x in [1, 3]: the same exact value
+    double patch = xph - (xph >= 3.0 ? 3.0 : (xph >= 2.0 ? 2.0 : 1.0));
+    const double P0 = b.P[0];
+    patch = patch < P0 ? patch + 1. : patch;
+    int i;
+    double lo, hi;
+    if (c.mono) {
+      i = near_bracket(b.P, c.n_fine + 1, patch, b.hidx[clampi((int)((patch - P0) * c.n_fine), 0, c.n_fine)], lo, hi);
+    } else {
+      i = vhunt_call(b.P, c.n_fine + 1, patch, af);
+      lo = b.P[i];
+    }
+    af = (patch - lo) * b.MU[i];
+    return i;
+  }
+  // flux/I and redshift of element jj where `on` (else 0 and 1)
+  static __device__ __forceinline__ double point(const ChunkCtx& c, const ChunkBufs& b, int jj, bool on, double ppt,
+                                                 double& z) {
+    double af;
+    const int i = bracket(c, b, jj, ppt, af);
+    const double flux = (1 - af) * b.F[i] + af * b.F[i + 1], zz = (1 - af) * b.Z[i] + af * b.Z[i + 1];
+    on = on && flux != 0.0;
+    z = on ? zz : 1.0;
+    return on ? flux : 0.0;
+  }
+  // one point at the grid's few energies, in FP32 arithmetic: the phase-major walk's form (pm_walk)
+  static __device__ __forceinline__ void point_few32(const ChunkCtx& c, const ChunkBufs& b, int jj, bool on, double ppt, double wgl,
+                                                     const float* E, int n_e, float inv_kT, double* acc, unsigned& vis) {
+    double afd;
+    const int i = bracket(c, b, jj, ppt, afd);
+    const float af = (float)afd;
+    const float f0 = (float)b.F[i], flux = fmaf(af, (float)b.F[i + 1] - f0, f0);
+    if (!on || flux == 0.f) return;
+    const float z0 = (float)b.Z[i], zb = fmaf(af, (float)b.Z[i + 1] - z0, z0), cb = flux * (float)wgl;
+    ++vis;
+#pragma unroll
+    for (int e = 0; e < kPhaseMajorMaxE; ++e) {
+      if (e >= n_e) break;
+      const float Ee = E[e] * zb, x = Ee * inv_kT;
+      acc[e] += (double)(cb * __fdividef(Ee * Ee * Ee, x > 0.5f ? __expf(x) - 1.f : expm1f(x)));
+    }
+  }
+  // a node's sum of energy e
+  __device__ __forceinline__ void store(const ChunkCtx& c, int v, int bin, int e, double sum) {
+    if (c.part) {
+      ((double*)c.part)[(size_t)v * c.n_e + e] = sum;
+    } else if (sum != 0.0) {
+      const size_t o = (size_t)c.flux_off + (size_t)bin * c.n_e + e;
+      comp_add(a.flux + o, a.comp ? a.comp + o : nullptr, sum * c.out_scale * c.invE[e]);
+    }
+  }
+  // few energies: m nodes at a time (rings of few elements), else two elements a lane
+  __device__ __forceinline__ void nodes_few(const ChunkCtx& c, const ChunkBufs& b, int u0) {
+    const int u_end = min(u0 + c.take, c.n_nodes), ne = c.n_e, n_act = c.n_act;
+    const Real inv_kT = (Real)1 / (Real)c.kT;
+    Real E[kPhaseMajorMaxE];
+#pragma unroll
+    for (int k = 0; k < kPhaseMajorMaxE; ++k) E[k] = k < ne ? (Real)c.E[k] : (Real)1;
+    const bool few32 = std::is_same<Real, float>::value && c.mono;
+    for (int u = u0; u < u_end; u += m) {
+      const bool live = sub < m && u + sub < u_end;
+      int v = u + (live ? sub : 0) + c.u_ofs, bin;
+      v -= v >= c.u_mod ? c.u_mod : 0;
+      double ppt, wgl;
+      node_phase(c.n_gl, c.width, v, bin, ppt, wgl);
+      double acc[kPhaseMajorMaxE] = {0.0, 0.0, 0.0, 0.0};
+      for (int jb = 0; jb < n_act; jb += 64) {
+        const int ja = jb + jl, jc = ja + 32;
+        const bool on_a = live && ja < n_act, on_b = m == 1 && jc < n_act;
+        if (few32) {
+          point_few32(c, b, ja, on_a, ppt, wgl, (const float*)E, ne, (float)inv_kT, acc, n_vis);
+          if (m == 1) point_few32(c, b, jc, on_b, ppt, wgl, (const float*)E, ne, (float)inv_kT, acc, n_vis);
+          continue;
+        }
+        double za = 1.0, zb = 1.0, ca = 0.0, cb = 0.0;
+        const double fa = point(c, b, ja, on_a, ppt, za);
+        double fb = 0.0;
+        if (m == 1) fb = point(c, b, jc, on_b, ppt, zb);
+        n_vis += (fa != 0.0 ? 1u : 0u) + (fb != 0.0 ? 1u : 0u);
+        ca = fa * wgl;
+        cb = fb * wgl;
+#pragma unroll
+        for (int k = 0; k < kPhaseMajorMaxE; ++k)
+          if (k < ne) {
+            if constexpr (std::is_same<Real, double>::value) {
+              acc[k] += planck_pair(ca, za, cb, zb, E[k], inv_kT);
+            } else {
+              if (fa != 0.0) acc[k] += planck((Real)ca, (Real)za, E[k], (Real)0, inv_kT, false);
+              if (fb != 0.0) acc[k] += planck((Real)cb, (Real)zb, E[k], (Real)0, inv_kT, false);
+            }
+          }
+      }
+      for (int off = 1; off < 32; off <<= 1) {
+        const bool same = m == 1 || (lane + off < 32 && jl + off < n_act);
+#pragma unroll
+        for (int k = 0; k < kPhaseMajorMaxE; ++k)
+          if (k < ne) {
+            const double o = __shfl_down_sync(0xffffffffu, acc[k], off);
+            if (same) acc[k] += o;
+          }
+      }
+      if (live && (m == 1 ? lane == 0 : jl == 0))
+#pragma unroll
+        for (int k = 0; k < kPhaseMajorMaxE; ++k)
+          if (k < ne) store(c, v, bin, k, acc[k]);
+    }
+  }
+  __device__ __forceinline__ void nodes(const ChunkCtx& c, const ChunkBufs& b, int u0) {
+    if (c.lanes_log == 0) {
+      nodes_few(c, b, u0);
+      return;
+    }
+    const int u_end = min(u0 + c.take, c.n_nodes);
+    const Real kT = (Real)c.kT, inv_kT = (Real)1 / kT;
+    const int ll = c.lanes_log, ln = 1 << ll, grp = lane >> ll, el = lane & (ln - 1), n_grp = 32 >> ll;
+    const bool divide = c.n_e > 64;
+    for (int u = u0; u < u_end; ++u) {
+      int pass = 0, v = u;
+      while (v >= c.u_mod) {
+        v -= c.u_mod;
+        ++pass;
+      }
+      const int e0 = pass * c.per_pass, ne = min(c.per_pass, c.n_e - e0), ke = (ne + ln - 1) >> ll;
+      v += c.u_ofs;
+      v -= v >= c.u_mod ? c.u_mod : 0;
+      int bin;
+      double ppt, wgl;
+      node_phase(c.n_gl, c.width, v, bin, ppt, wgl);
+      Real E[4];
+      double acc[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int e = el + (k << ll);
+        E[k] = e < ne ? (Real)c.E[e0 + e] : (Real)1;
+      }
+      for (int jb = 0; jb < c.n_act; jb += 32) {
+        const int jj = jb + lane;
+        double flux = 0.0, z = 0;
+        flux = point(c, b, jj, jj < c.n_act, ppt, z);
+        const unsigned bal = __ballot_sync(0xffffffffu, flux != 0.0);
+        if (flux != 0.0) {
+          rec[__popc(bal & lanemask_lt())] = make_double2(flux * wgl, z);
+          n_vis += pass == 0 ? 1u : 0u;
+        }
+        __syncwarp();
+        const int nv = __popc(bal);
+        for (int q = grp; q < nv; q += n_grp) {
+          const double2 r = rec[q];
+          const Real cb = (Real)r.x, zb = (Real)r.y;
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            if (k < ke) acc[k] += planck(cb, zb, E[k], kT, inv_kT, divide);
+        }
+        __syncwarp();
+      }
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1)
+        if (off >= ln)
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            if (k < ke) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], off);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int e = el + (k << ll);
+        if (grp == 0 && e < ne) store(c, v, bin, e0 + e, acc[k]);
+      }
+    }
+  }
+};
+
+template <typename Real>
+__global__ void __launch_bounds__(kBbRecThreads, 1) integrand_bb_rec_kernel(const KernelArgs a) {
+  extern __shared__ __align__(16) unsigned char sm[];
+  BbWork<Real> w(a, sm);
+  rec_loop<kBbRecThreads>(a, sm, w);
 }
 
 // ---------------------------------------------------------------------------
@@ -2321,6 +2621,7 @@ IntegrandShape make_shape(bool nsx, int nt, int ne_t, int pb, int max_cand, int 
   s.off_Q = off + batch;
   off += rows > batch + qbuf ? rows : batch + qbuf;
   s.total = off;
+  s.ring_bytes = s.off_rows + rows;
   return s;
 }
 
@@ -2350,6 +2651,7 @@ void* kernel_for(const IntegrandShape& s, int precision) {
       default: return (void*)integrand_nsx_kernel<4, 1>;
     }
   }
+  if (s.rec) return precision == 1 ? (void*)integrand_bb_rec_kernel<double> : (void*)integrand_bb_rec_kernel<float>;
   if (precision == 1) {
     switch (s.ne_t) {
       case 1: return (void*)integrand_bb_kernel<double, 1>;
@@ -2389,7 +2691,8 @@ cudaError_t set_integrand_smem() {
 #define PPM_CELL(E, C)                                                                            \
   (void*)integrand_nsx_cell_kernel<E, C, 512, 1>, (void*)integrand_nsx_cell_kernel<E, C, kCellThreads, 2>, \
       (void*)integrand_nsx_rec_kernel<E, C, rec_threads(E)>,
-  void* fns[] = {PPM_CELL_SHAPES(PPM_CELL)(void*) ring_kernel,
+  void* fns[] = {PPM_CELL_SHAPES(PPM_CELL)(void*) ring_kernel<true>, (void*)ring_kernel<false>,
+                 (void*)integrand_bb_rec_kernel<double>, (void*)integrand_bb_rec_kernel<float>,
                  (void*)integrand_nsx_kernel<1, 1>, (void*)integrand_nsx_kernel<1, 2>,
                  (void*)integrand_nsx_kernel<2, 1>, (void*)integrand_nsx_kernel<2, 2>, (void*)integrand_nsx_kernel<4, 1>,
                  (void*)integrand_bb_kernel<double, 1>, (void*)integrand_bb_kernel<double, 2>,
@@ -2447,7 +2750,7 @@ cudaError_t launch_add_comp(double* flux, const double* comp, long long n, int s
 }
 
 namespace {
-constexpr int kSumQ = 128, kSumSegs = 8, kSumRecs = 1024;
+constexpr int kSumThreads = 256, kSumQ = 32, kSumUnroll = 12, kSumList = 6 * kSumThreads;
 
 __device__ __forceinline__ void dd_add(double& s, double& c, double x) {
   // (intrinsics: x is a product, which must not be contracted into the sum)
@@ -2456,49 +2759,65 @@ __device__ __forceinline__ void dd_add(double& s, double& c, double x) {
   s = t;
 }
 
-// The flux of one (profile, bin) from its chunks' node sums: grid (bins, energy tiles of kSumQ, profiles), kSumSegs
-// threads an energy, each over every kSumSegs-th chunk.  Double-double sums: the exact sum to about 1e-32, in any
-// order of the records, as the pool's compensated atomics give it; what the atomics added is included.  Bound by the
-// read of the node sums (4 bytes per node and energy, from L2 for a single profile).
-__global__ void __launch_bounds__(kSumQ * kSumSegs) sum_parts_kernel(const KernelArgs a) {
+// The flux of one (profile, bin) from its chunks' node sums (T: float in t_E order for NSX, double in energy order
+// for blackbody): grid (bins, energy tiles of Q, profiles), Q energies x kSumThreads / Q segments of chunks.
+// Double-double sums: the exact sum to about 1e-32, in any order of the records, as the pool's compensated atomics
+// give it; what the atomics added is included.  Bound by the read of the node sums, from L2 for a single profile.
+template <typename T>
+__global__ void __launch_bounds__(kSumThreads) sum_parts_kernel(const KernelArgs a, int Q) {
   const RingWork& W = a.rings;
   const DevProfile& p = a.profiles[blockIdx.z];
-  const int bin = blockIdx.x, n_e = p.n_e;
-  const int ql = threadIdx.x % kSumQ, seg = threadIdx.x / kSumQ, q = blockIdx.y * kSumQ + ql;
-  if (bin >= p.n_bins || blockIdx.y * kSumQ >= n_e) return;
-  __shared__ int s_rec[kSumRecs], s_n;
-  __shared__ double s_s[kSumSegs][kSumQ], s_c[kSumSegs][kSumQ];
+  const int bin = blockIdx.x, n_e = p.n_e, segs = kSumThreads / Q;
+  const int ql = threadIdx.x % Q, seg = threadIdx.x / Q, q = blockIdx.y * Q + ql;
+  if (bin >= p.n_bins || blockIdx.y * Q >= n_e) return;
+  // the profile's (record, GL node) rows, in units of 4 bytes: the first spot's from the front, the second's from the
+  // back of the list
+  __shared__ unsigned s_ofs[kSumList];
+  __shared__ int s_n[kMaxSpots];
+  __shared__ double s_s[kSumThreads], s_c[kSumThreads];
   const int n_recs = min(*W.n_recs, min(W.rec_cap, W.part_cap));
-  const int e = q < n_e ? p.grid.perm[q] : 0;
+  const int e = q < n_e ? (std::is_same<T, float>::value ? p.grid.perm[q] : q) : 0;
   const double invE = q < n_e ? p.grid.invE[e] : 0.0;
   const int n_gl = max(p.n_gl, 1);
+  const double scale0 = p.spot[0].out_scale, scale1 = p.spot[1].out_scale;
+  const float* const src = (const float*)((const T*)W.parts + (size_t)bin * n_gl * n_e + min(q, n_e - 1));
   double s = 0.0, c = 0.0;
-  for (int r0 = 0; r0 < n_recs; r0 += kSumRecs) {
+  for (int r0 = 0; r0 < n_recs; r0 += kSumThreads) {
     __syncthreads();
-    if (threadIdx.x == 0) s_n = 0;
+    if (threadIdx.x < kMaxSpots) s_n[threadIdx.x] = 0;
     __syncthreads();
     const int r = r0 + (int)threadIdx.x;
-    if (r < n_recs && W.recs[r].profile == (int)blockIdx.z) s_rec[atomicAdd(&s_n, 1)] = r | W.recs[r].spot << 30;
-    __syncthreads();
-    const int n = s_n;
-    if (q < n_e)
-      for (int g = 0; g < n_gl; ++g) {
-        const float* src = W.parts + ((size_t)bin * n_gl + g) * n_e + q;
-#pragma unroll 4
-        for (int k = seg; k < n; k += kSumSegs) {
-          const float v = __ldcg(src + (size_t)(s_rec[k] & 0x3fffffff) * W.part_stride);
-          dd_add(s, c, __dmul_rn(__dmul_rn((double)v, p.spot[s_rec[k] >> 30].out_scale), invE));
-        }
-      }
-  }
-  s_s[seg][ql] = s;
-  s_c[seg][ql] = c;
-  __syncthreads();
-  if (seg == 0 && q < n_e) {
-    for (int k = 1; k < kSumSegs; ++k) {
-      dd_add(s, c, s_s[k][ql]);
-      c += s_c[k][ql];
+    if (r < n_recs && W.recs[r].profile == (int)blockIdx.z) {
+      const int sp = W.recs[r].spot, at = atomicAdd(&s_n[sp], n_gl);
+      for (int g = 0; g < n_gl; ++g)
+        s_ofs[sp ? kSumList - 1 - (at + g) : at + g] = (unsigned)(r * W.part_stride) + (unsigned)(g * n_e * (int)(sizeof(T) / 4));
     }
+    __syncthreads();
+    const int n0 = s_n[0], n = n0 + s_n[1];
+    for (int k0 = seg; k0 < n; k0 += kSumUnroll * segs) {
+      T v[kSumUnroll];  // (loads in flight together)
+#pragma unroll
+      for (int u = 0; u < kSumUnroll; ++u) {
+        const int k = k0 + u * segs;
+        v[u] = k < n ? __ldcg((const T*)(src + s_ofs[k < n0 ? k : kSumList - 1 - (k - n0)])) : (T)0;
+      }
+#pragma unroll
+      for (int u = 0; u < kSumUnroll; ++u)
+        dd_add(s, c, __dmul_rn(__dmul_rn((double)v[u], k0 + u * segs < n0 ? scale0 : scale1), invE));
+    }
+  }
+  s_s[threadIdx.x] = s;
+  s_c[threadIdx.x] = c;
+  for (int half = segs / 2; half > 0; half /= 2) {
+    __syncthreads();
+    if (seg < half) {
+      dd_add(s, c, s_s[threadIdx.x + half * Q]);
+      c += s_c[threadIdx.x + half * Q];
+      s_s[threadIdx.x] = s;
+      s_c[threadIdx.x] = c;
+    }
+  }
+  if (seg == 0 && q < n_e) {
     const size_t o = (size_t)p.flux_off + (size_t)bin * n_e + e;
     dd_add(s, c, a.flux[o]);
     c += a.comp[o];
@@ -2509,13 +2828,22 @@ __global__ void __launch_bounds__(kSumQ * kSumSegs) sum_parts_kernel(const Kerne
 }  // namespace
 
 cudaError_t launch_sum_parts(const KernelArgs& a, int bins_max, int ne_max, cudaStream_t st) {
-  sum_parts_kernel<<<dim3(bins_max, (ne_max + kSumQ - 1) / kSumQ, a.rings.n_profiles), kSumQ * kSumSegs, 0, st>>>(a);
+  int Q = 1;
+  while (Q < kSumQ && Q < ne_max) Q <<= 1;
+  const dim3 grid(bins_max, (ne_max + Q - 1) / Q, a.rings.n_profiles);
+  if (a.shape.nsx)
+    sum_parts_kernel<float><<<grid, kSumThreads, 0, st>>>(a, Q);
+  else
+    sum_parts_kernel<double><<<grid, kSumThreads, 0, st>>>(a, Q);
   return cudaGetLastError();
 }
 
 cudaError_t launch_rings(const KernelArgs& a, cudaStream_t st) {
   if (a.rings.n_jobs <= 0) return cudaSuccess;
-  ring_kernel<<<a.rings.n_jobs, 256, a.shape.ring_bytes, st>>>(a);
+  if (a.shape.nsx)
+    ring_kernel<true><<<a.rings.n_jobs, 256, a.shape.ring_bytes, st>>>(a);
+  else
+    ring_kernel<false><<<a.rings.n_jobs, 256, a.shape.ring_bytes, st>>>(a);
   return cudaGetLastError();
 }
 
