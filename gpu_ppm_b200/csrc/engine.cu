@@ -180,6 +180,8 @@ Engine::~Engine() {
   serve_shutdown();
   cudaStreamSynchronize(stream);
   block_cache.trim();
+  h_up.release();
+  h_down.release();
   if (d_err) cudaFree(d_err);
   for (void* p : owned) cudaFree(p);
   for (auto& kv : ring_tabs) cudaFree(kv.second);
@@ -697,14 +699,15 @@ void Engine::batch_build(BatchImpl& B, int n, const ppm_params* ps, cudaStream_t
   std::vector<long long> ring_off(n + 1, 0);
   for (int i = 0; i < n; ++i) ring_off[i + 1] = ring_off[i] + (long long)kMaxSpots * (4ll * ps[i].n_side / 32 + 1);
   B.ring_words = ring_off[n];
-  // the counters, the ring bits and the queue control words in one block (cleared by one memset per pass)
+  // the queue control words, the counters and the ring bits in one block (cleared by one memset per pass, the first
+  // two collected by one copy)
   const size_t stats_bytes = sizeof(unsigned long long) * kStats * (size_t)n;
   const size_t ring_bytes = (sizeof(unsigned) * (size_t)B.ring_words + 63) / 64 * 64;
   B.small_bytes = stats_bytes + ring_bytes + sizeof(int) * 16;
   unsigned char* small = (unsigned char*)B.mem.alloc(B.small_bytes);
-  B.d_stats = (unsigned long long*)small;
-  B.d_ring_seen = (unsigned*)(small + stats_bytes);
-  B.d_ctrl = (int*)(small + stats_bytes + ring_bytes);
+  B.d_ctrl = (int*)small;
+  B.d_stats = (unsigned long long*)(small + sizeof(int) * 16);
+  B.d_ring_seen = (unsigned*)(small + sizeof(int) * 16 + stats_bytes);
   std::vector<DevProfile> hp(n);
   GroupWork gw[NV];
   for (int k = 0; k < n; ++k) {
@@ -927,7 +930,7 @@ void Engine::batch_enqueue(BatchImpl& B, cudaStream_t st, cudaEvent_t* events) {
   if (!B.fused_points) {
     NvtxRange range("clear + plan");
     PPM_CUDA(cudaMemsetAsync(B.d_flux, 0, 2 * sizeof(double) * (size_t)std::max(1ll, B.flux_off[n]), st));
-    PPM_CUDA(cudaMemsetAsync(B.d_stats, 0, B.small_bytes, st));
+    PPM_CUDA(cudaMemsetAsync(B.d_ctrl, 0, B.small_bytes, st));
     for (const auto& G : B.groups)
       PPM_CUDA(G.args.shape.rec ? launch_rings(G.args, st) : launch_plan(B.d_prof + G.g0, G.g1 - G.g0, lens, G.args.queue, G.chunk, G.npt, st));
   }
@@ -1011,33 +1014,62 @@ void Engine::batch_launch(BatchImpl& B, cudaStream_t st) {
   B.last_stream = st;
 }
 
-void Engine::batch_collect(BatchImpl& B, double* flux, double* counts, ppm_result_info* info, cudaStream_t st) {
+// Uploads of a synchronous call's batch build from the engine's pinned area: asynchronous copies ordered on the
+// engine's stream.  The area is free again when the call returns (it has waited for the stream).
+void Engine::pin_uploads(BatchImpl& B) {
+  h_up.reserve(256 << 10);
+  B.h_upload = h_up.ptr;
+  B.h_upload_cap = h_up.cap;
+  B.last_stream = stream;  // waited for when the batch is destroyed, also by a build that fails half-way
+}
+
+void Engine::batch_collect(BatchImpl& B, double* flux, double* counts, ppm_result_info* info, cudaStream_t st,
+                           bool pinned) {
   NvtxRange range("collect");
   PPM_CUDA(cudaSetDevice(cfg.device));
   if (!st) st = B.last_stream ? B.last_stream : stream;
   const int n = B.n;
-  std::vector<unsigned long long> stats((size_t)kStats * n);
-  int ctrl[16];
-  if (flux)
-    PPM_CUDA(cudaMemcpyAsync(flux, B.d_flux, sizeof(double) * (size_t)B.flux_off[n], cudaMemcpyDeviceToHost, st));
-  if (counts && B.counts_off[n] > 0)
-    PPM_CUDA(cudaMemcpyAsync(counts, B.d_counts, sizeof(double) * (size_t)B.counts_off[n], cudaMemcpyDeviceToHost, st));
-  PPM_CUDA(cudaMemcpyAsync(stats.data(), B.d_stats, sizeof(unsigned long long) * stats.size(), cudaMemcpyDeviceToHost,
-                           st));
-  PPM_CUDA(cudaMemcpyAsync(ctrl, B.d_ctrl, sizeof(ctrl), cudaMemcpyDeviceToHost, st));
+  const size_t n_flux = flux ? sizeof(double) * (size_t)B.flux_off[n] : 0;
+  const size_t n_counts = counts ? sizeof(double) * (size_t)B.counts_off[n] : 0;
+  const size_t head = sizeof(int) * 16 + sizeof(unsigned long long) * kStats * (size_t)n;  // control words, counters
+  bool tc = false;  // a tensor-core fold may have set the error word
+  for (const auto& f : B.folds) tc |= f.mode == PPM_FOLD_BF16X3 && resps[f.resp].tc_ok;
+  // Small outputs go through pinned memory and one wait: each copy to pageable memory waits by itself (a light curve
+  // of one point source: 94 -> 52 us a call with the uploads').  Larger ones are bound by the copy out of it.
+  constexpr size_t kPinned = 1 << 20;
+  std::vector<unsigned char> pageable;
+  unsigned char* h;
+  const bool bounce = pinned && head + 64 + n_flux + n_counts <= kPinned;
+  if (bounce) {
+    h_down.reserve(kPinned);
+    h = (unsigned char*)h_down.ptr;
+  } else {
+    pageable.resize(head + 64);
+    h = pageable.data();
+  }
+  int* const err = (int*)(h + head);
+  *err = 0;
+  double* const to_flux = bounce ? (double*)(h + head + 64) : flux;
+  double* const to_counts = bounce ? to_flux + n_flux / sizeof(double) : counts;
+  if (n_flux) PPM_CUDA(cudaMemcpyAsync(to_flux, B.d_flux, n_flux, cudaMemcpyDeviceToHost, st));
+  if (n_counts) PPM_CUDA(cudaMemcpyAsync(to_counts, B.d_counts, n_counts, cudaMemcpyDeviceToHost, st));
+  PPM_CUDA(cudaMemcpyAsync(h, B.d_ctrl, head, cudaMemcpyDeviceToHost, st));
+  if (tc) PPM_CUDA(cudaMemcpyAsync(err, d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
   PPM_CUDA(cudaStreamSynchronize(st));
   PPM_CUDA(cudaGetLastError());
+  const int* ctrl = (const int*)h;
   if (ctrl[2] || ctrl[5] || ctrl[8] || ctrl[11] || ctrl[14]) throw Error(PPM_E_RANGE, "work queue overflow");
-  int err = 0;
-  PPM_CUDA(cudaMemcpy(&err, d_err, sizeof(int), cudaMemcpyDeviceToHost));
-  if (err) {
+  if (*err) {
     PPM_CUDA(cudaMemset(d_err, 0, sizeof(int)));
     throw Error(PPM_E_TIMEOUT, "a bounded wait in the tensor-core fold ran out");
   }
+  if (bounce && n_flux) std::memcpy(flux, to_flux, n_flux);
+  if (bounce && n_counts) std::memcpy(counts, to_counts, n_counts);
+  const unsigned long long* stats = (const unsigned long long*)(h + sizeof(int) * 16);
   if (info) {
     for (int i = 0; i < n; ++i) {
       ppm_result_info& r = info[i];
-      const unsigned long long* s = &stats[(size_t)kStats * i];
+      const unsigned long long* s = stats + (size_t)kStats * i;
       r.n_active = (int64_t)(s[0] + s[5]);
       r.n_rings = (int64_t)s[1];
       r.n_dropped_rings = (int64_t)s[2];
@@ -1055,10 +1087,10 @@ void Engine::profile(const ppm_params& p, double* flux, double* counts, ppm_resu
   std::lock_guard<std::mutex> lk(mu);
   if (counts && p.response < 0) throw Error(PPM_E_INVALID, "counts requested without a response");
   BatchImpl B;
-  batch_build(B, 1, &p);
+  pin_uploads(B);
+  batch_build(B, 1, &p, stream);
   batch_enqueue(B, stream, nullptr);  // plain form: direct launches, no graph
-  B.last_stream = stream;
-  batch_collect(B, flux, counts, info, stream);
+  batch_collect(B, flux, counts, info, stream, true);
 }
 
 // HEALPix elements in a profile's spots (disk 1 areas over the element area,
@@ -1209,20 +1241,20 @@ void Engine::profile_rings(const ppm_params& p, int ring_begin, int ring_end, do
   std::lock_guard<std::mutex> lk(mu);
   if (counts && p.response < 0) throw Error(PPM_E_INVALID, "counts requested without a response");
   BatchImpl B;
-  batch_build(B, 1, &p, nullptr, ring_begin, ring_end);
+  pin_uploads(B);
+  batch_build(B, 1, &p, stream, ring_begin, ring_end);
   batch_enqueue(B, stream, nullptr);
-  B.last_stream = stream;
-  batch_collect(B, flux, counts, info, stream);
+  batch_collect(B, flux, counts, info, stream, true);
 }
 
 void Engine::profile_batch(int n, const ppm_params* ps, double* flux, double* counts, ppm_result_info* info) {
   NvtxRange range("ppm_profile_batch");
   std::lock_guard<std::mutex> lk(mu);
   BatchImpl B;
-  batch_build(B, n, ps);
+  pin_uploads(B);
+  batch_build(B, n, ps, stream);
   batch_enqueue(B, stream, nullptr);
-  B.last_stream = stream;
-  batch_collect(B, flux, counts, info, stream);
+  batch_collect(B, flux, counts, info, stream, true);
 }
 
 IntegrandShape Engine::choose_shape(bool nsx_kernel, bool bb_fp64, int ne_max, int nf_max, int cells_max, int maxe_max,

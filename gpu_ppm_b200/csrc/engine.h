@@ -255,7 +255,9 @@ class Engine {
   void batch_enqueue(BatchImpl& B, cudaStream_t st, cudaEvent_t* events);
   void batch_capture(BatchImpl& B);
   void batch_launch(BatchImpl& B, cudaStream_t st);
-  void batch_collect(BatchImpl& B, double* flux, double* counts, ppm_result_info* info, cudaStream_t st);
+  // pinned: through the engine's pinned area where the outputs fit (callers that hold the engine lock until the end)
+  void batch_collect(BatchImpl& B, double* flux, double* counts, ppm_result_info* info, cudaStream_t st,
+                     bool pinned = false);
   int kernels_per_pass(const BatchImpl& B) const;
   void batch_launch_timed(BatchImpl& B, cudaStream_t st, float* ms);
   void output_sizes(const ppm_params& p, int64_t* n_flux, int64_t* n_counts) const;
@@ -320,6 +322,10 @@ class Engine {
   std::vector<Resp> resps;
   std::vector<Observed> observed;
   BlockCache block_cache;
+  // pinned areas of the synchronous calls, made at the first one, used under the lock: the batch build's uploads, the
+  // outputs of small calls
+  HostBuffer h_up, h_down;
+  void pin_uploads(BatchImpl& B);
   std::map<int, double*> ring_tabs, fine_tabs;
   std::map<int, std::vector<double>> host_rings;
   std::vector<void*> owned;

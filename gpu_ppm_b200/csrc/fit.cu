@@ -138,11 +138,11 @@ void Engine::batch_fit(BatchImpl& B, int obs, ppm_fit* out, cudaStream_t st) {
 void Engine::profile_fit(const ppm_params& p, int obs, ppm_fit* out, ppm_result_info* info) {
   std::lock_guard<std::mutex> lk(mu);
   BatchImpl B;
-  batch_build(B, 1, &p);
+  pin_uploads(B);
+  batch_build(B, 1, &p, stream);
   batch_enqueue(B, stream, nullptr);
-  B.last_stream = stream;
   batch_fit(B, obs, out, stream);
-  batch_collect(B, nullptr, nullptr, info, stream);
+  batch_collect(B, nullptr, nullptr, info, stream, true);
 }
 
 }  // namespace ppm

@@ -28,7 +28,9 @@
 #include <climits>
 #include <cstdint>
 #include <cstdio>
+#include <map>
 #include <mutex>
+#include <tuple>
 #include <type_traits>
 
 #include "kernels.cuh"
@@ -2718,9 +2720,22 @@ cudaError_t set_integrand_smem() {
 cudaError_t configure_integrand_smem(const IntegrandShape&) { return once_per_device(0, set_integrand_smem); }
 
 int max_active_ctas(const IntegrandShape& s) {
-  int n = 0;
+  // the occupancy query costs as much as a launch: the answers are kept, one for each kernel and launch size
+  static std::mutex m;
+  static std::map<std::tuple<int, void*, int, int>, int> known;
+  int n = 0, dev = 0;
   void* f = kernel_for(s, s.bb_fp64);
+  if (!f || cudaGetDevice(&dev) != cudaSuccess) return 0;
+  const auto key = std::make_tuple(dev, f, s.nt, s.total);
+  {
+    std::lock_guard<std::mutex> lk(m);
+    const auto it = known.find(key);
+    if (it != known.end()) return it->second;
+  }
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, f, s.nt, s.total) != cudaSuccess) return 0;
+  std::lock_guard<std::mutex> lk(m);
+  if (known.size() > 1024) known.clear();
+  known[key] = n;
   return n;
 }
 
