@@ -174,6 +174,8 @@ struct BatchImpl {
   bool fused_points = false;
   long long* d_fit_off = nullptr;  // counts offset per profile (fit statistics)
   ppm_fit* d_fit = nullptr;
+  void* d_fit_parts = nullptr;     // the blocks' partial sums and their counters
+  int* d_fit_done = nullptr;
   BatchImpl() = default;
   BatchImpl(const BatchImpl&) = delete;
   BatchImpl& operator=(const BatchImpl&) = delete;

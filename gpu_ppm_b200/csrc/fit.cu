@@ -5,6 +5,7 @@
 // instead of the [n_ch][n_bins] count arrays.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <string>
 #include <vector>
@@ -23,20 +24,34 @@ namespace {
   } while (0)
 
 constexpr int kFitThreads = 256;
+constexpr int kFitPerBlock = 1024, kFitMaxBlocks = 32;
 
-// One CTA per profile.  Per-thread partial sums over a fixed stride, then a
-// fixed-order warp and block reduction: the result does not depend on timing.
+// What one block sums of a profile's entries.
+struct FitPart {
+  double M, S, L;
+  long long nz;
+  int bad;
+};
+
+// Blocks of a profile: by its number of entries alone, so that its statistics do not depend on what it is batched with.
+int fit_blocks(int n_el) { return std::max(1, std::min(kFitMaxBlocks, (n_el + kFitPerBlock - 1) / kFitPerBlock)); }
+
+// grid (blocks, profiles).  Per-thread partial sums over a fixed stride, a
+// fixed-order warp and block reduction; the block that finishes a profile's last
+// part adds the parts in their order: the result does not depend on timing.
+// Bound by the latency of the FP64 logarithm: 300 x 64 entries took 53 us on one
+// block, 15 on five, 11 on the 19 that 1024 entries a block give.  done: zero before, zero after.
 __global__ void __launch_bounds__(kFitThreads) fit_kernel(const long long* counts_off, const double* counts,
                                                           const double* obs, int n_el, double lgamma_sum,
-                                                          ppm_fit* out) {
+                                                          FitPart* parts, int* done, ppm_fit* out) {
   __shared__ double s_red[3][kFitThreads / 32];
   __shared__ long long s_nz[kFitThreads / 32];
   __shared__ int s_bad[kFitThreads / 32];
-  const double* m = counts + counts_off[blockIdx.x];
+  const double* m = counts + counts_off[blockIdx.y];
   double M = 0.0, S = 0.0, L = 0.0;
   long long nz = 0;
   int bad = 0;
-  for (int i = threadIdx.x; i < n_el; i += kFitThreads) {
+  for (int i = blockIdx.x * kFitThreads + threadIdx.x; i < n_el; i += gridDim.x * kFitThreads) {
     const double mi = m[i], di = obs[i];
     M += mi;
     if (mi > 0.0) {
@@ -66,22 +81,35 @@ __global__ void __launch_bounds__(kFitThreads) fit_kernel(const long long* count
   }
   __syncthreads();
   if (threadIdx.x == 0) {
-    M = S = L = 0.0;
-    nz = 0;
-    bad = 0;
+    FitPart t{0.0, 0.0, 0.0, 0, 0};
     for (int w = 0; w < kFitThreads / 32; ++w) {
-      M += s_red[0][w];
-      S += s_red[1][w];
-      L += s_red[2][w];
-      nz += s_nz[w];
-      bad |= s_bad[w];
+      t.M += s_red[0][w];
+      t.S += s_red[1][w];
+      t.L += s_red[2][w];
+      t.nz += s_nz[w];
+      t.bad |= s_bad[w];
+    }
+    FitPart* mine = parts + (size_t)blockIdx.y * gridDim.x;
+    mine[blockIdx.x] = t;
+    __threadfence();
+    if (atomicAdd(&done[blockIdx.y], 1) != (int)gridDim.x - 1) return;
+    __threadfence();
+    done[blockIdx.y] = 0;
+    t = FitPart{0.0, 0.0, 0.0, 0, 0};
+    for (int k = 0; k < (int)gridDim.x; ++k) {
+      const volatile FitPart* p = mine + k;
+      t.M += p->M;
+      t.S += p->S;
+      t.L += p->L;
+      t.nz += p->nz;
+      t.bad |= p->bad;
     }
     ppm_fit f;
-    f.chi2 = M > 0.0 ? S * (1e6 / M) : (double)NAN;
-    f.loglike = bad ? -(double)INFINITY : L - lgamma_sum;
-    f.model_total = M;
-    f.n_zero_model = nz;
-    out[blockIdx.x] = f;
+    f.chi2 = t.M > 0.0 ? t.S * (1e6 / t.M) : (double)NAN;
+    f.loglike = t.bad ? -(double)INFINITY : t.L - lgamma_sum;
+    f.model_total = t.M;
+    f.n_zero_model = t.nz;
+    out[blockIdx.y] = f;
   }
 }
 
@@ -120,15 +148,23 @@ void Engine::batch_fit(BatchImpl& B, int obs, ppm_fit* out, cudaStream_t st) {
       throw Error(PPM_E_INVALID, "profile " + std::to_string(i) +
                                      " does not use the observed data's response and bin count");
   if (!st) st = B.last_stream ? B.last_stream : stream;
+  const int n_el = o.n_ch * o.n_bins;  // the same for every set of observed data this batch takes
+  const int blocks = fit_blocks(n_el);
   if (!B.d_fit) {
     B.d_fit_off = (long long*)B.mem.alloc(sizeof(long long) * (size_t)B.n);
     B.d_fit = (ppm_fit*)B.mem.alloc(sizeof(ppm_fit) * (size_t)B.n);
+    B.d_fit_parts = B.mem.alloc((sizeof(FitPart) * blocks + sizeof(int)) * (size_t)B.n);
+    B.d_fit_done = (int*)((FitPart*)B.d_fit_parts + (size_t)blocks * B.n);
     FIT_CUDA(cudaMemcpyAsync(B.d_fit_off, B.counts_off.data(), sizeof(long long) * (size_t)B.n,
                              cudaMemcpyHostToDevice, st));
+    FIT_CUDA(cudaMemsetAsync(B.d_fit_done, 0, sizeof(int) * (size_t)B.n, st));
   }
   if (B.n > 0) {
-    fit_kernel<<<B.n, kFitThreads, 0, st>>>(B.d_fit_off, B.d_counts, o.d_counts, o.n_ch * o.n_bins, o.lgamma_sum,
-                                             B.d_fit);
+    // (at most 65535 profiles a launch: grid y)
+    for (int k = 0; k < B.n; k += 65535)
+      fit_kernel<<<dim3(blocks, std::min(65535, B.n - k)), kFitThreads, 0, st>>>(
+          B.d_fit_off + k, B.d_counts, o.d_counts, n_el, o.lgamma_sum, (FitPart*)B.d_fit_parts + (size_t)k * blocks,
+          B.d_fit_done + k, B.d_fit + k);
     FIT_CUDA(cudaGetLastError());
     FIT_CUDA(cudaMemcpyAsync(out, B.d_fit, sizeof(ppm_fit) * (size_t)B.n, cudaMemcpyDeviceToHost, st));
   }
