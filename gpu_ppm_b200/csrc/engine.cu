@@ -950,15 +950,17 @@ void Engine::batch_enqueue(BatchImpl& B, cudaStream_t st, cudaEvent_t* events) {
   }
   if (events) PPM_CUDA(cudaEventRecord(events[2], st));
   NvtxRange fold_range("fold");
+  std::vector<TcFold> tc;
   for (const auto& f : B.folds) {
     const Resp& r = resps[f.resp];
     const FoldJob* jobs = B.d_jobs + f.job0;
     if (f.mode == PPM_FOLD_BF16X3 && r.tc_ok)
-      PPM_CUDA(fold_tc_launch(r, jobs, f.n_jobs, f.n_bins, B.d_flux, B.d_counts, st));
+      tc.push_back(TcFold{f.resp, jobs, f.n_jobs, f.n_bins});
     else
       PPM_CUDA(launch_fold_simt(jobs, f.n_jobs, r.d_rsp, r.n_ch, r.n_e, f.n_bins, B.d_flux, B.d_counts,
                                 f.mode != PPM_FOLD_FP32, st));
   }
+  if (!tc.empty()) PPM_CUDA(fold_tc_launch(tc.data(), (int)tc.size(), B.d_flux, B.d_counts, st));
   if (events) PPM_CUDA(cudaEventRecord(events[3], st));
 }
 
@@ -973,9 +975,12 @@ void Engine::batch_launch_timed(BatchImpl& B, cudaStream_t st, float* ms) {
 }
 
 int Engine::kernels_per_pass(const BatchImpl& B) const {
-  if (B.fused_points) return 1 + (int)B.folds.size();          // the fused integrand, folds
+  int folds = 0, tc = 0;  // tensor-core folds share launches
+  for (const auto& f : B.folds) (f.mode == PPM_FOLD_BF16X3 && resps[f.resp].tc_ok ? tc : folds) += 1;
+  folds += (tc + 15) / 16;
+  if (B.fused_points) return 1 + folds;  // the fused integrand, folds
   // per group the plan (or rings) and the integrand, and the sum of the node sums; add_comp for the others; folds
-  int n = (int)B.folds.size(), pool = 0;
+  int n = folds, pool = 0;
   for (const auto& G : B.groups) {
     n += G.args.shape.rec ? 3 : 2;
     pool |= G.args.shape.rec ? 0 : 1;
@@ -1429,9 +1434,10 @@ void Engine::fold(int resp, int mode, int n_prof, int n_bins, const double* alph
   }
   FoldJob* d_jobs = (FoldJob*)mem.alloc(sizeof(FoldJob) * jobs.size());
   PPM_CUDA(cudaMemcpyAsync(d_jobs, jobs.data(), sizeof(FoldJob) * jobs.size(), cudaMemcpyHostToDevice, st));
-  if (mode == PPM_FOLD_BF16X3 && r.tc_ok)
-    PPM_CUDA(fold_tc_launch(r, d_jobs, n_prof, n_bins, d_flux, d_counts, st));
-  else
+  if (mode == PPM_FOLD_BF16X3 && r.tc_ok) {
+    const TcFold f{resp, d_jobs, n_prof, n_bins};
+    PPM_CUDA(fold_tc_launch(&f, 1, d_flux, d_counts, st));
+  } else
     PPM_CUDA(launch_fold_simt(d_jobs, n_prof, r.d_rsp, r.n_ch, r.n_e, n_bins, d_flux, d_counts, mode != PPM_FOLD_FP32,
                               st));
   if (!device) {

@@ -309,9 +309,15 @@ class Engine {
   static bool rec_shape(IntegrandShape& s, const RingWork& W);
   long long tile_bound(const ppm_params& p, const DevProfile& d, int chunk, int npt) const;
   void fold_tc_prepare(Resp& r);
-  // error: word the kernel sets when a bounded wait runs out (nullptr = the engine's d_err)
-  cudaError_t fold_tc_launch(const Resp& r, const FoldJob* jobs, int n_jobs, int n_bins, const double* flux,
-                             double* counts, cudaStream_t st, int* error = nullptr);
+  // tensor-core folds of one flux and counts pool, up to 16 a launch.  error: word the kernel sets when a bounded
+  // wait runs out (nullptr = the engine's d_err)
+  struct TcFold {
+    int resp;
+    const FoldJob* jobs;
+    int n_jobs, n_bins;
+  };
+  cudaError_t fold_tc_launch(const TcFold* list, int n_list, const double* flux, double* counts, cudaStream_t st,
+                             int* error = nullptr);
   void track(void* p);
 
   std::mutex mu;

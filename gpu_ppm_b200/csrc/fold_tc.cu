@@ -18,12 +18,21 @@
 //     bulk copy (TMA) per chunk and part;
 //   * the flux rows (A) are loaded by all threads with coalesced 16-byte loads
 //     (four threads per row, eight rows per warp), two chunks ahead in
-//     registers, split to BF16 hi/lo and stored into the same layout;
+//     registers, split to BF16 hi/lo and stored into the same layout.  With
+//     each load's four threads on 64 consecutive bytes (they were 64 bytes
+//     apart) and the FP64 values narrowed on the integer pipe, 65 536 rows of
+//     300 energies into 300 channels take 105 us instead of 109.  Latency
+//     bounds it: on a form with a separate issuing warp, not kept (121 us), the
+//     kernel without its loads took 88, without its stores 99, with a third of
+//     the products 119;
 //   * two shared-memory stages of A and B: while the tensor cores multiply
 //     chunk c, the threads convert chunk c + 1 and the loads of chunk c + 2
 //     and the bulk copy of chunk c + 1 are in flight.  Copies and MMAs
 //     complete on separate mbarriers; one elected thread issues 2 k-steps x 3
 //     products of tcgen05.mma.cta_group::1.kind::f16 per chunk;
+//   * the folds of a pass (one per response and bin count) share launches of up
+//     to 16: a fold of a few profiles takes about 20 us, whatever its size, on a
+//     few SMs (ten folds of 24 profiles: 180 -> 27 us);
 //   * every wait has an iteration limit; a wait that runs out sets an error
 //     word, and the CTA waits (bounded) for its own copies and MMAs in flight,
 //     releases its tensor memory and returns;
@@ -35,6 +44,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <climits>
 #include <cstdint>
 #include <cstdlib>
 #include <cstring>
@@ -59,6 +69,7 @@ __host__ __device__ constexpr int b_part_bytes(int ng) { return ng * TC_KC * 2; 
 // dynamic shared memory of a launch: two stages of A (hi, lo) and B (hi, lo), 1 KB alignment slack
 __host__ __device__ constexpr int fold_smem_bytes(int ng) { return 1024 + 2 * (2 * A_PART) + 2 * (2 * b_part_bytes(ng)); }
 constexpr int SMEM_MAX = fold_smem_bytes(TC_NMAX);
+constexpr int TC_FOLDS = 16;  // folds per launch
 
 __host__ __device__ constexpr uint32_t idesc(int n) {
   return (1u << 4)                         // D: FP32
@@ -99,12 +110,6 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int lim
   return false;
 }
 
-__device__ __forceinline__ uint32_t bf16_bits(__nv_bfloat16 h) {
-  uint16_t u;
-  memcpy(&u, &h, 2);
-  return u;
-}
-
 struct TcArgs {
   const uint16_t* b_hi;  // [groups][k_chunks][ng x TC_KC] core-matrix layout
   const uint16_t* b_lo;
@@ -116,46 +121,77 @@ struct TcArgs {
   // failure-path test: > 0 issues no bulk copy and no MMA and waits at most this many
   // polls, so the first wait runs out and the kernel reports it through *error
   int stall_wait_limit;
+  int groups, first;  // channel groups, first block of the fold in its launch
+};
+struct TcFolds {
+  int n;
+  TcArgs fold[TC_FOLDS];
 };
 
-// Eight consecutive energies k0 .. k0 + 7 of one flux row (zeros past n_e or for no row).
+// A thread's eight energies of a chunk of one flux row: k0 + 8 i and the next, i = 0 .. 3, with k0 = 2 (lane & 3) past
+// the chunk's start, so that four lanes read 64 consecutive bytes and a load of a warp touches each line once (zeros
+// past n_e or for no row).
 struct Row8 {
   double v[8];
 };
 __device__ __forceinline__ void load_row8(const double* src, bool vec, int k0, int n_e, Row8& r) {
-  if (src && vec && k0 + 8 <= n_e) {
-    const double2* p = reinterpret_cast<const double2*>(src + k0);
+  if (src && vec && k0 + 26 <= n_e) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const double2 t = __ldg(p + i);
+      const double2 t = __ldg(reinterpret_cast<const double2*>(src + k0 + 8 * i));
       r.v[2 * i] = t.x;
       r.v[2 * i + 1] = t.y;
     }
   } else {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) r.v[i] = (src && k0 + i < n_e) ? __ldg(src + k0 + i) : 0.0;
+    for (int i = 0; i < 8; ++i) {
+      const int k = k0 + 8 * (i >> 1) + (i & 1);
+      r.v[i] = (src && k < n_e) ? __ldg(src + k) : 0.0;
+    }
   }
 }
 
-// Splits eight values into BF16 hi / lo parts and stores them as one 16-byte
-// row of a core matrix in each part.
+// d rounded to the nearest FP32 value (ties to even) where that is a normal number, or d is zero or subnormal; ok is
+// left alone then and cleared otherwise.  On the integer pipe, which has room: the conversion instruction runs on the
+// special-function pipe, 35 % of whose issue the kernel took (12 % with this).
+__device__ __forceinline__ float narrow(double d, bool& ok) {
+  const uint32_t hi = (uint32_t)__double2hiint(d), lo = (uint32_t)__double2loint(d), mag = hi & 0x7fffffffu;
+  uint32_t t = __funnelshift_l(lo, hi, 3);  // 23 bits of the significand under 9 of the exponent
+  // round up when the 29 bits below are above half, or half and t is odd; exponent bias 1023 -> 127
+  const uint32_t rest = (lo << 3) | (t & 1u);
+  uint32_t unused;
+  asm("add.cc.u32 %0, %2, 0x7fffffff;\n\taddc.u32 %1, %3, 0x40000000;" : "=r"(unused), "=r"(t) : "r"(rest), "r"(t));
+  (void)unused;
+  if (mag < 0x00100000u) t = 0;
+  ok = ok && (mag < 0x00100000u || mag - 0x38100000u < 0x0fe00000u);
+  return __uint_as_float((t & 0x7fffffffu) | (hi & 0x80000000u));
+}
+
+// Splits eight values into BF16 hi / lo parts and stores them, two to a core matrix row of each part.
 __device__ __forceinline__ void store_row8(const Row8& r, unsigned char* hi, unsigned char* lo, uint32_t off) {
-  uint32_t h[4], l[4];
+  float f[8];
+  bool ok = true;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) f[i] = narrow(r.v[i], ok);
+  if (!ok) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) f[i] = (float)r.v[i];
+  }
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const float a = (float)r.v[2 * i], b = (float)r.v[2 * i + 1];
-    const __nv_bfloat16 ha = __float2bfloat16_rn(a), hb = __float2bfloat16_rn(b);
-    const __nv_bfloat16 la = __float2bfloat16_rn(a - __bfloat162float(ha)),
-                        lb = __float2bfloat16_rn(b - __bfloat162float(hb));
-    h[i] = bf16_bits(ha) | (bf16_bits(hb) << 16);
-    l[i] = bf16_bits(la) | (bf16_bits(lb) << 16);
+    const float a = f[2 * i], b = f[2 * i + 1];
+    const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+    const __nv_bfloat162 l = __floats2bfloat162_rn(a - __bfloat162float(h.x), b - __bfloat162float(h.y));
+    *(__nv_bfloat162*)(hi + off + i * LBO_A) = h;
+    *(__nv_bfloat162*)(lo + off + i * LBO_A) = l;
   }
-  *(uint4*)(hi + off) = make_uint4(h[0], h[1], h[2], h[3]);
-  *(uint4*)(lo + off) = make_uint4(l[0], l[1], l[2], l[3]);
 }
 
-__global__ void __launch_bounds__(TC_THREADS, 2) fold_tc_kernel(const TcArgs a) {
+__global__ void __launch_bounds__(TC_THREADS, 2) fold_tc_kernel(const __grid_constant__ TcFolds all) {
   extern __shared__ unsigned char sm_raw[];
+  int f = 0;
+  while (f + 1 < all.n && (int)blockIdx.x >= all.fold[f + 1].first) ++f;
+  const TcArgs& a = all.fold[f];
   unsigned char* sm = (unsigned char*)(((uintptr_t)sm_raw + 1023) & ~(uintptr_t)1023);
   const int b_part = b_part_bytes(a.ng);
   // stage s: A hi, A lo, then B hi, B lo
@@ -165,8 +201,9 @@ __global__ void __launch_bounds__(TC_THREADS, 2) fold_tc_kernel(const TcArgs a) 
   __shared__ uint32_t s_tmem;
   __shared__ int s_ok;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int grp = blockIdx.x;
-  const int n0 = blockIdx.y * TC_M;
+  const int blk = (int)blockIdx.x - a.first;
+  const int grp = blk % a.groups;
+  const int n0 = blk / a.groups * TC_M;
   const int rows_total = a.n_jobs * a.n_bins;
   const int nk = a.k_chunks;
   const bool stall = a.stall_wait_limit > 0;
@@ -208,11 +245,12 @@ __global__ void __launch_bounds__(TC_THREADS, 2) fold_tc_kernel(const TcArgs a) 
     }
   }
   const bool vec0 = ((uintptr_t)src0 & 15) == 0, vec1 = ((uintptr_t)src1 & 15) == 0;
-  const uint32_t off0 = cm_offset(rl0, 8 * kg, TC_M), off1 = cm_offset(rl1, 8 * kg, TC_M);
+  const uint32_t off0 = cm_offset(rl0, 2 * kg, TC_M), off1 = cm_offset(rl1, 2 * kg, TC_M);
 
-  // bulk copy of the response chunk kc into stage s (elected thread)
+  // bulk copy of the response chunk kc into stage kc mod 2 (elected thread)
   const size_t b_blk = (size_t)b_part / 2;  // uint16 elements per part and chunk
-  auto issue_b = [&](int kc, int s) {
+  auto issue_b = [&](int kc) {
+    const int s = kc & 1;
     const uint32_t bar = smem_u32(&bar_b[s]);
     unsigned char* dst = sB0 + s * 2 * b_part;
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(2 * b_part) : "memory");
@@ -226,25 +264,19 @@ __global__ void __launch_bounds__(TC_THREADS, 2) fold_tc_kernel(const TcArgs a) 
                  "l"(a.b_lo + blk), "r"(b_part), "r"(bar)
                  : "memory");
   };
-  // the elected thread's bookkeeping: copies issued and not yet waited for, last chunk multiplied
-  bool b_pending0 = false, b_pending1 = false;
+  // the elected thread's bookkeeping: chunks whose copies were issued and waited for, last chunk multiplied
+  int b_issued = 0, b_waited = 0;
   int mma_issued = -1;
 
-  if (tid == 0 && !stall) {
-    issue_b(0, 0);
-    b_pending0 = true;
-    if (nk > 1) {
-      issue_b(1, 1);
-      b_pending1 = true;
-    }
-  }
+  if (tid == 0 && !stall)
+    for (; b_issued < min(2, nk); ++b_issued) issue_b(b_issued);
   // two register sets of flux rows: chunk c lives in set c & 1 until it is converted
   Row8 ra0, ra1, rb0, rb1;  // set 0 rows 0/1, set 1 rows 0/1
-  load_row8(src0, vec0, 8 * kg, a.n_e, ra0);
-  load_row8(src1, vec1, 8 * kg, a.n_e, ra1);
+  load_row8(src0, vec0, 2 * kg, a.n_e, ra0);
+  load_row8(src1, vec1, 2 * kg, a.n_e, ra1);
   if (nk > 1) {
-    load_row8(src0, vec0, TC_KC + 8 * kg, a.n_e, rb0);
-    load_row8(src1, vec1, TC_KC + 8 * kg, a.n_e, rb1);
+    load_row8(src0, vec0, TC_KC + 2 * kg, a.n_e, rb0);
+    load_row8(src1, vec1, TC_KC + 2 * kg, a.n_e, rb1);
   }
 
   const uint32_t id = idesc(a.ng);
@@ -258,8 +290,8 @@ __global__ void __launch_bounds__(TC_THREADS, 2) fold_tc_kernel(const TcArgs a) 
     store_row8(r0, ahi, alo, off0);
     store_row8(r1, ahi, alo, off1);
     if (c + 2 < nk) {
-      load_row8(src0, vec0, (c + 2) * TC_KC + 8 * kg, a.n_e, r0);
-      load_row8(src1, vec1, (c + 2) * TC_KC + 8 * kg, a.n_e, r1);
+      load_row8(src0, vec0, (c + 2) * TC_KC + 2 * kg, a.n_e, r0);
+      load_row8(src1, vec1, (c + 2) * TC_KC + 2 * kg, a.n_e, r1);
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();
@@ -267,7 +299,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2) fold_tc_kernel(const TcArgs a) 
       const bool ok = s_ok && mbar_wait(smem_u32(&bar_b[s]), (uint32_t)(c >> 1) & 1u, wait_limit);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       if (ok) {
-        if (s) b_pending1 = false; else b_pending0 = false;
+        b_waited = c + 1;
         const uint32_t ah = smem_u32(ahi), al = smem_u32(alo), bh = smem_u32(bhi), bl = smem_u32(bhi + b_part);
 #pragma unroll
         for (int ks = 0; ks < TC_KC / 16; ++ks) {
@@ -298,10 +330,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2) fold_tc_kernel(const TcArgs a) 
     // stage s ^ 1 is free once the MMAs of chunk c - 1 are done: then chunk c + 1's copy may land there
     if (c >= 1) {
       if (!mbar_wait(smem_u32(&bar_mma[s ^ 1]), (uint32_t)((c - 1) >> 1) & 1u, wait_limit)) s_ok = 0;
-      if (tid == 0 && s_ok && c + 1 < nk) {
-        issue_b(c + 1, s ^ 1);
-        if (s) b_pending0 = true; else b_pending1 = true;
-      }
+      if (tid == 0 && s_ok && b_issued < nk) issue_b(b_issued++);
     }
     return true;
   };
@@ -349,16 +378,10 @@ __global__ void __launch_bounds__(TC_THREADS, 2) fold_tc_kernel(const TcArgs a) 
       }
     }
   } else if (tid == 0) {
-    // a wait ran out: record it, then give this CTA's copies and MMAs in flight one more bounded wait.  A
-    // pending copy of stage s carries the first chunk of that stage not yet multiplied: chunk kc lands in
-    // stage kc & 1 with phase parity (kc >> 1) & 1.
+    // a wait ran out: record it, then give this CTA's copies and MMAs in flight one more bounded wait (chunk kc
+    // lands in stage kc mod 2 with phase parity kc / 2)
     atomicExch(a.error, 1);
-    for (int s = 0; s < 2; ++s)
-      if (s ? b_pending1 : b_pending0) {
-        int kc = s;
-        while (kc <= mma_issued) kc += 2;
-        mbar_wait(smem_u32(&bar_b[s]), (uint32_t)(kc >> 1) & 1u, kWaitLimit);
-      }
+    for (int kc = b_waited; kc < b_issued; ++kc) mbar_wait(smem_u32(&bar_b[kc & 1]), (uint32_t)(kc >> 1) & 1u, kWaitLimit);
     if (mma_issued >= 0) mbar_wait(smem_u32(&bar_mma[mma_issued & 1]), (uint32_t)(mma_issued >> 1) & 1u, kWaitLimit);
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -438,38 +461,58 @@ void Engine::fold_tc_prepare(Resp& r) {
   r.tc_ok = true;
 }
 
-cudaError_t Engine::fold_tc_launch(const Resp& r, const FoldJob* jobs, int n_jobs, int n_bins, const double* flux,
-                                   double* counts, cudaStream_t st, int* error) {
+cudaError_t Engine::fold_tc_launch(const TcFold* list, int n_list, const double* flux, double* counts, cudaStream_t st,
+                                   int* error) {
   cudaError_t e = once_per_device(1, [] {
     return cudaFuncSetAttribute(fold_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX);
   });
   if (e != cudaSuccess) return e;
-  TcArgs a{};
-  a.b_hi = (const uint16_t*)r.d_b_hi;
-  a.b_lo = (const uint16_t*)r.d_b_lo;
-  a.n_ch = r.n_ch;
-  a.n_e = r.n_e;
-  a.ng = r.tc_ng;
-  a.k_chunks = r.tc_k_chunks;
-  a.n_bins = n_bins;
-  a.flux = flux;
-  a.counts = counts;
-  a.error = error ? error : d_err;
   // PPM_FOLD_TC_STALL_TEST=<polls>: the failure-path test of the bounded waits (no copy or MMA is issued, so the
   // first wait runs out after that many polls and the call reports PPM_E_TIMEOUT)
-  if (const char* v = std::getenv("PPM_FOLD_TC_STALL_TEST")) a.stall_wait_limit = std::max(0, std::atoi(v));
-  // at most 65535 row tiles per launch (grid y): longer job lists go in several launches
-  const int jobs_per_launch = std::max(1, (int)(65535ll * TC_M / n_bins));
-  for (int j0 = 0; j0 < n_jobs; j0 += jobs_per_launch) {
-    a.jobs = jobs + j0;
-    a.n_jobs = std::min(jobs_per_launch, n_jobs - j0);
-    const long long rows = (long long)a.n_jobs * n_bins;
-    dim3 grid(r.tc_groups, (unsigned)((rows + TC_M - 1) / TC_M));
-    fold_tc_kernel<<<grid, TC_THREADS, fold_smem_bytes(r.tc_ng), st>>>(a);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
+  int stall = 0;
+  if (const char* v = std::getenv("PPM_FOLD_TC_STALL_TEST")) stall = std::max(0, std::atoi(v));
+  TcFolds all{};
+  long long blocks = 0;
+  auto launch = [&]() -> cudaError_t {
+    if (all.n == 0) return cudaSuccess;
+    int smem = 0;
+    for (int k = 0; k < all.n; ++k) smem = std::max(smem, fold_smem_bytes(all.fold[k].ng));
+    fold_tc_kernel<<<(unsigned)blocks, TC_THREADS, smem, st>>>(all);
+    all.n = 0;
+    blocks = 0;
+    return cudaGetLastError();
+  };
+  for (int k = 0; k < n_list; ++k) {
+    const Resp& r = resps[list[k].resp];
+    TcArgs a{};
+    a.b_hi = (const uint16_t*)r.d_b_hi;
+    a.b_lo = (const uint16_t*)r.d_b_lo;
+    a.n_ch = r.n_ch;
+    a.n_e = r.n_e;
+    a.ng = r.tc_ng;
+    a.groups = r.tc_groups;
+    a.k_chunks = r.tc_k_chunks;
+    a.n_bins = list[k].n_bins;
+    a.flux = flux;
+    a.counts = counts;
+    a.error = error ? error : d_err;
+    a.stall_wait_limit = stall;
+    // rows as 32-bit numbers: longer job lists go in several folds
+    const int jobs_per_fold = std::max(1, (1 << 30) / list[k].n_bins);
+    for (int j0 = 0; j0 < list[k].n_jobs; j0 += jobs_per_fold) {
+      a.jobs = list[k].jobs + j0;
+      a.n_jobs = std::min(jobs_per_fold, list[k].n_jobs - j0);
+      const long long n = ((long long)a.n_jobs * a.n_bins + TC_M - 1) / TC_M * a.groups;
+      if (all.n == TC_FOLDS || blocks + n > INT_MAX) {
+        e = launch();
+        if (e != cudaSuccess) return e;
+      }
+      a.first = (int)blocks;
+      all.fold[all.n++] = a;
+      blocks += n;
+    }
   }
-  return cudaSuccess;
+  return launch();
 }
 
 }  // namespace ppm

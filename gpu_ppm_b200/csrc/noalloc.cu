@@ -239,9 +239,10 @@ void Engine::profile_noalloc(const ppm_params& p, double* flux_d, double* counts
     FoldJob job{0, 0, p.exposure_s * (1. / p.n_bins)};
     ck(cudaMemcpyAsync(base + o_job, &job, sizeof(FoldJob), cudaMemcpyHostToDevice, st), "fold job upload");
     const FoldJob* dj = (const FoldJob*)(base + o_job);
-    if (p.fold == PPM_FOLD_BF16X3 && r.tc_ok)
-      ck(fold_tc_launch(r, dj, 1, p.n_bins, flux_d, counts_d, st, (int*)(base + o_status)), "fold launch");
-    else
+    if (p.fold == PPM_FOLD_BF16X3 && r.tc_ok) {
+      const TcFold f{p.response, dj, 1, p.n_bins};
+      ck(fold_tc_launch(&f, 1, flux_d, counts_d, st, (int*)(base + o_status)), "fold launch");
+    } else
       ck(launch_fold_simt(dj, 1, r.d_rsp, r.n_ch, r.n_e, p.n_bins, flux_d, counts_d, p.fold != PPM_FOLD_FP32, st),
          "fold launch");
   }
