@@ -766,7 +766,7 @@ void Engine::batch_build(BatchImpl& B, int n, const ppm_params* ps, cudaStream_t
     if (cell && !shapes[v].cellk) throw Error(PPM_E_STATE, "home-cell NSX kernel expected for the grid");
     // a group whose nodes are split over several tiles a ring runs from ring records: each ring's sweep and slice
     // are computed once (by ring_kernel) instead of by every tile.  A single profile of 408 rings, N_side 256:
-    // 1660 -> 1250 us a call (integrand 1410 -> 1000).  Groups with rings enough to fill the GPU keep the tiles: their rings
+    // 1640 -> 1080 us a call.  Groups with rings enough to fill the GPU keep the tiles: their rings
     // have one tile each, and their images (60 KB a ring) would be read back from HBM.
     // Blackbody groups run from ring records too.  Light curves (few energies) do so between about 200 and 592 rings
     // on 148 SMs only: the tiles' phase-major walk evaluates a point in fewer instructions, and loses where its rings

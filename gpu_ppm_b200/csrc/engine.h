@@ -214,7 +214,7 @@ struct Tuning {
   int ne_t = 0;      // energies per thread (0 = automatic)
   int minb = 2;      // CTAs per SM targeted by the register budget
   int kernel = 0;    // NSX integrand: 0 = home-cell kernel where the grid allows, 1 = pooled-polynomial kernel
-  int sets = 0;      // home-cell kernel: warp sets per CTA (0 = about 256 threads)
+  int sets = 0;      // home-cell kernel: warp sets per CTA (0 = as many as the kernel's threads hold)
   int cpl = 0;       // home-cell kernel: cells per lane (0 = by estimated cost)
   int splits = 0;    // phase-node splits per element chunk (0 = by the batch's work)
   int bb_nt = 0;     // blackbody point paths (<= 64 energies): threads per CTA (0 = 512 up to 4 energies, else 256)

@@ -1,6 +1,12 @@
 // Engine kernels: work planner, persistent integrand (NSX FP32 and blackbody
 // FP64/FP32 variants) and SIMT response folds.
 //
+// Two forms.  Batches whose rings fill the GPU run from tiles: a CTA per tile does
+// all of the steps below.  Small ones (a single profile, a served batch) run from
+// ring records: ring_kernel does steps 1 to 5 once a ring, the *_rec kernels do
+// step 6 for a ring's phase nodes, any CTA taking any node, and sum_parts_kernel
+// adds the stored node sums.  The results are the same bits.
+//
 // Integrand structure (one CTA per tile = candidate elements of one ring of
 // one spot of one profile; CTAs pull tiles from a device queue, except in the
 // blackbody kernel's fused point-source mode, where CTA b takes profile b's
@@ -20,7 +26,8 @@
 //      per-element atomics); a bin's partial sums are flushed once into the
 //      FP64 flux pool                     cpu/devarshi24st_cpu.cpp:214-241
 //      Home-cell kernel (default): each lane owns the energies of a few NSX
-//      cells and builds their cubics in registers from shuffled slice rows.
+//      cells and builds their cubics in registers from shuffled slice rows,
+//      two records at a time.
 //      Pooled-polynomial kernel (grids with > 16 energies in one cell): one
 //      warp per point writes the cubics to shared memory, one thread per
 //      energy reads its cell's cubic.
@@ -1454,7 +1461,8 @@ __global__ void __launch_bounds__(NTMAX, MINB) integrand_nsx_cell_kernel(const K
 // memory (L2); integrand_nsx_rec_kernel's CTAs load a ring's record and take its
 // phase nodes one at a time from the chunk's counter in global memory.
 
-// One CTA per (profile, spot, ring).
+// One CTA per (profile, spot, ring).  Bound by latency, a chain of block barriers (geometry, arcs, rows, sweep, gap
+// fill, slice): 14 us for 48 rings, 30 for 412, 62 for 819, of which the plan alone took 16 before.
 template <bool NSX>
 __global__ void __launch_bounds__(256) ring_kernel(const KernelArgs a) {
   extern __shared__ __align__(16) unsigned char sm[];
@@ -1590,7 +1598,8 @@ constexpr unsigned kSlotDead = 1u << 18;     // no chunk left to load
 // One CTA per SM with up to four chunk slots: the warp sets take nodes from any
 // loaded chunk; the last set to leave a drained slot loads its next chunk (the
 // one with the most work left per slot on it) while the others go on with the
-// other slots, so that nobody waits for a chunk's slowest node.
+// other slots, so that nobody waits for a chunk's slowest node (three CTAs per SM
+// with one chunk each spent 32 % of the warps' time in that wait).
 // Work is what a set does with the nodes it took (fill: a loaded chunk's context;
 // enter: the set comes to another chunk; nodes: the nodes [u, u + take)).
 template <int NTMAX, class Work>
@@ -1766,7 +1775,9 @@ __device__ __forceinline__ void rec_loop(const KernelArgs& a, unsigned char* sm,
   w.count(profile);
 }
 
-// Work of the home-cell NSX kernel: one node at a time.
+// Work of the home-cell NSX kernel: one node at a time.  Bound by the FMA pipe and the register file's ports, as over
+// tiles.  What a node is added to no longer shows: its sums are stored, not added atomically.  N_side 256, two spots,
+// 64 bins x 2 nodes, 300 energies: 1492 us from tiles, 937 with rings and sum from records.
 template <int MAXE, int C, int NTMAX>
 struct NsxWork : SetPlace<C> {
   const KernelArgs& a;
@@ -1820,7 +1831,10 @@ __global__ void __launch_bounds__(NTMAX, 1) integrand_nsx_rec_kernel(const Kerne
 // own the energies (c.lanes of them, up to four each; the lane groups take the
 // records in turn), kBbPass energies a pass, each pass a task of its own.  The
 // sums are FP64 in every arithmetic; a node's are combined over the lanes and
-// stored.  Bound by the FP64 pipe (about 60 operations a point and energy).
+// stored.  Bound by instruction issue (66 % of it; the FP64 pipe is at 31 %): the
+// point's bracket walk and the node's bookkeeping, not the Planck factor, whose
+// exponential in another form changed nothing.  A spectrum of 48 rings, 64
+// energies: 496 us a call from tiles, 95 from records.
 // FP32 arithmetic keeps the form of the tile kernel's path for the grid's size.
 template <typename Real>
 struct BbWork {
@@ -2777,7 +2791,9 @@ __device__ __forceinline__ void dd_add(double& s, double& c, double x) {
 // The flux of one (profile, bin) from its chunks' node sums (T: float in t_E order for NSX, double in energy order
 // for blackbody): grid (bins, energy tiles of Q, profiles), Q energies x kSumThreads / Q segments of chunks.
 // Double-double sums: the exact sum to about 1e-32, in any order of the records, as the pool's compensated atomics
-// give it; what the atomics added is included.  Bound by the read of the node sums, from L2 for a single profile.
+// give it; what the atomics added is included.  Bound by the read of the node sums, from L2 for a single profile:
+// 125 MB in 69 us with 12 loads in flight a thread and 256-thread blocks (512 threads, 8 loads: 83 to 108; 1024
+// threads, one after the other: 177), of an 1080 us call that took 1640 with every node's compensated atomics.
 template <typename T>
 __global__ void __launch_bounds__(kSumThreads) sum_parts_kernel(const KernelArgs a, int Q) {
   const RingWork& W = a.rings;
