@@ -1831,10 +1831,11 @@ __global__ void __launch_bounds__(NTMAX, 1) integrand_nsx_rec_kernel(const Kerne
 // own the energies (c.lanes of them, up to four each; the lane groups take the
 // records in turn), kBbPass energies a pass, each pass a task of its own.  The
 // sums are FP64 in every arithmetic; a node's are combined over the lanes and
-// stored.  Bound by instruction issue (66 % of it; the FP64 pipe is at 31 %): the
-// point's bracket walk and the node's bookkeeping, not the Planck factor, whose
-// exponential in another form changed nothing.  A spectrum of 48 rings, 64
-// energies: 496 us a call from tiles, 95 from records.
+// stored.  Bound by issue and latency (51 % of the issue slots, the FP64 pipe at
+// 16 %; 32 us for 48 rings, 64 energies, 32 x 2 nodes): the point's bracket walk
+// and the node's bookkeeping, not the Planck factor, whose exponential in another
+// form changed nothing.  That spectrum takes 425 us a call from tiles, 90 from
+// records.
 // FP32 arithmetic keeps the form of the tile kernel's path for the grid's size.
 template <typename Real>
 struct BbWork {

@@ -42,11 +42,12 @@ IntegrandShape make_shape(bool nsx, int nt, int ne_t, int pb, int max_cand, int 
 constexpr int kMaxRecSlots = 4;
 // Home-cell kernel over tiles: two CTAs of this many threads per SM.  The record loop is bound by the FMA pipe and the
 // register file's ports, not by the number of warps: 96 profiles of the batching prior took 64.4 ms with 24 warps per SM
-// at 80 registers, 59.5 ms with 20 at 96, 65.2 ms with 16 at 128.
+// at 80 registers, 59.5 ms with 20 at 96, 65.2 ms with 16 at 128 (with the
+// autotuned shape 52.4 now, 61.9 before pairs of records).
 constexpr int kCellThreads = 320;
 constexpr int kBbRecThreads = 768;  // integrand_bb_rec_kernel: 24 warps per SM at 80 registers
 constexpr int kPairFloats = 20;  // home-cell kernels: floats per pair of point records (80 bytes: 2-way bank conflicts)
-// threads of integrand_nsx_rec_kernel's CTA, one per SM: 80 registers a thread, 128 where a cell has many slots
+// threads of integrand_nsx_rec_kernel's CTA, one per SM: 96 registers a thread, 128 where a cell has many slots
 __host__ __device__ constexpr int rec_threads(int maxe_t) { return maxe_t <= 4 ? 640 : 512; }
 
 struct KernelArgs {

@@ -51,6 +51,12 @@ HostBuffer take(HostBuffer& b) {
 // hundred MB) ever runs while requests wait; admission caps a batch by the
 // bytes it stages, and only a single request larger than a buffer gets its own.
 constexpr size_t kStageBytes = size_t(32) << 20;
+// Most device memory of a served batch's ring records and node sums.  The first
+// batches that need it grow the stream-ordered pool on the scheduler thread while
+// requests wait: with 1 GiB a batch that took up to 525 ms once under overload,
+// with this as much as the batches' other blocks do (up to about 90 ms), and 24
+// mixed requests take 26.3 ms instead of 24.8 (31.3 from tiles).
+constexpr size_t kServeRingBytes = size_t(256) << 20;
 constexpr size_t kStageFixed = 64 + 256;  // control words and slack around the per-request arrays
 // a full batch's uploads (profiles, fold jobs, control words), each rounded up to 256 bytes
 constexpr size_t kUploadBytes = kMaxRequestsPerBatch * (sizeof(DevProfile) + sizeof(FoldJob)) + 4 * 256;
@@ -319,7 +325,7 @@ struct Server {
       f->slot = free_slot;
       f->bytes = bytes;
       f->reqs = std::move(take_reqs);
-      f->ring_limit = std::max<size_t>(1, std::min<size_t>(kRingBytesMax, (budget - in_use) / 2));
+      f->ring_limit = std::max<size_t>(1, std::min<size_t>(kServeRingBytes, (budget - in_use) / 2));
       f->trace.t_admit = since_start_us(Clock::now());
       f->trace.n_requests = (int32_t)f->reqs.size();
       f->trace.stream_slot = free_slot;
