@@ -779,15 +779,18 @@ void Engine::batch_build(BatchImpl& B, int n, const ppm_params* ps, cudaStream_t
       const size_t bytes = ring_work(shapes[v], hp.data(), order.data(), ps, g0, g1, chunk[v], rings[v]);
       unsigned char* base = nullptr;
       IntegrandShape rs = shapes[v];
+      auto ring_alloc = [&](size_t n) {
+        return B.ring_area ? B.ring_area + B.ring_bytes : (unsigned char*)B.mem.alloc(n);
+      };
       if (bytes && rec_shape(rs, rings[v]) && B.ring_bytes + bytes <= limit) {
         try {
-          base = (unsigned char*)B.mem.alloc(bytes);
+          base = ring_alloc(bytes);
         } catch (const Error&) {  // no room: the tiles need none
           cudaGetLastError();
         }
       }
       if (base) {
-        B.ring_bytes += bytes;
+        B.ring_bytes += (bytes + 255) / 256 * 256;
         RingWork& W = rings[v];
         W.recs = (RingRec*)base;
         W.ctr = (int4*)(W.recs + W.rec_cap);
@@ -806,7 +809,7 @@ void Engine::batch_build(BatchImpl& B, int n, const ppm_params* ps, cudaStream_t
         W.part_cap = (int)std::min<size_t>(cls / each, (size_t)W.rec_cap);
         if (W.part_cap > 0) {
           try {
-            W.parts = B.mem.alloc(cls);
+            W.parts = ring_alloc(cls);
             B.ring_bytes += cls;
           } catch (const Error&) {
             cudaGetLastError();

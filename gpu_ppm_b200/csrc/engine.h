@@ -160,6 +160,7 @@ struct BatchImpl {
   std::vector<Fold> folds;
   // device memory that ring records may take (0: the engine's default share) and what they took
   size_t ring_limit = 0, ring_bytes = 0;
+  unsigned char* ring_area = nullptr;  // their memory (ring_limit bytes, a multiple of 256); nullptr: from mem
   size_t h2d_bytes = 0;
   // pinned host memory the build stages its uploads in, when given (serving: one area per stream slot, untouched
   // until the slot's batch has finished, so the copies run asynchronously); pageable copies otherwise

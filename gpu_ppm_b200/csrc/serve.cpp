@@ -51,11 +51,12 @@ HostBuffer take(HostBuffer& b) {
 // hundred MB) ever runs while requests wait; admission caps a batch by the
 // bytes it stages, and only a single request larger than a buffer gets its own.
 constexpr size_t kStageBytes = size_t(32) << 20;
-// Most device memory of a served batch's ring records and node sums.  The first
-// batches that need it grow the stream-ordered pool on the scheduler thread while
-// requests wait: with 1 GiB a batch that took up to 525 ms once under overload,
-// with this as much as the batches' other blocks do (up to about 90 ms), and 24
-// mixed requests take 26.3 ms instead of 24.8 (31.3 from tiles).
+// Device memory of a served batch's ring records and node sums: an area per stream
+// slot, allocated when the server starts (all of them at most an eighth of the
+// memory budget beside it) and used by the slot's batches one after the other.
+// Taken from the stream-ordered pool, the first batches grew it on the scheduler
+// thread while requests waited, up to 525 ms at once under overload (at most 0.7
+// now); 24 mixed requests take 24.9 ms, 31.7 from tiles.
 constexpr size_t kServeRingBytes = size_t(256) << 20;
 constexpr size_t kStageFixed = 64 + 256;  // control words and slack around the per-request arrays
 // a full batch's uploads (profiles, fold jobs, control words), each rounded up to 256 bytes
@@ -84,6 +85,7 @@ struct Server {
   struct Slot {
     cudaStream_t stream = nullptr;
     bool busy = false;
+    DeviceBuffer rings;  // memory of the batch's ring records (see kServeRingBytes)
     HostBuffer upload;  // pinned source of the batch build's uploads; reused once the slot's batch has finished
   };
   struct InFlight {
@@ -93,7 +95,6 @@ struct Server {
     HostBuffer stage;                  // device-to-host staging of this batch, from the pool
     int slot = 0;
     size_t bytes = 0;
-    size_t ring_limit = 1;             // spare budget that the batch's ring records may take
     std::atomic<bool> finished{false};
     Server* server = nullptr;
     int* ctrl = nullptr;                 // pinned copy of the queue control words
@@ -140,11 +141,20 @@ struct Server {
       stage_pool.resize(slots.size() + kMaxCompleting);
       for (auto& b : stage_pool) b.reserve(kStageBytes);
       for (auto& s : slots) s.upload.reserve(kUploadBytes);
+      const size_t area = std::min(kServeRingBytes, budget / (8 * slots.size())) / 256 * 256;
+      for (auto& s : slots) {
+        try {
+          if (area) s.rings.reserve(area);
+        } catch (const Error&) {  // no room: its batches run from tiles
+          cudaGetLastError();
+        }
+      }
     } catch (...) {  // the destructor does not run for a constructor that throws
       for (auto& b : stage_pool) b.release();
       for (auto& s : slots) {
         if (s.stream) cudaStreamDestroy(s.stream);
         s.upload.release();
+        s.rings.release();
       }
       throw;
     }
@@ -177,6 +187,7 @@ struct Server {
         cudaStreamDestroy(s.stream);
       }
       s.upload.release();
+      s.rings.release();
     }
     for (auto& b : stage_pool) b.release();
   }
@@ -325,7 +336,6 @@ struct Server {
       f->slot = free_slot;
       f->bytes = bytes;
       f->reqs = std::move(take_reqs);
-      f->ring_limit = std::max<size_t>(1, std::min<size_t>(kServeRingBytes, (budget - in_use) / 2));
       f->trace.t_admit = since_start_us(Clock::now());
       f->trace.n_requests = (int32_t)f->reqs.size();
       f->trace.stream_slot = free_slot;
@@ -349,8 +359,6 @@ struct Server {
         fail(f->reqs, err);
         continue;
       }
-      f->bytes += f->B->ring_bytes;  // in flight with the batch, returned with it (retire)
-      in_use += f->B->ring_bytes;
       inflight.push_back(std::move(f));
     }
   }
@@ -363,7 +371,8 @@ struct Server {
     f.B.reset(new BatchImpl());
     BatchImpl& B = *f.B;
     B.mem.stream = slot.stream;
-    B.ring_limit = f.ring_limit;
+    B.ring_area = (unsigned char*)slot.rings.ptr;
+    B.ring_limit = std::max<size_t>(1, slot.rings.ptr ? slot.rings.cap / 256 * 256 : 0);
     B.h_upload = slot.upload.ptr;
     B.h_upload_cap = slot.upload.cap;
     {
