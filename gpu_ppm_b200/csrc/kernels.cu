@@ -43,6 +43,30 @@
 #include "kernels.cuh"
 
 namespace ppm {
+namespace {
+
+// Barrier of one warp set of n threads (a multiple of 32): the warp itself for
+// a one-warp set, else named barrier 1 + set.
+__device__ __forceinline__ void set_sync(int set, int n) {
+  if (n == 32)
+    __syncwarp();
+  else
+    asm volatile("bar.sync %0, %1;" ::"r"(1 + set), "r"(n) : "memory");
+}
+
+// 16-byte asynchronous copy from global to shared memory.
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+}  // namespace
+}  // namespace ppm
+
+#include "rec_loop.cuh"
+
+namespace ppm {
 
 namespace {
 
@@ -329,15 +353,6 @@ __device__ __forceinline__ double phase_point(const DevProfile& p, const SmemPtr
   double ppt;
   node_phase(p, u0 + du, bin, ppt, wgl);
   return node_point(p, s, rp, point, jj, ppt, z, mu);
-}
-
-// Barrier of one warp set of n threads (a multiple of 32): the warp itself for
-// a one-warp set, else named barrier 1 + set.
-__device__ __forceinline__ void set_sync(int set, int n) {
-  if (n == 32)
-    __syncwarp();
-  else
-    asm volatile("bar.sync %0, %1;" ::"r"(1 + set), "r"(n) : "memory");
 }
 
 // phase_point's arithmetic for one element at phase point i_pp, for the
@@ -868,27 +883,6 @@ __device__ __forceinline__ void pair_slots(const Cubic2 (&Q)[C + 1], const float
   }
 }
 
-// One chunk of a ring's active elements as the deposit needs it, in shared memory
-// (read at every step of 32 points: global loads there cost their latency).
-struct ChunkCtx {
-  double dphi, jofs, l10kT, tE_lo, tE_hi, out_scale, width;  // width: 1 / n_bins
-  long long flux_off;
-  const int *perm, *cell_first;
-  const float* fEs;
-  const double* invE;
-  unsigned long long* stats;
-  float* part;             // the chunk's node sums (stored plainly), or nullptr: added to the flux pool
-  int n_act, n_nodes, u_ofs, n_gl, n_fine, n_e, span, iE_min, mode;
-  int mono, held;          // phase_o non-decreasing; logT or log g outside the table (points count as clamped)
-  int profile, spot, rec;
-  int take;                // nodes a set takes at a time (ring records)
-  // blackbody: temperature, energies; tasks of per_pass energies, u_mod nodes each; lanes that own energies
-  double kT;
-  const double* E;
-  int per_pass, u_mod, lanes_log;
-  float glo[4], ghi[4];    // smallest and largest energy fraction of each slot group
-};
-
 // Fills a context (one thread); MAXE slots a cell.
 template <int MAXE, int MOST>
 __device__ __forceinline__ void fill_ctx(ChunkCtx& c, const DevProfile& p, const DevSpot& sp, int ring, int n_act, bool mono,
@@ -930,14 +924,6 @@ __device__ __forceinline__ void fill_ctx(ChunkCtx& c, const DevProfile& p, const
     c.ghi[g] = hi;
   }
 }
-
-// A chunk's tables in shared memory.  Sx: slice row 0.
-struct ChunkBufs {
-  const unsigned short* j;
-  const double *P, *F, *Z, *MU;
-  const unsigned short* hidx;
-  const float* Sx;
-};
 
 // A phase node taken by a warp set: its number, bin, phase and weight.
 struct Node {
@@ -1326,10 +1312,6 @@ __device__ __forceinline__ int nsx_taps(const DevNsx& X, const DevProfile& p, co
   return n;
 }
 
-// The home-cell kernels' slice image: rows 0..nE-1 start 16-byte aligned after
-// room for rows -1 - C .. -1; rows nE .. nE + C follow them.
-__host__ __device__ __forceinline__ int slice_row0(int ldS, int C) { return ((C + 1) * ldS + 3) & ~3; }
-
 // Reduces the NSX table into S[E][mu] (row stride ldS, Sx = row 0, in shared or
 // global memory); all threads of the block, block barriers inside.
 __device__ __forceinline__ void build_slice(const DevNsx& X, int ldS, int C, const float* tapw, const int* tapo, int ntap,
@@ -1582,197 +1564,6 @@ __global__ void __launch_bounds__(256) ring_kernel(const KernelArgs a) {
   for (int k = tid; k < n16; k += nt) ((float4*)img)[k] = ((const float4*)(sm + S.off_P))[k];
   if (NSX)
     build_slice(a.nsx, S.ldS, S.cpl, s_tapw, s_tapo, s_ntap, (float*)(img + W.off_slice) + slice_row0(S.ldS, S.cpl));
-}
-
-// 16-byte asynchronous copy from global to shared memory.
-__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
-               : "memory");
-}
-
-// State of a chunk slot: the warp sets inside it (low bits) and its flags.
-constexpr unsigned kSlotDrain = 1u << 16;    // its chunk has no nodes left to take
-constexpr unsigned kSlotLoading = 1u << 17;  // one set is loading its next chunk
-constexpr unsigned kSlotDead = 1u << 18;     // no chunk left to load
-
-// One CTA per SM with up to four chunk slots: the warp sets take nodes from any
-// loaded chunk; the last set to leave a drained slot loads its next chunk (the
-// one with the most work left per slot on it) while the others go on with the
-// other slots, so that nobody waits for a chunk's slowest node (three CTAs per SM
-// with one chunk each spent 32 % of the warps' time in that wait).
-// Work is what a set does with the nodes it took (fill: a loaded chunk's context;
-// enter: the set comes to another chunk; nodes: the nodes [u, u + take)).
-template <int NTMAX, class Work>
-__device__ __forceinline__ void rec_loop(const KernelArgs& a, unsigned char* sm, Work& w) {
-  const IntegrandShape& S = a.shape;
-  const RingWork& W = a.rings;
-  constexpr int kSets = NTMAX / 32;
-  __shared__ ChunkCtx s_ctx[kMaxRecSlots];
-  __shared__ unsigned s_word[kMaxRecSlots];
-  __shared__ int s_got[kSets], s_u[kSets];
-  __shared__ unsigned long long s_best[kSets];
-  const int tid = threadIdx.x, nt = blockDim.x;
-  const int n_recs = min(*W.n_recs, W.rec_cap);
-  if (n_recs == 0) return;
-  const int NS = S.rec_slots;
-  if (tid < NS) {
-    s_word[tid] = kSlotDrain;
-    s_ctx[tid].rec = -1;
-  }
-  __syncthreads();
-  const int per_slot = max(1, nt / w.ST / NS);  // warp sets per slot
-  const int a16 = (S.off_F - S.off_P) / 8;      // doubles between the sweep's arrays
-  volatile unsigned* const word = s_word;
-
-  // leader of a set: leaves slot sl; true if the set has become the loader of the drained slot
-  auto leave = [&](int sl) {
-    return atomicSub(&s_word[sl], 1u) == (kSlotDrain | 1u) && atomicCAS(&s_word[sl], kSlotDrain, kSlotLoading) == kSlotDrain;
-  };
-  constexpr int kExit = -1;  // s_got: a slot to work in, kExit, or -2 - slot to load
-  int cur_rec = -1, cur_slot = -1, profile = -1, pref = w.set % NS;
-  bool claimed = false;  // (leader) the slot just left is this set's to load
-  for (;;) {
-    if (w.st == 0) {
-      int got = kExit;
-      if (claimed) {
-        got = -2 - cur_slot;
-        claimed = false;
-      } else {
-        // bounded: a set that finds nothing for a second leaves, the others finish the work
-        for (int spin = 0; spin < (1 << 21); ++spin) {
-          bool live = false;
-          for (int k = 0; k < NS && got == kExit; ++k) {
-            int sl = pref + k;
-            sl -= sl >= NS ? NS : 0;
-            const unsigned v = word[sl];
-            if (v & kSlotDead) continue;
-            live = true;
-            if (v == kSlotDrain) {
-              if (atomicCAS(&s_word[sl], kSlotDrain, kSlotLoading) == kSlotDrain) got = -2 - sl;
-              continue;
-            }
-            if (v & (kSlotDrain | kSlotLoading)) continue;
-            if (!(atomicAdd(&s_word[sl], 1u) & (kSlotDrain | kSlotLoading | kSlotDead))) {
-              __threadfence_block();
-              const ChunkCtx& c = s_ctx[sl];
-              const int u = atomicAdd(&W.ctr[c.rec].x, c.take);
-              if (u < c.n_nodes) {
-                s_u[w.set] = u;
-                got = sl;
-                continue;
-              }
-              atomicOr(&s_word[sl], kSlotDrain);
-            }
-            if (leave(sl)) got = -2 - sl;
-          }
-          if (got != kExit || !live) break;
-          __nanosleep(500);
-        }
-      }
-      s_got[w.set] = got;
-    }
-    set_sync(w.set, w.ST);
-    const int got = s_got[w.set];
-    if (got == kExit) break;
-    if (got < kExit) {
-      const int sl = -2 - got;
-      int r = -1;
-      for (;;) {
-        if (s_ctx[sl].rec < 0) {  // the slot's first chunk
-          r = (int)((blockIdx.x + (unsigned)sl * gridDim.x) % (unsigned)n_recs);
-          if (w.st == 0) atomicAdd(&W.ctr[r].y, 1);
-          set_sync(w.set, w.ST);
-          break;
-        }
-        // chunks that nobody has yet, in order
-        if (w.st == 0) {
-          s_best[w.set] = 0;
-          const int nx = NS * (int)gridDim.x < n_recs ? NS * (int)gridDim.x + atomicAdd(&W.ctr[W.rec_cap].x, 1) : n_recs;
-          s_got[w.set] = nx < n_recs ? nx : -1;
-          if (nx < n_recs) atomicAdd(&W.ctr[nx].y, 1);
-        }
-        set_sync(w.set, w.ST);
-        r = s_got[w.set];
-        if (r >= 0) break;
-        // then the one with the most work left per slot on it
-        unsigned long long best = 0;
-#pragma unroll 4
-        for (int q = w.st; q < n_recs; q += w.ST) {
-          const int4 t = __ldcg(W.ctr + q);
-          const int left = t.z - t.x;
-          // (scattered a little, so that slots that look at the same time choose differently)
-          const float jitter = 0.5f + (float)(((unsigned)q * 2654435761u + blockIdx.x * 40503u) >> 24) * (1.f / 512.f);
-          const float score = (float)left * (float)t.w / (float)(t.y + 1) * jitter;
-          const unsigned long long key = ((unsigned long long)__float_as_uint(score) << 32) | (unsigned)q;
-          // a chunk whose slots' sets will take the remaining nodes at once is left to them
-          best = left > per_slot * t.y / 2 && key > best ? key : best;
-        }
-        if (best) atomicMax(&s_best[w.set], best);
-        set_sync(w.set, w.ST);
-        if (s_best[w.set] == 0) break;
-        r = (int)(unsigned)s_best[w.set];
-        if (w.st == 0) {
-          const int y = atomicAdd(&W.ctr[r].y, 1);
-          s_got[w.set] = W.recs[r].n_nodes - __ldcg(&W.ctr[r].x) > per_slot * y / 2 ? 1 : 0;
-        }
-        set_sync(w.set, w.ST);
-        const bool ok = s_got[w.set] != 0;
-        set_sync(w.set, w.ST);
-        if (ok) break;
-        r = -1;
-      }
-      if (r < 0) {
-        if (w.st == 0) atomicXor(&s_word[sl], kSlotLoading | kSlotDead);
-        continue;
-      }
-      const RingRec q = W.recs[r];
-      unsigned char* const dst = sm + (size_t)sl * S.rec_slot_bytes;
-      const unsigned char* const img = W.data + (size_t)q.job * W.stride;
-      const int n16 = (W.off_slice + W.slice_bytes) >> 4;
-      for (int k = w.st; k < n16; k += w.ST) cp_async16(dst + 16 * k, img + 16 * k);
-      const int l16 = (q.n_act * W.elem_bytes + 15) >> 4;
-      for (int k = w.st; k < l16; k += w.ST) cp_async16(dst + 16 * (n16 + k), W.lists + (size_t)q.list * W.elem_bytes + 16 * k);
-      if (w.st == 0) {
-        const DevProfile& p = a.profiles[q.profile];
-        ChunkCtx& c = s_ctx[sl];
-        w.fill(c, p, p.spot[q.spot], q);
-        // nodes are taken from a chunk's own first one on: chunks that run at the same time add to different bins
-        c.u_ofs = (int)((unsigned)q.job * 40503u % (unsigned)c.u_mod);
-        c.part = r < W.part_cap ? (float*)W.parts + (size_t)r * W.part_stride : nullptr;
-        c.profile = q.profile;
-        c.spot = q.spot;
-        c.rec = r;
-      }
-      asm volatile("cp.async.wait_all;" ::: "memory");
-      __threadfence_block();
-      set_sync(w.set, w.ST);
-      if (w.st == 0) {
-        __threadfence_block();
-        atomicAnd(&s_word[sl], ~kSlotLoading);
-      }
-      continue;
-    }
-    // a node of the chunk in slot `got`
-    __threadfence_block();
-    cur_slot = pref = got;
-    const ChunkCtx& c = s_ctx[got];
-    if (c.rec != cur_rec) {
-      cur_rec = c.rec;
-      if (profile != c.profile) w.count(profile);
-      profile = c.profile;
-      w.enter(c);
-    }
-    const unsigned char* const base = sm + (size_t)got * S.rec_slot_bytes;
-    const double* P = (const double*)base;
-    const ChunkBufs bufs{(const unsigned short*)(base + W.off_slice + W.slice_bytes), P, P + a16, P + 2 * a16, P + 3 * a16,
-                         (const unsigned short*)(base + W.off_hidx),
-                         (const float*)(base + W.off_slice) + slice_row0(S.ldS, S.cpl)};
-    w.nodes(c, bufs, s_u[w.set]);
-    __threadfence_block();
-    set_sync(w.set, w.ST);
-    if (w.st == 0) claimed = leave(got);
-  }
-  w.count(profile);
 }
 
 // Work of the home-cell NSX kernel: one node at a time.  Bound by the FMA pipe and the register file's ports, as over
