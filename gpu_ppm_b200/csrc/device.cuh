@@ -73,7 +73,8 @@ struct DevSpot {
   int kind;            // PPM_SPOT_*
   int i_lo, i_hi;      // HEALPix ring range that can hold active elements
   int T_clamped;       // logT outside the NSX axis
-  int job0;            // ring records: index of the spot's first ring job in its kernel group
+  int job0;            // ring records: index of the spot's first ring job in its kernel group (never decreasing over
+                       // the group's profiles and spots, spots without jobs included)
   int nT_taps;         // 2 (linear logT) or 4 (cubic logT)
   int iT[4];
   double wT[4];
@@ -129,6 +130,10 @@ struct RingWork {
   int elem_bytes;
   int *n_recs, *list_next;
   int rec_cap, list_cap, n_jobs, n_profiles, chunk;
+  // each profile's records, 2 x record + spot, in any order: from by_profile[per_job x its first job] on, as many as
+  // its ring_seen[0] says (the ring bits' first word, cleared before each pass: ring_kernel keeps no ring bits)
+  int* by_profile;
+  int per_job;            // most records of a job
   // node sums of the first part_cap records, [record][node][energy in t_E order], part_stride floats a record,
   // summed into the flux pool by sum_parts_kernel; further records add to the pool atomically
   void* parts;           // float (NSX) or double (blackbody); part_stride in units of 4 bytes

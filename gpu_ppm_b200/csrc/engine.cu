@@ -795,7 +795,8 @@ void Engine::batch_build(BatchImpl& B, int n, const ppm_params* ps, cudaStream_t
         W.recs = (RingRec*)base;
         W.ctr = (int4*)(W.recs + W.rec_cap);
         W.lists = (unsigned char*)(base + ((sizeof(RingRec) + sizeof(int4)) * ((size_t)W.rec_cap + 1) + 255) / 256 * 256);
-        W.data = W.lists + ((size_t)W.elem_bytes * (size_t)W.list_cap + 255) / 256 * 256;
+        W.by_profile = (int*)(W.lists + ((size_t)W.elem_bytes * (size_t)W.list_cap + 255) / 256 * 256);
+        W.data = (unsigned char*)W.by_profile + (sizeof(int) * (size_t)W.per_job * (size_t)W.n_jobs + 255) / 256 * 256;
         W.n_recs = B.d_ctrl + 3 * v;
         W.list_next = B.d_ctrl + 3 * v + 1;
         shapes[v] = rs;
@@ -818,9 +819,9 @@ void Engine::batch_build(BatchImpl& B, int n, const ppm_params* ps, cudaStream_t
         }
         int job = 0;
         for (int k = g0; k < g1; ++k)
-          for (int s = 0; s < hp[k].n_spots; ++s) {
+          for (int s = 0; s < kMaxSpots; ++s) {
             hp[k].spot[s].job0 = job;
-            job += ring_jobs(hp[k].spot[s]);
+            if (s < hp[k].n_spots) job += ring_jobs(hp[k].spot[s]);
           }
       } else {
         rings[v] = RingWork{};
@@ -1171,16 +1172,18 @@ void Engine::group_tiling(bool pooled, const GroupWork& w, int chunk_override, i
 // holds the records, their counters, the element lists and the images, 0 if there is nothing to hold or too much.
 size_t Engine::ring_work(const IntegrandShape& shape, const DevProfile* hp, const int* order, const ppm_params* ps, int g0,
                          int g1, int chunk, RingWork& W) const {
-  long long recs = 0, list = 0, jobs = 0;
+  long long recs = 0, list = 0, jobs = 0, per_job = 1;
   for (int k = g0; k < g1; ++k) {
     recs += tile_bound(ps[order[k]], hp[k], chunk, 0);
     for (int s = 0; s < hp[k].n_spots; ++s) {
       const long long nj = ring_jobs(hp[k].spot[s]), per = 4ll * hp[k].n_side;
       jobs += nj;
+      per_job = std::max(per_job, 2 + (per + chunk - 1) / chunk);
       list += nj * (per + 8 * (2 + (per + chunk - 1) / chunk));
     }
   }
-  if (jobs <= 0 || recs > (1 << 24) || list > (1 << 30) || jobs > (1 << 24)) return 0;
+  if (jobs <= 0 || recs > (1 << 24) || list > (1 << 30) || jobs > (1 << 24) || per_job * jobs > (1 << 30))
+    return 0;
   auto up = [](size_t v) { return (v + 255) / 256 * 256; };
   W.elem_bytes = shape.nsx ? 2 : 8;
   W.hidx_bytes = (int)((2 * ((size_t)shape.n_fine + 1) + 15) / 16 * 16);
@@ -1192,10 +1195,11 @@ size_t Engine::ring_work(const IntegrandShape& shape, const DevProfile* hp, cons
   W.rec_cap = (int)recs;
   W.list_cap = (int)list;
   W.n_jobs = (int)jobs;
+  W.per_job = (int)per_job;
   W.n_profiles = g1 - g0;
   W.chunk = chunk;
   const size_t bytes = up((sizeof(RingRec) + sizeof(int4)) * ((size_t)recs + 1)) + up((size_t)W.elem_bytes * (size_t)list) +
-                       (size_t)W.stride * (size_t)jobs;
+                       up(sizeof(int) * (size_t)per_job * (size_t)jobs) + (size_t)W.stride * (size_t)jobs;
   // whole powers of two, so that the blocks of a sampler's next proposals fit the cached ones
   size_t cls = 1 << 20;
   while (cls < bytes) cls <<= 1;

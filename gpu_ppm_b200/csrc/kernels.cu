@@ -1453,7 +1453,7 @@ __global__ void __launch_bounds__(256) ring_kernel(const KernelArgs a) {
   const SmemPtrs s = carve(sm, S);
   __shared__ RingGeom s_g;
   __shared__ int s_int[48];
-  __shared__ int s_job[3];
+  __shared__ int s_first;
   __shared__ int s_range[2][2], s_nr;
   __shared__ float s_tapw[16];
   __shared__ int s_tapo[16];
@@ -1461,22 +1461,22 @@ __global__ void __launch_bounds__(256) ring_kernel(const KernelArgs a) {
   const int tid = threadIdx.x, nt = blockDim.x;
   const int job = blockIdx.x;
   if (job == 0 && tid == 0) W.ctr[W.rec_cap] = make_int4(0, 0, 0, 0);
-  for (int t = tid; t < W.n_profiles * kMaxSpots; t += nt) {
-    const DevProfile& q = a.profiles[t / kMaxSpots];
-    const int si = t % kMaxSpots;
-    if (si >= q.n_spots) continue;
-    const int at = job - q.spot[si].job0, n = ring_jobs(q.spot[si]);
-    if (at >= 0 && at < n) {
-      s_job[0] = t / kMaxSpots;
-      s_job[1] = si;
-      s_job[2] = q.spot[si].kind == 1 ? 0 : q.spot[si].i_lo + at;
-    }
+  // the job's profile, in [first, last): an nt-fold search, none for one profile, a step up to nt of them (every CTA
+  // over every spot would be profiles^2: 16384 point sources took 2.8 ms in this kernel)
+  int first = 0;
+  for (int last = W.n_profiles; last - first > 1;) {
+    const int step = (last - first + nt - 1) / nt, k = first + tid * step, k1 = min(k + step, last);
+    if (k < last && a.profiles[k].spot[0].job0 <= job && (k1 == last || job < a.profiles[k1].spot[0].job0)) s_first = k;
+    __syncthreads();
+    first = s_first;
+    last = min(first + step, last);
+    __syncthreads();
   }
-  __syncthreads();
-  const DevProfile& p = a.profiles[s_job[0]];
-  const DevSpot& sp = p.spot[s_job[1]];
-  const int ring = s_job[2];
+  const DevProfile& p = a.profiles[first];
+  const int spot = job - p.spot[0].job0 < ring_jobs(p.spot[0]) ? 0 : 1;
+  const DevSpot& sp = p.spot[spot];
   const bool point = sp.kind == 1;
+  const int ring = point ? 0 : sp.i_lo + job - sp.job0;
   const DevLens& L = a.lens;
   const double z = point ? sp.cos_theta_pt : p.ring[3 * ring];
   const double c2 = point ? 0.0 : p.ring[3 * ring + 1], s2 = point ? 0.0 : p.ring[3 * ring + 2];
@@ -1506,10 +1506,10 @@ __global__ void __launch_bounds__(256) ring_kernel(const KernelArgs a) {
   const RingPhi rp = point ? RingPhi{0.0, 0.0} : healpix_ring_phi(p.n_side, ring);
   // active elements, one record per chunk of candidates
   int n_ring = 0;
-  bool first = true;
+  bool first_chunk = true;
   for (int k = 0; k < nr; ++k) {
     const int j_end = point ? 1 : s_range[k][1] + 1;
-    for (int j0 = point ? 0 : s_range[k][0]; j0 < j_end; j0 += W.chunk, first = false) {
+    for (int j0 = point ? 0 : s_range[k][0]; j0 < j_end; j0 += W.chunk, first_chunk = false) {
       const int n_c = min(W.chunk, j_end - j0);
       int n_act = 0;
       for (int k0 = 0; k0 < n_c; k0 += nt) {
@@ -1525,18 +1525,19 @@ __global__ void __launch_bounds__(256) ring_kernel(const KernelArgs a) {
       if (n_act == 0 || dropped) continue;
       if (tid == 0) {
         const int at = atomicAdd(W.n_recs, 1), lo = atomicAdd(W.list_next, (n_act + 7) & ~7);
+        const int nth = (int)atomicAdd(p.ring_seen, 1u);
         s_int[43] = lo;
         const bool held = NSX && (sp.T_clamped || s_g.logg < a.nsx.g_min || s_g.logg > a.nsx.g_max);
         const int tasks = p.n_bins * max(p.n_gl, 1) * (NSX ? 1 : (p.n_e + kBbPass - 1) / kBbPass);
         if (at < W.rec_cap && lo + n_act <= W.list_cap) {
-          W.recs[at] = RingRec{s_job[0], s_job[1], ring, job, n_act, lo, tasks,
-                               (mono ? 1 : 0) | (held ? 2 : 0)};
+          W.recs[at] = RingRec{first, spot, ring, job, n_act, lo, tasks, (mono ? 1 : 0) | (held ? 2 : 0)};
           W.ctr[at] = make_int4(0, 0, tasks, n_act);
         } else {
           s_int[43] = -1;
           atomicOr(a.queue.overflow, 1);
         }
-        if (s_g.u_clamped && first) atomicAdd(&p.stats[4], 1ull);
+        W.by_profile[W.per_job * p.spot[0].job0 + nth] = s_int[43] >= 0 ? 2 * at + spot : INT_MAX;
+        if (s_g.u_clamped && first_chunk) atomicAdd(&p.stats[4], 1ull);
       }
       __syncthreads();
       const int lo = s_int[43];
@@ -2598,7 +2599,8 @@ __global__ void __launch_bounds__(kSumThreads) sum_parts_kernel(const KernelArgs
   __shared__ unsigned s_ofs[kSumList];
   __shared__ int s_n[kMaxSpots];
   __shared__ double s_s[kSumThreads], s_c[kSumThreads];
-  const int n_recs = min(*W.n_recs, min(W.rec_cap, W.part_cap));
+  const int n_recs = (int)*p.ring_seen;
+  const int* const recs = W.by_profile + (size_t)W.per_job * p.spot[0].job0;
   const int e = q < n_e ? (std::is_same<T, float>::value ? p.grid.perm[q] : q) : 0;
   const double invE = q < n_e ? p.grid.invE[e] : 0.0;
   const int n_gl = max(p.n_gl, 1);
@@ -2609,9 +2611,9 @@ __global__ void __launch_bounds__(kSumThreads) sum_parts_kernel(const KernelArgs
     __syncthreads();
     if (threadIdx.x < kMaxSpots) s_n[threadIdx.x] = 0;
     __syncthreads();
-    const int r = r0 + (int)threadIdx.x;
-    if (r < n_recs && W.recs[r].profile == (int)blockIdx.z) {
-      const int sp = W.recs[r].spot, at = atomicAdd(&s_n[sp], n_gl);
+    const int entry = r0 + (int)threadIdx.x < n_recs ? recs[r0 + threadIdx.x] : 2 * W.part_cap, r = entry >> 1;
+    if (r < W.part_cap) {
+      const int sp = entry & 1, at = atomicAdd(&s_n[sp], n_gl);
       for (int g = 0; g < n_gl; ++g)
         s_ofs[sp ? kSumList - 1 - (at + g) : at + g] = (unsigned)(r * W.part_stride) + (unsigned)(g * n_e * (int)(sizeof(T) / 4));
     }
