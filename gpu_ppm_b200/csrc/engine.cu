@@ -986,7 +986,7 @@ int Engine::kernels_per_pass(const BatchImpl& B) const {
   // per group the plan (or rings) and the integrand, and the sum of the node sums; add_comp for the others; folds
   int n = folds, pool = 0;
   for (const auto& G : B.groups) {
-    n += G.args.shape.rec ? 3 : 2;
+    n += G.args.shape.rec ? 2 + (G.g1 - G.g0 + kSumProfiles - 1) / kSumProfiles : 2;
     pool |= G.args.shape.rec ? 0 : 1;
   }
   return n + pool;

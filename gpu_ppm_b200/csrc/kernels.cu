@@ -2582,15 +2582,15 @@ __device__ __forceinline__ void dd_add(double& s, double& c, double x) {
 }
 
 // The flux of one (profile, bin) from its chunks' node sums (T: float in t_E order for NSX, double in energy order
-// for blackbody): grid (bins, energy tiles of Q, profiles), Q energies x kSumThreads / Q segments of chunks.
+// for blackbody): grid (bins, energy tiles of Q, profiles from p0 on), Q energies x kSumThreads / Q segments of chunks.
 // Double-double sums: the exact sum to about 1e-32, in any order of the records, as the pool's compensated atomics
 // give it; what the atomics added is included.  Bound by the read of the node sums, from L2 for a single profile:
 // 125 MB in 69 us with 12 loads in flight a thread and 256-thread blocks (512 threads, 8 loads: 83 to 108; 1024
 // threads, one after the other: 177), of an 1080 us call that took 1640 with every node's compensated atomics.
 template <typename T>
-__global__ void __launch_bounds__(kSumThreads) sum_parts_kernel(const KernelArgs a, int Q) {
+__global__ void __launch_bounds__(kSumThreads) sum_parts_kernel(const KernelArgs a, int Q, int p0) {
   const RingWork& W = a.rings;
-  const DevProfile& p = a.profiles[blockIdx.z];
+  const DevProfile& p = a.profiles[p0 + (int)blockIdx.z];
   const int bin = blockIdx.x, n_e = p.n_e, segs = kSumThreads / Q;
   const int ql = threadIdx.x % Q, seg = threadIdx.x / Q, q = blockIdx.y * Q + ql;
   if (bin >= p.n_bins || blockIdx.y * Q >= n_e) return;
@@ -2655,11 +2655,13 @@ __global__ void __launch_bounds__(kSumThreads) sum_parts_kernel(const KernelArgs
 cudaError_t launch_sum_parts(const KernelArgs& a, int bins_max, int ne_max, cudaStream_t st) {
   int Q = 1;
   while (Q < kSumQ && Q < ne_max) Q <<= 1;
-  const dim3 grid(bins_max, (ne_max + Q - 1) / Q, a.rings.n_profiles);
-  if (a.shape.nsx)
-    sum_parts_kernel<float><<<grid, kSumThreads, 0, st>>>(a, Q);
-  else
-    sum_parts_kernel<double><<<grid, kSumThreads, 0, st>>>(a, Q);
+  for (int p0 = 0; p0 < a.rings.n_profiles; p0 += kSumProfiles) {
+    const dim3 grid(bins_max, (ne_max + Q - 1) / Q, std::min(kSumProfiles, a.rings.n_profiles - p0));
+    if (a.shape.nsx)
+      sum_parts_kernel<float><<<grid, kSumThreads, 0, st>>>(a, Q, p0);
+    else
+      sum_parts_kernel<double><<<grid, kSumThreads, 0, st>>>(a, Q, p0);
+  }
   return cudaGetLastError();
 }
 

@@ -71,7 +71,9 @@ cudaError_t launch_plan(const DevProfile* profiles, int n_profiles, const DevLen
 cudaError_t launch_add_comp(double* flux, const double* comp, long long n, int sm_count, cudaStream_t st);
 // ring records of a group (a.rings): plan, sweep and slice of every ring
 cudaError_t launch_rings(const KernelArgs& a, cudaStream_t st);
-// the group's flux from the records' node sums and the pools (whose compensation it clears)
+// the group's flux from the records' node sums and the pools (whose compensation it clears), a launch for each
+// kSumProfiles profiles (grid z)
+constexpr int kSumProfiles = 65535;
 cudaError_t launch_sum_parts(const KernelArgs& a, int bins_max, int ne_max, cudaStream_t st);
 cudaError_t launch_integrand(const KernelArgs& a, int grid, cudaStream_t st);
 // counts[c][b] = alpha * sum_E rsp[c][E] * flux[b][E] for each listed profile, FP64 or FP32 SIMT

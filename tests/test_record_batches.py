@@ -42,3 +42,33 @@ def test_profiles_of_a_batch(n, n_e):
         assert infos[k].as_dict() == info.as_dict(), k
         assert max_rel(flux[k], one) < 1e-12, k  # FP64 sums of another order
     e.close()
+
+
+def test_more_profiles_than_a_grid_dimension_holds():
+    """65 540 profiles, of which the ring window leaves five with rings, the last one among them."""
+    from gpu_ppm_b200.engine import Engine
+
+    e = Engine(max_batch=70000)
+    e.load_lensing(synth.lensing("std"))
+    g = e.add_energy_grid(synth.energy_grid(5, 0.1, 12.0))
+    # one cap around the pole (rings 1 and 2 of 15), the others around the equator
+    polar, far = [synth.params(mass_msun=1.4, r_eq_km=12.0, spin_hz=400.0, inclination_rad=1.1, distance_kpc=0.2,
+                               spots=[synth.spot(t, 0.0, 0.4, kT_keV=0.3)], atmosphere=_abi.ATM_BLACKBODY, beaming=0,
+                               n_side=4, n_bins=2, n_gl=0, n_fine=8, energy_grid=g, precision=_abi.PREC_FP64)
+                  for t in (0.1, 1.6)]
+    plist = [far] * 65540
+    own = [0, 1, 40000, 65535, 65539]
+    for k in own:
+        plist[k] = polar
+    batch = e.batch(plist, rings=(1, 3))
+    batch.launch()
+    flux, _, infos = batch.collect(want_flux=True, want_counts=False)
+    batch.close()
+    one, _, info = e.profile_rings(polar, 1, 3, want_counts=False)
+    e.close()
+    flux = np.asarray(flux).reshape(len(plist), -1)
+    assert info.n_points > 0 and one.any()
+    for k in own:
+        assert infos[k].as_dict() == info.as_dict()
+        assert max_rel(flux[k], one.ravel()) < 1e-12
+    assert not np.delete(flux, own, axis=0).any()
