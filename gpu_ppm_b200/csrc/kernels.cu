@@ -1675,16 +1675,11 @@ struct BbWork {
     const Real Ee = E * zb;
     return (double)(cb * (Ee * Ee * Ee / expm1(std::is_same<Real, float>::value && divide ? Ee / kT : Ee * inv_kT)));
   }
-  // The same of two points.  Where x = E / kT > 1 for every lane's, e^x - 1 loses nothing to cancellation (two
-  // roundings, as expm1 has) and is cheaper; hidden points have c = 0 and z = 1.  In one block, so that the two
-  // evaluations overlap and share their constants.  All lanes call it.
+  // The same of two points, in one block, so that the two evaluations overlap and share their constants; hidden points
+  // have c = 0 and z = 1.  A point's value is its own: what the other lanes hold depends on the batch.
   static __device__ __forceinline__ double planck_pair(double ca, double za, double cb, double zb, double E, double inv_kT) {
-    const double ea = E * za, eb = E * zb, xa = ea * inv_kT, xb = eb * inv_kT;
-    if (__all_sync(0xffffffffu, xa > 1.0 && xb > 1.0)) {
-      const double ya = exp(xa) - 1.0, yb = exp(xb) - 1.0;
-      return ca * (ea * ea * ea / ya) + cb * (eb * eb * eb / yb);
-    }
-    return ca * (ea * ea * ea / expm1(xa)) + cb * (eb * eb * eb / expm1(xb));
+    const double ea = E * za, eb = E * zb;
+    return ca * (ea * ea * ea / expm1(ea * inv_kT)) + cb * (eb * eb * eb / expm1(eb * inv_kT));
   }
   // The bracket and fraction of element jj's patch phase (node_point_tab, with the element's phase shift and the
   // reciprocal interval widths from the ring's image).  All lanes call it.
@@ -1775,7 +1770,7 @@ struct BbWork {
         for (int k = 0; k < kPhaseMajorMaxE; ++k)
           if (k < ne) {
             if constexpr (std::is_same<Real, double>::value) {
-              acc[k] += planck_pair(ca, za, cb, zb, E[k], inv_kT);
+              acc[k] += m == 1 ? planck_pair(ca, za, cb, zb, E[k], inv_kT) : planck(ca, za, E[k], 0.0, inv_kT, false);
             } else {
               if (fa != 0.0) acc[k] += planck((Real)ca, (Real)za, E[k], (Real)0, inv_kT, false);
               if (fb != 0.0) acc[k] += planck((Real)cb, (Real)zb, E[k], (Real)0, inv_kT, false);
