@@ -1670,10 +1670,11 @@ struct BbWork {
     if (lane == 0 && profile >= 0 && n_vis) atomicAdd(&a.profiles[profile].stats[3], (unsigned long long)n_vis);
     n_vis = 0;
   }
-  // Ibb without its constant, times the point's flux (cpu/unit.hpp:28-31).
+  // Ibb without its constant, times the point's flux (cpu/unit.hpp:28-31).  divide: E / kT as a division, as the tile
+  // kernel's path for more than 64 energies has it (one rounding less), else by the reciprocal.
   static __device__ __forceinline__ double planck(Real cb, Real zb, Real E, Real kT, Real inv_kT, bool divide) {
     const Real Ee = E * zb;
-    return (double)(cb * (Ee * Ee * Ee / expm1(std::is_same<Real, float>::value && divide ? Ee / kT : Ee * inv_kT)));
+    return (double)(cb * (Ee * Ee * Ee / expm1(divide ? Ee / kT : Ee * inv_kT)));
   }
   // The same of two points, in one block, so that the two evaluations overlap and share their constants; hidden points
   // have c = 0 and z = 1.  A point's value is its own: what the other lanes hold depends on the batch.
@@ -1681,31 +1682,30 @@ struct BbWork {
     const double ea = E * za, eb = E * zb;
     return ca * (ea * ea * ea / expm1(ea * inv_kT)) + cb * (eb * eb * eb / expm1(eb * inv_kT));
   }
-  // The bracket and fraction of element jj's patch phase (node_point_tab, with the element's phase shift and the
-  // reciprocal interval widths from the ring's image).  All lanes call it.
-  static __device__ __forceinline__ int bracket(const ChunkCtx& c, const ChunkBufs& b, int jj, double ppt, double& af) {
+  // The bracket and fraction of element jj's patch phase (node_point_tab, with the element's phase shift from the
+  // chunk's list and, unless divide, the reciprocal interval widths from the ring's image).  All lanes call it.
+  static __device__ __forceinline__ int bracket(const ChunkCtx& c, const ChunkBufs& b, int jj, double ppt, bool divide,
+                                                double& af) {
     const double xph = ppt + ((const double*)b.j)[min(jj, c.n_act - 1)] + 1.;
     // x - floor(x) for x in [1, 3]: the same exact value
     double patch = xph - (xph >= 3.0 ? 3.0 : (xph >= 2.0 ? 2.0 : 1.0));
     const double P0 = b.P[0];
     patch = patch < P0 ? patch + 1. : patch;
-    int i;
+    if (!c.mono) return vhunt_call(b.P, c.n_fine + 1, patch, af);
     double lo, hi;
-    if (c.mono) {
-      i = near_bracket(b.P, c.n_fine + 1, patch, b.hidx[clampi((int)((patch - P0) * c.n_fine), 0, c.n_fine)], lo, hi);
-    } else {
-      i = vhunt_call(b.P, c.n_fine + 1, patch, af);
-      lo = b.P[i];
-    }
-    af = (patch - lo) * b.MU[i];
+    const int i = near_bracket(b.P, c.n_fine + 1, patch, b.hidx[clampi((int)((patch - P0) * c.n_fine), 0, c.n_fine)], lo, hi);
+    af = divide ? (patch - lo) / (hi - lo) : (patch - lo) * b.MU[i];
     return i;
   }
   // flux/I and redshift of element jj where `on` (else 0 and 1)
   static __device__ __forceinline__ double point(const ChunkCtx& c, const ChunkBufs& b, int jj, bool on, double ppt,
-                                                 double& z) {
+                                                 bool divide, double& z) {
     double af;
-    const int i = bracket(c, b, jj, ppt, af);
-    const double flux = (1 - af) * b.F[i] + af * b.F[i + 1], zz = (1 - af) * b.Z[i] + af * b.Z[i + 1];
+    const int i = bracket(c, b, jj, ppt, divide, af);
+    // (fused as the tile kernel's two paths are compiled)
+    const double g = 1 - af;
+    const double flux = divide ? __fma_rn(af, b.F[i + 1], g * b.F[i]) : __fma_rn(g, b.F[i], af * b.F[i + 1]);
+    const double zz = g * b.Z[i] + af * b.Z[i + 1];
     on = on && flux != 0.0;
     z = on ? zz : 1.0;
     return on ? flux : 0.0;
@@ -1714,7 +1714,7 @@ struct BbWork {
   static __device__ __forceinline__ void point_few32(const ChunkCtx& c, const ChunkBufs& b, int jj, bool on, double ppt, double wgl,
                                                      const float* E, int n_e, float inv_kT, double* acc, unsigned& vis) {
     double afd;
-    const int i = bracket(c, b, jj, ppt, afd);
+    const int i = bracket(c, b, jj, ppt, false, afd);
     const float af = (float)afd;
     const float f0 = (float)b.F[i], flux = fmaf(af, (float)b.F[i + 1] - f0, f0);
     if (!on || flux == 0.f) return;
@@ -1760,9 +1760,9 @@ struct BbWork {
           continue;
         }
         double za = 1.0, zb = 1.0, ca = 0.0, cb = 0.0;
-        const double fa = point(c, b, ja, on_a, ppt, za);
+        const double fa = point(c, b, ja, on_a, ppt, false, za);
         double fb = 0.0;
-        if (m == 1) fb = point(c, b, jc, on_b, ppt, zb);
+        if (m == 1) fb = point(c, b, jc, on_b, ppt, false, zb);
         n_vis += (fa != 0.0 ? 1u : 0u) + (fb != 0.0 ? 1u : 0u);
         ca = fa * wgl;
         cb = fb * wgl;
@@ -1823,7 +1823,7 @@ struct BbWork {
       for (int jb = 0; jb < c.n_act; jb += 32) {
         const int jj = jb + lane;
         double flux = 0.0, z = 0;
-        flux = point(c, b, jj, jj < c.n_act, ppt, z);
+        flux = point(c, b, jj, jj < c.n_act, ppt, divide, z);
         const unsigned bal = __ballot_sync(0xffffffffu, flux != 0.0);
         if (flux != 0.0) {
           rec[__popc(bal & lanemask_lt())] = make_double2(flux * wgl, z);

@@ -36,3 +36,22 @@ def test_light_curve_bits_do_not_depend_on_the_batch(precision):
     for a, b in zip(*out):
         assert a.any() and np.array_equal(a, b)
     e.close()
+
+
+@pytest.mark.parametrize("precision", [_abi.PREC_FP64, _abi.PREC_FP32])
+@pytest.mark.parametrize("n_e", [5, 64, 65, 300])
+def test_one_point_has_the_bits_of_the_tiles(n_e, precision):
+    """One term a bin, so that no order of summation shows: the phase fraction, the lerps and the Planck factor round as
+    from tiles (which a budget without room for records selects)."""
+    out = []
+    for budget in (0, 4 << 20):
+        e = _engine(budget)
+        g = e.add_energy_grid(synth.energy_grid(n_e, 0.05, 15.0))
+        one = synth.params(mass_msun=1.4, r_eq_km=12.0, spin_hz=400.0, inclination_rad=1.1, distance_kpc=0.2,
+                           spots=[synth.spot(0.9, 0.1, 0.1, kT_keV=0.3)], atmosphere=_abi.ATM_BLACKBODY, beaming=1,
+                           n_side=32, n_bins=200, n_gl=0, n_fine=150, energy_grid=g, precision=precision)
+        one.spots[0].kind = _abi.SPOT_POINT
+        out.append(e.profile(one, want_counts=False))
+        e.close()
+    assert out[0][2].as_dict() == out[1][2].as_dict() and out[0][2].n_points > 0
+    assert np.array_equal(out[0][0], out[1][0])
