@@ -159,7 +159,7 @@ Engine::Engine(const ppm_engine_config& c) : cfg(c) {
   PPM_CUDA(cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, cfg.device));
   PPM_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
   // launch-shape overrides for experiments: PPM_PB, PPM_CHUNK, PPM_SMALL_CHUNK, PPM_NE_T, PPM_MINB, PPM_KERNEL,
-  // PPM_SETS, PPM_CPL, PPM_SPLITS, PPM_BB_NT
+  // PPM_SETS, PPM_CPL, PPM_SPLITS, PPM_BB_NT, PPM_RECORDS
   if (const char* v = std::getenv("PPM_PB")) tune.pb = std::max(1, std::atoi(v));
   if (const char* v = std::getenv("PPM_CHUNK")) tune.chunk = std::max(32, std::atoi(v));
   if (const char* v = std::getenv("PPM_SMALL_CHUNK")) tune.small_chunk = std::max(32, std::atoi(v));
@@ -170,6 +170,7 @@ Engine::Engine(const ppm_engine_config& c) : cfg(c) {
   if (const char* v = std::getenv("PPM_CPL")) tune.cpl = std::max(0, std::min(3, std::atoi(v)));
   if (const char* v = std::getenv("PPM_SPLITS")) tune.splits = std::max(0, std::atoi(v));
   if (const char* v = std::getenv("PPM_BB_NT")) tune.bb_nt = std::atoi(v) >= 512 ? 512 : (std::atoi(v) > 0 ? 256 : 0);
+  if (const char* v = std::getenv("PPM_RECORDS")) tune.records = std::max(-1, std::min(1, std::atoi(v)));
   for (int k = 0; k < 4; ++k) PPM_CUDA(cudaEventCreate(&ev[k]));
   PPM_CUDA(cudaMalloc(&d_err, sizeof(int)));
   PPM_CUDA(cudaMemset(d_err, 0, sizeof(int)));
@@ -768,13 +769,9 @@ void Engine::batch_build(BatchImpl& B, int n, const ppm_params* ps, cudaStream_t
     // are computed once (by ring_kernel) instead of by every tile.  A single profile of 408 rings, N_side 256:
     // 1640 -> 1080 us a call.  Groups with rings enough to fill the GPU keep the tiles: their rings
     // have one tile each, and their images (60 KB a ring) would be read back from HBM.
-    // Blackbody groups run from ring records too.  Light curves (few energies) do so between about 200 and 592 rings
-    // on 148 SMs only: the tiles' phase-major walk evaluates a point in fewer instructions, and loses where its rings
-    // come to little more than a round of its CTAs (one energy: 302 rings 234 -> 184 us a call, 474 rings 367 -> 231;
-    // 190 rings would take 149 -> 183 us, 683 rings 335 -> 410).
-    const bool bb_rec = (v == 1 || v == 2) && !points_only &&
-                        (ne_max > 4 || (gw[v].rings > 1.35 * sm_count && gw[v].rings < 4ll * sm_count));
-    if ((cell && npt[v] > 0) || bb_rec) {
+    bool want_rec = cell ? npt[v] > 0 : (v == 1 || v == 2) && !points_only && bb_records(gw[v], g1 - g0, bins_max);
+    if (tune.records >= 0) want_rec = tune.records > 0 && (cell || ((v == 1 || v == 2) && !points_only));
+    if (want_rec) {
       const size_t limit = B.ring_limit ? B.ring_limit : std::min<size_t>(kRingBytesMax, (size_t)cfg.memory_budget / 8);
       const size_t bytes = ring_work(shapes[v], hp.data(), order.data(), ps, g0, g1, chunk[v], rings[v]);
       unsigned char* base = nullptr;
@@ -1204,6 +1201,34 @@ size_t Engine::ring_work(const IntegrandShape& shape, const DevProfile* hp, cons
   size_t cls = 1 << 20;
   while (cls < bytes) cls <<= 1;
   return cls;
+}
+
+// Whether a blackbody group is faster from ring records than from tiles.  Times of a pass (FP64, tiles -> records;
+// FP32 alike) on 148 SMs, where the lines lie:
+//  * Light curves (at most four energies): the tiles' phase-major walk evaluates a point in fewer instructions.  It
+//    loses between one round of its CTAs and four rings an SM where a ring's segments add to few nodes' sums: one
+//    energy, 213 to 492 rings of 78 to 188 elements, 32 nodes 128..260 -> 66..130 us, 64 nodes 134..276 -> 83..176,
+//    but 96 nodes 101..199 -> 94..225 and 128 nodes 90..188 -> 107..272; four energies, 96 nodes 249..486 ->
+//    130..389, 128 nodes 233 -> 151 but 426 -> 469.  With 16 elements a ring only several energies gain (one: 54 -> 69).
+//  * Up to 64 energies a tile pays each energy with a reduction over the warp, a record with a lane: records win with
+//    the values (elements x energies) of a ring, however many rings there are: 192 values and 8 energies or more
+//    458 -> 229 us (32 energies, 546 rings) or 3052 -> 2472 (8 energies, 17298 rings); fewer values 1136 -> 875 (320)
+//    but 716 -> 759 (160), 430 -> 722 (50).  Few rings gain with less, as long as there are few sums to add:
+//    133 rings of 3 elements and 16 energies 57 -> 51 us; 128 point sources of 128 nodes and 16 energies 52 -> 86.
+//  * Above 64 energies a tile's threads own the energies, as a record's lanes do: records only spread few rings over
+//    the GPU (118 rings, 65 energies 718 -> 126 us), and lose to the tiles once these fill it (546 rings, 300 energies
+//    1293 -> 1487), or to the sums of many profiles (64 point sources, 300 energies 54 -> 82).
+bool Engine::bb_records(const GroupWork& w, int n_profiles, int bins_max) const {
+  const int ne = w.ne_max;
+  const double rings = (double)w.rings, per_ring = w.elements / std::max(1.0, rings), values = per_ring * ne;
+  const double sum_blocks = (double)n_profiles * bins_max * ((ne + 31) / 32);
+  if (ne <= 4)
+    return rings > 1.35 * sm_count && rings < 4.0 * sm_count && w.nodes_max <= (ne == 1 ? 64 : 96) &&
+           (per_ring >= 32 || ne >= 3);
+  if (ne <= 64)
+    return (values >= 192 && ne >= 8) ||
+           (rings <= 1.5 * sm_count && sum_blocks <= 5.0 * sm_count && (ne >= 12 || values >= 150));
+  return rings <= 2.0 * sm_count && w.work * ne <= 40e6 && sum_blocks <= 15.0 * sm_count;
 }
 
 // Turns a home-cell shape into the ring-record kernel's: one CTA per SM, as many chunk slots (an image and its

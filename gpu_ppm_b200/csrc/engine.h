@@ -218,6 +218,7 @@ struct Tuning {
   int sets = 0;      // home-cell kernel: warp sets per CTA (0 = as many as the kernel's threads hold)
   int cpl = 0;       // home-cell kernel: cells per lane (0 = by estimated cost)
   int splits = 0;    // phase-node splits per element chunk (0 = by the batch's work)
+  int records = -1;  // ring records: 0 = never (tiles), 1 = wherever they fit, -1 = by the rules of batch_build
   int bb_nt = 0;     // blackbody point paths (<= 64 energies): threads per CTA (0 = 512 up to 4 energies, else 256)
 };
 
@@ -308,6 +309,7 @@ class Engine {
   size_t ring_work(const IntegrandShape& shape, const DevProfile* hp, const int* order, const ppm_params* ps, int g0,
                    int g1, int chunk, RingWork& W) const;
   static bool rec_shape(IntegrandShape& s, const RingWork& W);
+  bool bb_records(const GroupWork& w, int n_profiles, int bins_max) const;
   long long tile_bound(const ppm_params& p, const DevProfile& d, int chunk, int npt) const;
   void fold_tc_prepare(Resp& r);
   // tensor-core folds of one flux and counts pool, up to 16 a launch.  error: word the kernel sets when a bounded

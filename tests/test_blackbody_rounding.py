@@ -8,16 +8,17 @@ from gpu_ppm_b200.engine import Engine
 pytestmark = pytest.mark.gpu
 
 
-def _engine(budget=0):
-    e = Engine(memory_budget=budget)
+def _engine():
+    e = Engine()
     e.load_lensing(synth.lensing("std"))
     return e
 
 
 @pytest.mark.parametrize("precision", [_abi.PREC_FP64, _abi.PREC_FP32])
-def test_light_curve_bits_do_not_depend_on_the_batch(precision):
+def test_light_curve_bits_do_not_depend_on_the_batch(monkeypatch, precision):
     """Small caps of a fast star, E / kT around 1 at their points: rings of few elements, of which several nodes share a
     warp (how many depends on the records of the batch)."""
+    monkeypatch.setenv("PPM_RECORDS", "1")
     e = _engine()
     g = e.add_energy_grid(np.array([0.36, 0.37, 0.38, 0.39]))
 
@@ -40,12 +41,13 @@ def test_light_curve_bits_do_not_depend_on_the_batch(precision):
 
 @pytest.mark.parametrize("precision", [_abi.PREC_FP64, _abi.PREC_FP32])
 @pytest.mark.parametrize("n_e", [5, 64, 65, 300])
-def test_one_point_has_the_bits_of_the_tiles(n_e, precision):
+def test_one_point_has_the_bits_of_the_tiles(monkeypatch, n_e, precision):
     """One term a bin, so that no order of summation shows: the phase fraction, the lerps and the Planck factor round as
-    from tiles (which a budget without room for records selects)."""
+    from tiles."""
     out = []
-    for budget in (0, 4 << 20):
-        e = _engine(budget)
+    for records in ("1", "0"):
+        monkeypatch.setenv("PPM_RECORDS", records)
+        e = _engine()
         g = e.add_energy_grid(synth.energy_grid(n_e, 0.05, 15.0))
         one = synth.params(mass_msun=1.4, r_eq_km=12.0, spin_hz=400.0, inclination_rad=1.1, distance_kpc=0.2,
                            spots=[synth.spot(0.9, 0.1, 0.1, kT_keV=0.3)], atmosphere=_abi.ATM_BLACKBODY, beaming=1,

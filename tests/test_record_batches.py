@@ -29,9 +29,10 @@ def _spectra(g, n):
 
 
 @pytest.mark.parametrize("n,n_e", [(2, 33), (255, 5), (256, 7), (257, 6), (700, 40)])
-def test_profiles_of_a_batch(n, n_e):
+def test_profiles_of_a_batch(monkeypatch, n, n_e):
     from gpu_ppm_b200.engine import Engine
 
+    monkeypatch.setenv("PPM_RECORDS", "1")
     e = Engine()
     e.load_lensing(synth.lensing("std"))
     g = e.add_energy_grid(synth.energy_grid(n_e, 0.1, 12.0))
@@ -44,10 +45,11 @@ def test_profiles_of_a_batch(n, n_e):
     e.close()
 
 
-def test_more_profiles_than_a_grid_dimension_holds():
+def test_more_profiles_than_a_grid_dimension_holds(monkeypatch):
     """65 540 profiles, of which the ring window leaves five with rings, the last one among them."""
     from gpu_ppm_b200.engine import Engine
 
+    monkeypatch.setenv("PPM_RECORDS", "1")
     e = Engine(max_batch=70000)
     e.load_lensing(synth.lensing("std"))
     g = e.add_energy_grid(synth.energy_grid(5, 0.1, 12.0))
