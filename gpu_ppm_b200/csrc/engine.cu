@@ -730,8 +730,8 @@ void Engine::batch_build(BatchImpl& B, int n, const ppm_params* ps, cudaStream_t
     }
     gw[vof[i]].add(ps[i], hp[k]);
   }
-  int chunk[NV], npt[NV];
-  for (int v = 0; v < NV; ++v) group_tiling(v == 3, gw[v], chunk_override, &chunk[v], &npt[v]);
+  int chunk[NV], npt[NV], npt_few[NV];
+  for (int v = 0; v < NV; ++v) group_tiling(v, gw[v], chunk_override, &chunk[v], &npt[v], &npt_few[v]);
   B.chunk = chunk[0];
   long long cap[NV] = {0, 0, 0, 0, 0};
   int start[NV + 1] = {0, 0, 0, 0, 0, 0};
@@ -763,7 +763,8 @@ void Engine::batch_build(BatchImpl& B, int n, const ppm_params* ps, cudaStream_t
     gb[v] = bins_max;
     gne[v] = ne_max;
     const bool cell = v == 0 || v == 4;
-    shapes[v] = choose_shape(cell || v == 3, v == 1, ne_max, nf_max, cells_max, maxe_max, bins_max, cell, gw[v].rings);
+    shapes[v] = choose_shape(cell || v == 3, v == 1, ne_max, nf_max, cells_max, maxe_max, bins_max, cell, gw[v].rings,
+                             cell && small_tiles(gw[v], npt_few[v]));
     if (cell && !shapes[v].cellk) throw Error(PPM_E_STATE, "home-cell NSX kernel expected for the grid");
     // a group whose nodes are split over several tiles a ring runs from ring records: each ring's sweep and slice
     // are computed once (by ring_kernel) instead of by every tile.  A single profile of 408 rings, N_side 256:
@@ -824,6 +825,7 @@ void Engine::batch_build(BatchImpl& B, int n, const ppm_params* ps, cudaStream_t
         rings[v] = RingWork{};
       }
     }
+    npt[v] = npt_few[v];
     if (!shapes[v].rec)
       for (int k = g0; k < g1; ++k) cap[v] += tile_bound(ps[order[k]], hp[k], chunk[v], npt[v]);
   }
@@ -1131,38 +1133,58 @@ void GroupWork::add(const ppm_params& p, const DevProfile& d) {
   work += Engine::spot_elements(p) * (double)pts;
   for (int s = 0; s < p.n_spots; ++s) {
     const DevSpot& sp = d.spot[s];
-    if (sp.kind == PPM_SPOT_POINT)
-      rings += sp.i_hi >= sp.i_lo ? 1 : 0;
-    else if (sp.i_hi >= sp.i_lo)
-      rings += sp.i_hi - sp.i_lo + 1;
+    const int n = sp.i_hi >= sp.i_lo ? (sp.kind == PPM_SPOT_POINT ? 1 : sp.i_hi - sp.i_lo + 1) : 0;
+    rings += n;
+    // half the spot's range of azimuths
+    const double sin_r = std::sin(std::min(std::fabs(p.spots[s].angrad1), 0.5 * pi));
+    const double half = sin_r < std::fabs(sp.s1) ? std::asin(sin_r / std::fabs(sp.s1)) : pi;
+    ranges += n * (sp.kind != PPM_SPOT_POINT && half < pi && (sp.ph1 < half || sp.ph1 > two_pi - half) ? 2 : 1);
   }
 }
 
 // Tiling of one kernel group.  The home-cell NSX and the blackbody kernels
 // keep the tuned element chunk in every batch, so that a profile's tiles cover
 // the same elements alone and in any batch; a batch with few rings is spread
-// over the SMs by splitting each tile's phase nodes instead: about 8 tiles per
-// CTA slot, but every tile keeps at least kMinNodesPerTile nodes and enough
+// over the SMs by splitting each tile's phase nodes instead: about 24 tiles an
+// SM, but every tile keeps at least kMinNodesPerTile nodes and enough
 // (element, node, energy) evaluations to outweigh its prologue (the FP64
 // fine-phase sweep and the tables it stages, repeated by every tile of a ring).
+// npt says so and, for the home-cell kernel, decides on ring records.  Where that
+// kernel runs from tiles all the same (ppm_profile_noalloc, no memory for
+// records), its two CTAs an SM take four tiles an SM (npt_few): N_side 200, 64
+// nodes, 300 energies take 484 us, with npt's 689 (633 with the three smaller CTAs
+// an SM that its 24 tiles were measured with).
 // The pooled kernel splits the elements (tile_chunk) and takes all nodes.
-void Engine::group_tiling(bool pooled, const GroupWork& w, int chunk_override, int* chunk, int* npt) const {
-  if (pooled) {
+void Engine::group_tiling(int variant, const GroupWork& w, int chunk_override, int* chunk, int* npt, int* npt_few) const {
+  if (variant == 3) {
     *chunk = chunk_override > 0 ? chunk_override : tile_chunk(w.work, w.pts_max);
-    *npt = 0;
+    *npt = *npt_few = 0;
     return;
   }
   *chunk = chunk_override > 0 ? chunk_override : tune.chunk;
   const double rings = std::max<double>(1.0, (double)w.rings);
-  const double want = 8.0 * sm_count * 3;
-  double splits_d = std::ceil(want / rings);
   // nodes per tile for kMinEvalsPerTile evaluations at the group's mean active elements per ring
   const double per_ring = std::max(1.0, std::min<double>(w.elements / rings, *chunk));
   const double min_nodes = std::max<double>(kMinNodesPerTile, std::ceil(kMinEvalsPerTile / (per_ring * w.ne_max)));
-  splits_d = std::min(splits_d, std::floor(w.nodes_max / min_nodes));
-  int splits = (int)std::max(1.0, splits_d);
-  if (tune.splits > 0) splits = std::min(tune.splits, std::max(1, w.nodes_max));
-  *npt = splits <= 1 ? 0 : (w.nodes_max + splits - 1) / splits;
+  auto nodes = [&](double want) {
+    int splits = (int)std::max(1.0, std::min(std::ceil(want), std::floor(w.nodes_max / min_nodes)));
+    if (tune.splits > 0) splits = std::min(tune.splits, std::max(1, w.nodes_max));
+    return splits <= 1 ? 0 : (w.nodes_max + splits - 1) / splits;
+  };
+  *npt = nodes(24.0 * sm_count / rings);
+  *npt_few = variant == 0 || variant == 4 ? nodes(4.0 * sm_count / std::max<double>(1.0, (double)w.ranges)) : *npt;
+}
+
+// Whether a home-cell group's tiles are so small that their prologues' latency
+// bounds them: then three CTAs an SM of six warps, where two of ten would take
+// more rounds.  16 profiles of 15 rings, 16 nodes, 60 energies (5 elements a ring):
+// a pass takes 80 us with ten warps, 65 with six (61 with the three eight-warp CTAs
+// of the kernel before pairs of records); from about 40 000 evaluations a tile on
+// both are alike, and the ten warps win with more.  Up to two tiles an SM there is
+// one round either way.
+bool Engine::small_tiles(const GroupWork& w, int npt) const {
+  const double tiles = (double)w.ranges * (npt > 0 ? (w.nodes_max + npt - 1) / npt : 1);
+  return tiles > 2.0 * sm_count && w.work * w.ne_max < 40000.0 * tiles;
 }
 
 // Sizes of the ring records of profiles g0 .. g1 - 1 (fills W's sizes, not its pointers): the bytes of one block that
@@ -1295,7 +1317,7 @@ void Engine::profile_batch(int n, const ppm_params* ps, double* flux, double* co
 }
 
 IntegrandShape Engine::choose_shape(bool nsx_kernel, bool bb_fp64, int ne_max, int nf_max, int cells_max, int maxe_max,
-                                    int bins_max, bool allow_cell, double rings) {
+                                    int bins_max, bool allow_cell, double rings, bool small_tiles) {
   // home-cell NSX kernel: cpl cells per lane (the last (cpl + 3) / cpl lanes of a warp
   // only supply slice rows), warp sets up to 512 threads
   const int span_max = cells_max - 1;
@@ -1320,7 +1342,8 @@ IntegrandShape Engine::choose_shape(bool nsx_kernel, bool bb_fp64, int ne_max, i
     if (tune.cpl > 0) cpl = std::min(tune.cpl, cmax);
     const int cell_warps = (span_max + cells_per_warp(cpl) - 1) / cells_per_warp(cpl);
     if (best >= 0 && cell_warps <= 16) {
-      int sets = std::min(16 / cell_warps, tune.sets > 0 ? tune.sets : std::max(1, kCellThreads / 32 / cell_warps));
+      const int warps = small_tiles ? kCellSmallThreads / 32 : kCellThreads / 32;
+      int sets = std::min(16 / cell_warps, tune.sets > 0 ? tune.sets : std::max(1, warps / cell_warps));
       IntegrandShape s;
       for (;;) {
         const int nt = 32 * cell_warps * sets;

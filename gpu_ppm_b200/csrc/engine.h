@@ -202,6 +202,7 @@ struct GroupWork {
   double work = 0;        // phase points, estimated from the spots' areas
   long long pts_max = 1;  // phase points per element, largest profile
   long long rings = 0;    // rings that may hold active elements
+  long long ranges = 0;   // their ranges of candidate elements (two where the spot crosses azimuth 0)
   double elements = 0;    // active elements, estimated from the spots' areas
   int nodes_max = 1;      // phase nodes per profile, largest profile
   int ne_max = 1;         // energies per profile, largest grid
@@ -301,11 +302,13 @@ class Engine {
   DevGrid dev_grid(int id);
   const double* ring_table(int N);
   const double* fine_table(int nf);
-  // rings: rings the group's spots span (sizes the blackbody phase-major walk's blocks; 0 = unknown)
+  // rings: rings the group's spots span (sizes the blackbody phase-major walk's blocks; 0 = unknown);
+  // small_tiles: see there (home-cell kernel)
   IntegrandShape choose_shape(bool nsx_kernel, bool bb_fp64, int ne_max, int nf_max, int cells_max, int maxe_max = 0,
-                              int bins_max = 0, bool allow_cell = true, double rings = 0);
+                              int bins_max = 0, bool allow_cell = true, double rings = 0, bool small_tiles = false);
+  bool small_tiles(const GroupWork& w, int npt) const;
   bool cell_kernel_takes(int grid);
-  void group_tiling(bool pooled, const GroupWork& w, int chunk_override, int* chunk, int* npt) const;
+  void group_tiling(int variant, const GroupWork& w, int chunk_override, int* chunk, int* npt, int* npt_few) const;
   size_t ring_work(const IntegrandShape& shape, const DevProfile* hp, const int* order, const ppm_params* ps, int g0,
                    int g1, int chunk, RingWork& W) const;
   static bool rec_shape(IntegrandShape& s, const RingWork& W);

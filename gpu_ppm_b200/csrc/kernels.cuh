@@ -45,6 +45,7 @@ constexpr int kMaxRecSlots = 4;
 // at 80 registers, 59.5 ms with 20 at 96, 65.2 ms with 16 at 128 (with the
 // autotuned shape 52.4 now, 61.9 before pairs of records).
 constexpr int kCellThreads = 320;
+constexpr int kCellSmallThreads = 192;  // three CTAs per SM of these where tiles are small (Engine::small_tiles)
 constexpr int kBbRecThreads = 768;  // integrand_bb_rec_kernel: 24 warps per SM at 80 registers
 constexpr int kPairFloats = 20;  // home-cell kernels: floats per pair of point records (80 bytes: 2-way bank conflicts)
 // threads of integrand_nsx_rec_kernel's CTA, one per SM: 96 registers a thread, 128 where a cell has many slots

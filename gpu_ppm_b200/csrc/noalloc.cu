@@ -178,17 +178,19 @@ void Engine::profile_noalloc(const ppm_params& p, double* flux_d, double* counts
   // kernel and tiling as batch_build gives a one-profile batch
   const bool bb64 = !nsx_atm && p.precision == PPM_PREC_FP64;
   IntegrandShape shape = choose_shape(nsx_atm, bb64, n_e, nf, g.span + 1, g.maxe, p.n_bins);
-  const bool pooled = nsx_atm && !shape.cellk;
   GroupWork w;
   w.add(p, d);
-  int chunk = 0, npt = 0;
-  group_tiling(pooled, w, 0, &chunk, &npt);
+  int chunk = 0, npt = 0, npt_few = 0;
+  group_tiling(!nsx_atm ? 1 : (shape.cellk ? 0 : 3), w, 0, &chunk, &npt, &npt_few);
   const long long cap = tile_bound(p, d, chunk, npt);
   if (cap > tile_cap)
     throw Error(PPM_E_RANGE, "ppm_profile_noalloc: the profile needs up to " + std::to_string(cap) +
                                  " work tiles, the 1 MiB scratch array holds " + std::to_string(tile_cap) +
                                  " (lower N_side or use ppm_profile)");
 
+  npt = npt_few;
+  if (shape.cellk && small_tiles(w, npt))
+    shape = choose_shape(nsx_atm, bb64, n_e, nf, g.span + 1, g.maxe, p.n_bins, true, 0, true);
   auto ck = [](cudaError_t e, const char* what) {
     if (e != cudaSuccess) throw Error(PPM_E_CUDA, std::string("ppm_profile_noalloc: ") + what + ": " + cudaGetErrorString(e));
   };
