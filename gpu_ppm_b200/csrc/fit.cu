@@ -151,13 +151,22 @@ void Engine::batch_fit(BatchImpl& B, int obs, ppm_fit* out, cudaStream_t st) {
   const int n_el = o.n_ch * o.n_bins;  // the same for every set of observed data this batch takes
   const int blocks = fit_blocks(n_el);
   if (!B.d_fit) {
-    B.d_fit_off = (long long*)B.mem.alloc(sizeof(long long) * (size_t)B.n);
-    B.d_fit = (ppm_fit*)B.mem.alloc(sizeof(ppm_fit) * (size_t)B.n);
-    B.d_fit_parts = B.mem.alloc((sizeof(FitPart) * blocks + sizeof(int)) * (size_t)B.n);
-    B.d_fit_done = (int*)((FitPart*)B.d_fit_parts + (size_t)blocks * B.n);
-    FIT_CUDA(cudaMemcpyAsync(B.d_fit_off, B.counts_off.data(), sizeof(long long) * (size_t)B.n,
-                             cudaMemcpyHostToDevice, st));
-    FIT_CUDA(cudaMemsetAsync(B.d_fit_done, 0, sizeof(int) * (size_t)B.n, st));
+    // one block, and the batch has it only when it is complete: a call that runs out of memory here leaves nothing
+    // half made to the next one
+    const size_t n = (size_t)B.n;
+    static_assert(sizeof(FitPart) % 8 == 0 && sizeof(ppm_fit) % 8 == 0, "the parts of the block are 8-byte aligned");
+    unsigned char* const mem = (unsigned char*)B.mem.alloc(
+        (sizeof(long long) + sizeof(ppm_fit) + sizeof(FitPart) * blocks + sizeof(int)) * n);
+    long long* const off = (long long*)mem;
+    ppm_fit* const fit = (ppm_fit*)(off + n);
+    FitPart* const parts = (FitPart*)(fit + n);
+    int* const done = (int*)(parts + (size_t)blocks * n);
+    FIT_CUDA(cudaMemcpyAsync(off, B.counts_off.data(), sizeof(long long) * n, cudaMemcpyHostToDevice, st));
+    FIT_CUDA(cudaMemsetAsync(done, 0, sizeof(int) * n, st));
+    B.d_fit_off = off;
+    B.d_fit_parts = parts;
+    B.d_fit_done = done;
+    B.d_fit = fit;
   }
   if (B.n > 0) {
     // (at most 65535 profiles a launch: grid y)
