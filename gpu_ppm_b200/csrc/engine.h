@@ -177,6 +177,7 @@ struct BatchImpl {
   ppm_fit* d_fit = nullptr;
   void* d_fit_parts = nullptr;     // the blocks' partial sums and their counters
   int* d_fit_done = nullptr;
+  std::mutex fit_mu;               // held by a fit call from its first use of these to the end of its wait
   BatchImpl() = default;
   BatchImpl(const BatchImpl&) = delete;
   BatchImpl& operator=(const BatchImpl&) = delete;

@@ -150,6 +150,7 @@ void Engine::batch_fit(BatchImpl& B, int obs, ppm_fit* out, cudaStream_t st) {
   if (!st) st = B.last_stream ? B.last_stream : stream;
   const int n_el = o.n_ch * o.n_bins;  // the same for every set of observed data this batch takes
   const int blocks = fit_blocks(n_el);
+  std::lock_guard<std::mutex> lk(B.fit_mu);
   if (!B.d_fit) {
     // one block, and the batch has it only when it is complete: a call that runs out of memory here leaves nothing
     // half made to the next one
