@@ -125,6 +125,7 @@ BatchImpl::~BatchImpl() {
   if (graph) cudaGraphExecDestroy(graph);
   // cached blocks are handed to the next batch at once: the last launch must be done with them
   if (mem.cache && !mem.stream && last_stream) cudaStreamSynchronize(last_stream);
+  if (ring_held) ring_held->fetch_sub((long long)ring_bytes);
 }
 
 void DeviceBuffer::release() {
@@ -733,10 +734,38 @@ void Engine::batch_build(BatchImpl& B, int n, const ppm_params* ps, cudaStream_t
   int chunk[NV], npt[NV], npt_few[NV];
   for (int v = 0; v < NV; ++v) group_tiling(v, gw[v], chunk_override, &chunk[v], &npt[v], &npt_few[v]);
   B.chunk = chunk[0];
-  long long cap[NV] = {0, 0, 0, 0, 0};
   int start[NV + 1] = {0, 0, 0, 0, 0, 0};
   for (int k = 0; k < n; ++k) start[vof[order[k]] + 1] = k + 1;
   for (int v = 1; v <= NV; ++v) start[v] = std::max(start[v], start[v - 1]);
+  // what the batch needs, from tiles too; the memory of ring records is taken after it, as far as there is some
+  long long cap[NV] = {0, 0, 0, 0, 0}, cap_total = 0;
+  for (int v = 0; v < NV; ++v) {
+    for (int k = start[v]; k < start[v + 1]; ++k) cap[v] += tile_bound(ps[order[k]], hp[k], chunk[v], npt_few[v]);
+    cap_total += cap[v];
+  }
+  if (cap_total > (1ll << 31) - 1) throw Error(PPM_E_RANGE, "batch too large for one work queue");
+  B.d_prof = (DevProfile*)B.mem.alloc(sizeof(DevProfile) * (size_t)n);
+  // the flux pool and its compensation pool in one block (cleared by one memset per pass)
+  B.d_flux = (double*)B.mem.alloc(2 * sizeof(double) * (size_t)std::max(1ll, B.flux_off[n]));
+  B.d_comp = B.d_flux + std::max(1ll, B.flux_off[n]);
+  B.d_counts = (double*)B.mem.alloc(sizeof(double) * (size_t)std::max(1ll, B.counts_off[n]));
+  Tile* tiles = (Tile*)B.mem.alloc(sizeof(Tile) * (size_t)std::max(1ll, cap_total));
+  // folds grouped by (response, n_bins, arithmetic)
+  std::map<std::tuple<int, int, int>, std::vector<FoldJob>> folds;
+  for (int i = 0; i < n; ++i) {
+    if (ps[i].response < 0) continue;
+    FoldJob j{B.flux_off[i], B.counts_off[i], ps[i].exposure_s * (1. / ps[i].n_bins)};
+    folds[std::make_tuple(ps[i].response, ps[i].n_bins, ps[i].fold)].push_back(j);
+  }
+  std::vector<FoldJob> jobs;
+  B.folds.clear();
+  for (auto& kv : folds) {
+    BatchImpl::Fold f{std::get<0>(kv.first), std::get<1>(kv.first), std::get<2>(kv.first), (int)jobs.size(),
+                      (int)kv.second.size()};
+    B.folds.push_back(f);
+    jobs.insert(jobs.end(), kv.second.begin(), kv.second.end());
+  }
+  if (!jobs.empty()) B.d_jobs = (FoldJob*)B.mem.alloc(sizeof(FoldJob) * jobs.size());
   // every spot a point source taking the phase-major walk, at most two flux additions per (bin, energy): the fused
   // point-source mode below
   bool points_only = true;
@@ -773,22 +802,11 @@ void Engine::batch_build(BatchImpl& B, int n, const ppm_params* ps, cudaStream_t
     bool want_rec = cell ? npt[v] > 0 : (v == 1 || v == 2) && !points_only && bb_records(gw[v], g1 - g0, bins_max);
     if (tune.records >= 0) want_rec = tune.records > 0 && (cell || ((v == 1 || v == 2) && !points_only));
     if (want_rec) {
-      const size_t limit = B.ring_limit ? B.ring_limit : std::min<size_t>(kRingBytesMax, (size_t)cfg.memory_budget / 8);
       const size_t bytes = ring_work(shapes[v], hp.data(), order.data(), ps, g0, g1, chunk[v], rings[v]);
       unsigned char* base = nullptr;
       IntegrandShape rs = shapes[v];
-      auto ring_alloc = [&](size_t n) {
-        return B.ring_area ? B.ring_area + B.ring_bytes : (unsigned char*)B.mem.alloc(n);
-      };
-      if (bytes && rec_shape(rs, rings[v]) && B.ring_bytes + bytes <= limit) {
-        try {
-          base = ring_alloc(bytes);
-        } catch (const Error&) {  // no room: the tiles need none
-          cudaGetLastError();
-        }
-      }
+      if (bytes && rec_shape(rs, rings[v])) base = (unsigned char*)ring_alloc(B, bytes, bytes).first;
       if (base) {
-        B.ring_bytes += (bytes + 255) / 256 * 256;
         RingWork& W = rings[v];
         W.recs = (RingRec*)base;
         W.ctr = (int4*)(W.recs + W.rec_cap);
@@ -801,20 +819,12 @@ void Engine::batch_build(BatchImpl& B, int n, const ppm_params* ps, cudaStream_t
         // node sums for two chunks a ring (a spot across azimuth 0 has two), as far as the memory goes (further chunks
         // add atomically)
         W.part_stride = ((long long)ne_max * gw[v].nodes_max * (cell ? 1 : 2) + 63) / 64 * 64;
-        const size_t each = sizeof(float) * (size_t)W.part_stride, left = limit - B.ring_bytes;
+        const size_t each = sizeof(float) * (size_t)W.part_stride;
         size_t cls = 1 << 20;
         while (cls < each * std::min<size_t>(2 * (size_t)W.n_jobs + 8, (size_t)W.rec_cap)) cls <<= 1;
-        while (cls > left && cls > 0) cls >>= 1;
-        W.part_cap = (int)std::min<size_t>(cls / each, (size_t)W.rec_cap);
-        if (W.part_cap > 0) {
-          try {
-            W.parts = ring_alloc(cls);
-            B.ring_bytes += cls;
-          } catch (const Error&) {
-            cudaGetLastError();
-            W.part_cap = 0;
-          }
-        }
+        const auto parts = ring_alloc(B, cls, each);
+        W.parts = parts.first;
+        W.part_cap = (int)std::min<size_t>(parts.second / each, (size_t)W.rec_cap);
         int job = 0;
         for (int k = g0; k < g1; ++k)
           for (int s = 0; s < kMaxSpots; ++s) {
@@ -826,18 +836,7 @@ void Engine::batch_build(BatchImpl& B, int n, const ppm_params* ps, cudaStream_t
       }
     }
     npt[v] = npt_few[v];
-    if (!shapes[v].rec)
-      for (int k = g0; k < g1; ++k) cap[v] += tile_bound(ps[order[k]], hp[k], chunk[v], npt[v]);
   }
-  long long cap_total = 0;
-  for (int v = 0; v < NV; ++v) cap_total += cap[v];
-  if (cap_total > (1ll << 31) - 1) throw Error(PPM_E_RANGE, "batch too large for one work queue");
-  B.d_prof = (DevProfile*)B.mem.alloc(sizeof(DevProfile) * (size_t)n);
-  // the flux pool and its compensation pool in one block (cleared by one memset per pass)
-  B.d_flux = (double*)B.mem.alloc(2 * sizeof(double) * (size_t)std::max(1ll, B.flux_off[n]));
-  B.d_comp = B.d_flux + std::max(1ll, B.flux_off[n]);
-  B.d_counts = (double*)B.mem.alloc(sizeof(double) * (size_t)std::max(1ll, B.counts_off[n]));
-  Tile* tiles = (Tile*)B.mem.alloc(sizeof(Tile) * (size_t)std::max(1ll, cap_total));
   // uploads: from the caller's pinned area when it has room (asynchronous), else from the pageable source (the
   // copy returns once the source is staged, ordered on the batch's stream), else synchronous
   size_t staged = 0;
@@ -903,23 +902,7 @@ void Engine::batch_build(BatchImpl& B, int n, const ppm_params* ps, cudaStream_t
     const int zeros[16] = {0};
     upload(B.d_ctrl, zeros, sizeof(zeros));
   }
-  // folds grouped by (response, n_bins, arithmetic)
-  std::map<std::tuple<int, int, int>, std::vector<FoldJob>> folds;
-  for (int i = 0; i < n; ++i) {
-    if (ps[i].response < 0) continue;
-    FoldJob j{B.flux_off[i], B.counts_off[i], ps[i].exposure_s * (1. / ps[i].n_bins)};
-    folds[std::make_tuple(ps[i].response, ps[i].n_bins, ps[i].fold)].push_back(j);
-  }
-  std::vector<FoldJob> jobs;
-  B.folds.clear();
-  for (auto& kv : folds) {
-    BatchImpl::Fold f{std::get<0>(kv.first), std::get<1>(kv.first), std::get<2>(kv.first), (int)jobs.size(),
-                      (int)kv.second.size()};
-    B.folds.push_back(f);
-    jobs.insert(jobs.end(), kv.second.begin(), kv.second.end());
-  }
   if (!jobs.empty()) {
-    B.d_jobs = (FoldJob*)B.mem.alloc(sizeof(FoldJob) * jobs.size());
     upload(B.d_jobs, jobs.data(), sizeof(FoldJob) * jobs.size());
     B.h2d_bytes += sizeof(FoldJob) * jobs.size();
   }
@@ -1185,6 +1168,39 @@ void Engine::group_tiling(int variant, const GroupWork& w, int chunk_override, i
 bool Engine::small_tiles(const GroupWork& w, int npt) const {
   const double tiles = (double)w.ranges * (npt > 0 ? (w.nodes_max + npt - 1) / npt : 1);
   return tiles > 2.0 * sm_count && w.work * w.ne_max < 40000.0 * tiles;
+}
+
+// Memory of a batch's ring records: `bytes`, or as much as a half, a quarter, .. of it fits but at least `least`; from
+// the batch's area, or from its arena within the batch's share (kRingBytesMax) and the engine's (an eighth of the
+// budget, all batches that exist together).  Its address and size; nullptr and 0: no room, or none to be had.
+std::pair<void*, size_t> Engine::ring_alloc(BatchImpl& B, size_t bytes, size_t least) {
+  auto up = [](size_t v) { return (v + 255) / 256 * 256; };
+  if (B.ring_limit) {
+    while (bytes >= least && B.ring_bytes + up(bytes) > B.ring_limit) bytes >>= 1;
+    if (!B.ring_area || bytes < least) return {nullptr, 0};
+    unsigned char* p = B.ring_area + B.ring_bytes;
+    B.ring_bytes += up(bytes);
+    return {p, bytes};
+  }
+  for (; bytes >= least; bytes >>= 1) {
+    if (B.ring_bytes + up(bytes) > kRingBytesMax) continue;
+    const long long n = (long long)up(bytes);
+    if (ring_held.fetch_add(n) + n > (long long)cfg.memory_budget / 8) {
+      ring_held.fetch_sub(n);
+      continue;
+    }
+    try {
+      void* p = B.mem.alloc(up(bytes));
+      B.ring_held = &ring_held;
+      B.ring_bytes += up(bytes);
+      return {p, bytes};
+    } catch (const Error&) {  // the device is full: what is left is not for memory that the tiles do without
+      cudaGetLastError();
+      ring_held.fetch_sub(n);
+      break;
+    }
+  }
+  return {nullptr, 0};
 }
 
 // Sizes of the ring records of profiles g0 .. g1 - 1 (fills W's sizes, not its pointers): the bytes of one block that

@@ -158,9 +158,11 @@ struct BatchImpl {
   };
   std::vector<Group> groups;
   std::vector<Fold> folds;
-  // device memory that ring records may take (0: the engine's default share) and what they took
+  // device memory of ring records: what they took, and the area they take it from (ring_limit bytes, a multiple of 256;
+  // a limit without an area: none).  0: from mem, counted in the engine's ring_held
   size_t ring_limit = 0, ring_bytes = 0;
-  unsigned char* ring_area = nullptr;  // their memory (ring_limit bytes, a multiple of 256); nullptr: from mem
+  unsigned char* ring_area = nullptr;
+  std::atomic<long long>* ring_held = nullptr;
   size_t h2d_bytes = 0;
   // pinned host memory the build stages its uploads in, when given (serving: one area per stream slot, untouched
   // until the slot's batch has finished, so the copies run asynchronously); pageable copies otherwise
@@ -310,6 +312,7 @@ class Engine {
   bool small_tiles(const GroupWork& w, int npt) const;
   bool cell_kernel_takes(int grid);
   void group_tiling(int variant, const GroupWork& w, int chunk_override, int* chunk, int* npt, int* npt_few) const;
+  std::pair<void*, size_t> ring_alloc(BatchImpl& B, size_t bytes, size_t least);
   size_t ring_work(const IntegrandShape& shape, const DevProfile* hp, const int* order, const ppm_params* ps, int g0,
                    int g1, int chunk, RingWork& W) const;
   static bool rec_shape(IntegrandShape& s, const RingWork& W);
@@ -340,6 +343,7 @@ class Engine {
   // pinned areas of the synchronous calls, made at the first one, used under the lock: the batch build's uploads, the
   // outputs of small calls
   HostBuffer h_up, h_down;
+  std::atomic<long long> ring_held{0};  // device memory of the ring records of the batches that exist (serving's areas apart)
   void pin_uploads(BatchImpl& B);
   std::map<int, double*> ring_tabs, fine_tabs;
   std::map<int, std::vector<double>> host_rings;

@@ -163,12 +163,19 @@ typedef struct ppm_engine_config {
   int32_t device;             /* CUDA device ordinal */
   int32_t max_batch;          /* largest batch ppm_profile_batch accepts (profiles) */
   int64_t memory_budget;      /* bytes of device memory for in-flight request state (0 = 64 GiB); also
-                                 the most device memory the engine keeps cached between synchronous calls */
+                                 the most device memory the engine keeps cached between synchronous calls.
+                                 Beside its outputs a batch of few rings takes up to 1 GiB for ring records
+                                 (one profile of N_side 256, 64 x 2 nodes, 300 energies: 160 MB; a batch
+                                 object keeps it until it is destroyed), all batches that exist together up
+                                 to an eighth of the budget; batches beyond that, or on a full device, run
+                                 without, slower and with the same results */
   int32_t autotune;           /* 1: time candidate launch shapes at first use */
   int32_t n_streams;          /* serving: concurrent batches in flight (0 = 3: batches overlap on the GPU
                                  while the next is staged); the server also pins n_streams + 4 staging
                                  buffers of 32 MiB and, per stream, a small upload area for the batch
-                                 build's host-to-device copies when it starts (first ppm_submit) */
+                                 build's host-to-device copies when it starts (first ppm_submit), and takes
+                                 256 MiB of device memory per stream for ring records, beside the budget
+                                 (all of them at most an eighth of it) */
 } ppm_engine_config;
 
 /* ---- engine ---------------------------------------------------------------- */
