@@ -800,7 +800,7 @@ __device__ __forceinline__ void pair_window(const float* ra, const float* rb, in
 // differences shared by neighbouring cells.
 template <int C>
 __device__ __forceinline__ void window_cubics(const f32x2 (&h)[C + 4], Cubic2 (&Q)[C + 1]) {
-  const f32x2 half = pk(0.5f, 0.5f), sixth = pk(1.f / 6.f, 1.f / 6.f), msixth = pk(-1.f / 6.f, -1.f / 6.f);
+  const f32x2 half = pk(0.5f, 0.5f), sixth = pk(1.f / 6.f, 1.f / 6.f);
   f32x2 d1[C + 3], d2[C + 2], d3[C + 1];
 #pragma unroll
   for (int j = 0; j < C + 3; ++j) d1[j] = sub2(h[j + 1], h[j]);
@@ -813,11 +813,7 @@ __device__ __forceinline__ void window_cubics(const f32x2 (&h)[C + 4], Cubic2 (&
     Q[i].x = h[i + 1];
     Q[i].z = mul2(half, d2[i]);
     Q[i].w = mul2(d3[i], sixth);
-#ifdef PPM_YB
-    Q[i].y = fma2(d3[i], msixth, fma2(half, d2[i], d1[i]));
-#else
     Q[i].y = sub2(fma2(half, d2[i], d1[i]), Q[i].w);
-#endif
   }
 }
 
