@@ -51,6 +51,7 @@
 #include <vector>
 
 #include "engine.h"
+#include "narrow.cuh"
 
 namespace ppm {
 
@@ -151,20 +152,9 @@ __device__ __forceinline__ void load_row8(const double* src, bool vec, int k0, i
   }
 }
 
-// d rounded to the nearest FP32 value (ties to even) where that is a normal number, or d is zero or subnormal; ok is
-// left alone then and cleared otherwise.  On the integer pipe, which has room: the conversion instruction runs on the
-// special-function pipe, 35 % of whose issue the kernel took (12 % with this).
+// d rounded to the nearest FP32 value (narrow_bits); ok is left alone, or cleared where the result is not meant.
 __device__ __forceinline__ float narrow(double d, bool& ok) {
-  const uint32_t hi = (uint32_t)__double2hiint(d), lo = (uint32_t)__double2loint(d), mag = hi & 0x7fffffffu;
-  uint32_t t = __funnelshift_l(lo, hi, 3);  // 23 bits of the significand under 9 of the exponent
-  // round up when the 29 bits below are above half, or half and t is odd; exponent bias 1023 -> 127
-  const uint32_t rest = (lo << 3) | (t & 1u);
-  uint32_t unused;
-  asm("add.cc.u32 %0, %2, 0x7fffffff;\n\taddc.u32 %1, %3, 0x40000000;" : "=r"(unused), "=r"(t) : "r"(rest), "r"(t));
-  (void)unused;
-  if (mag < 0x00100000u) t = 0;
-  ok = ok && (mag < 0x00100000u || mag - 0x38100000u < 0x0fe00000u);
-  return __uint_as_float((t & 0x7fffffffu) | (hi & 0x80000000u));
+  return __uint_as_float(narrow_bits((uint32_t)__double2hiint(d), (uint32_t)__double2loint(d), ok));
 }
 
 // Splits eight values into BF16 hi / lo parts and stores them, two to a core matrix row of each part.
