@@ -1255,7 +1255,9 @@ size_t Engine::ring_work(const IntegrandShape& shape, const DevProfile* hp, cons
 //    133 rings of 3 elements and 16 energies 57 -> 51 us; 128 point sources of 128 nodes and 16 energies 52 -> 86.
 //  * Above 64 energies a tile's threads own the energies, as a record's lanes do: records only spread few rings over
 //    the GPU (118 rings, 65 energies 718 -> 126 us), and lose to the tiles once these fill it (546 rings, 300 energies
-//    1293 -> 1487), or to the sums of many profiles (64 point sources, 300 energies 54 -> 82).
+//    1293 -> 1487) or have work enough (the tiles' divisions count for less with many energies: one profile, 84e6
+//    evaluations, 300 energies 401 -> 417; 93e6, 80 energies 631 -> 461), or to the sums of many profiles (64 point
+//    sources, 300 energies 54 -> 82).
 bool Engine::bb_records(const GroupWork& w, int n_profiles, int bins_max) const {
   const int ne = w.ne_max;
   const double rings = (double)w.rings, per_ring = w.elements / std::max(1.0, rings), values = per_ring * ne;
@@ -1266,7 +1268,7 @@ bool Engine::bb_records(const GroupWork& w, int n_profiles, int bins_max) const 
   if (ne <= 64)
     return (values >= 192 && ne >= 8) ||
            (rings <= 1.5 * sm_count && sum_blocks <= 5.0 * sm_count && (ne >= 12 || values >= 150));
-  return rings <= 2.0 * sm_count && w.work * ne <= 40e6 && sum_blocks <= 15.0 * sm_count;
+  return rings <= 2.0 * sm_count && w.work * ne <= std::max(40e6, 8e9 / ne) && sum_blocks <= 15.0 * sm_count;
 }
 
 // Turns a home-cell shape into the ring-record kernel's: one CTA per SM, as many chunk slots (an image and its
