@@ -795,11 +795,15 @@ void Engine::batch_build(BatchImpl& B, int n, const ppm_params* ps, cudaStream_t
     shapes[v] = choose_shape(cell || v == 3, v == 1, ne_max, nf_max, cells_max, maxe_max, bins_max, cell, gw[v].rings,
                              cell && small_tiles(gw[v], npt_few[v]));
     if (cell && !shapes[v].cellk) throw Error(PPM_E_STATE, "home-cell NSX kernel expected for the grid");
-    // a group whose nodes are split over several tiles a ring runs from ring records: each ring's sweep and slice
-    // are computed once (by ring_kernel) instead of by every tile.  A single profile of 408 rings, N_side 256:
-    // 1640 -> 1080 us a call.  Groups with rings enough to fill the GPU keep the tiles: their rings
-    // have one tile each, and their images (60 KB a ring) would be read back from HBM.
-    bool want_rec = cell ? npt[v] > 0 : (v == 1 || v == 2) && !points_only && bb_records(gw[v], g1 - g0, bins_max);
+    // A home-cell group whose nodes would be split over several tiles a ring runs from ring records: each ring's sweep
+    // and slice are computed once (by ring_kernel) instead of by every tile, and any CTA takes any node.  One profile of
+    // 408 rings, N_side 256, 128 nodes, 300 energies: 1192 us a call from tiles, 1083 from records; of 34 rings with 5
+    // elements 0.69 of the tiles' time on average.  Groups with rings enough to fill the GPU keep the tiles: their
+    // rings have one tile each, and their images (60 KB a ring) would be read back from HBM.  So do many profiles with
+    // few elements a ring, whose node sums are most of the records' cost (14 profiles: alike; 24 of 3 to 20 elements
+    // 1.0 to 1.1 of the tiles' time, 64 of them 1.1 to 1.3; 20 elements and more 0.96).
+    bool want_rec = cell ? npt[v] > 0 && (g1 - g0 <= 12 || gw[v].elements >= 20.0 * (double)gw[v].rings)
+                         : (v == 1 || v == 2) && !points_only && bb_records(gw[v], g1 - g0, bins_max);
     if (tune.records >= 0) want_rec = tune.records > 0 && (cell || ((v == 1 || v == 2) && !points_only));
     if (want_rec) {
       const size_t bytes = ring_work(shapes[v], hp.data(), order.data(), ps, g0, g1, chunk[v], rings[v]);
