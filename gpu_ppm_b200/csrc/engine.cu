@@ -796,8 +796,8 @@ void Engine::batch_build(BatchImpl& B, int n, const ppm_params* ps, cudaStream_t
                              cell && small_tiles(gw[v], npt_few[v]));
     if (cell && !shapes[v].cellk) throw Error(PPM_E_STATE, "home-cell NSX kernel expected for the grid");
     // A home-cell group whose nodes would be split over several tiles a ring runs from ring records: each ring's sweep
-    // and slice are computed once (by ring_kernel) instead of by every tile, and any CTA takes any node.  One profile of
-    // 408 rings, N_side 256, 128 nodes, 300 energies: 1192 us a call from tiles, 1083 from records; of 34 rings with 5
+    // and slice are computed once (by ring_kernel) instead of by every tile, and any CTA takes any node.  One profile
+    // of 408 rings, N_side 256, 128 nodes, 300 energies: 1192 us a call from tiles, 1083 from records; of 34 rings with 5
     // elements 0.69 of the tiles' time on average.  Groups with rings enough to fill the GPU keep the tiles: their
     // rings have one tile each, and their images (60 KB a ring) would be read back from HBM.  So do many profiles with
     // few elements a ring, whose node sums are most of the records' cost (14 profiles: alike; 24 of 3 to 20 elements
@@ -814,9 +814,10 @@ void Engine::batch_build(BatchImpl& B, int n, const ppm_params* ps, cudaStream_t
         RingWork& W = rings[v];
         W.recs = (RingRec*)base;
         W.ctr = (int4*)(W.recs + W.rec_cap);
-        W.lists = (unsigned char*)(base + ((sizeof(RingRec) + sizeof(int4)) * ((size_t)W.rec_cap + 1) + 255) / 256 * 256);
-        W.by_profile = (int*)(W.lists + ((size_t)W.elem_bytes * (size_t)W.list_cap + 255) / 256 * 256);
-        W.data = (unsigned char*)W.by_profile + (sizeof(int) * (size_t)W.per_job * (size_t)W.n_jobs + 255) / 256 * 256;
+        auto up = [](size_t b) { return (b + 255) / 256 * 256; };
+        W.lists = (unsigned char*)base + up((sizeof(RingRec) + sizeof(int4)) * ((size_t)W.rec_cap + 1));
+        W.by_profile = (int*)(W.lists + up((size_t)W.elem_bytes * (size_t)W.list_cap));
+        W.data = (unsigned char*)W.by_profile + up(sizeof(int) * (size_t)W.per_job * (size_t)W.n_jobs);
         W.n_recs = B.d_ctrl + 3 * v;
         W.list_next = B.d_ctrl + 3 * v + 1;
         shapes[v] = rs;
@@ -922,7 +923,9 @@ void Engine::batch_enqueue(BatchImpl& B, cudaStream_t st, cudaEvent_t* events) {
     PPM_CUDA(cudaMemsetAsync(B.d_flux, 0, 2 * sizeof(double) * (size_t)std::max(1ll, B.flux_off[n]), st));
     PPM_CUDA(cudaMemsetAsync(B.d_ctrl, 0, B.small_bytes, st));
     for (const auto& G : B.groups)
-      PPM_CUDA(G.args.shape.rec ? launch_rings(G.args, st) : launch_plan(B.d_prof + G.g0, G.g1 - G.g0, lens, G.args.queue, G.chunk, G.npt, st));
+      PPM_CUDA(G.args.shape.rec
+                   ? launch_rings(G.args, st)
+                   : launch_plan(B.d_prof + G.g0, G.g1 - G.g0, lens, G.args.queue, G.chunk, G.npt, st));
   }
   if (events) PPM_CUDA(cudaEventRecord(events[1], st));
   {
@@ -1142,7 +1145,8 @@ void GroupWork::add(const ppm_params& p, const DevProfile& d) {
 // nodes, 300 energies take 484 us, with npt's 689 (633 with the three smaller CTAs
 // an SM that its 24 tiles were measured with).
 // The pooled kernel splits the elements (tile_chunk) and takes all nodes.
-void Engine::group_tiling(int variant, const GroupWork& w, int chunk_override, int* chunk, int* npt, int* npt_few) const {
+void Engine::group_tiling(int variant, const GroupWork& w, int chunk_override, int* chunk, int* npt,
+                          int* npt_few) const {
   if (variant == 3) {
     *chunk = chunk_override > 0 ? chunk_override : tile_chunk(w.work, w.pts_max);
     *npt = *npt_few = 0;
@@ -1209,8 +1213,8 @@ std::pair<void*, size_t> Engine::ring_alloc(BatchImpl& B, size_t bytes, size_t l
 
 // Sizes of the ring records of profiles g0 .. g1 - 1 (fills W's sizes, not its pointers): the bytes of one block that
 // holds the records, their counters, the element lists and the images, 0 if there is nothing to hold or too much.
-size_t Engine::ring_work(const IntegrandShape& shape, const DevProfile* hp, const int* order, const ppm_params* ps, int g0,
-                         int g1, int chunk, RingWork& W) const {
+size_t Engine::ring_work(const IntegrandShape& shape, const DevProfile* hp, const int* order, const ppm_params* ps,
+                         int g0, int g1, int chunk, RingWork& W) const {
   long long recs = 0, list = 0, jobs = 0, per_job = 1;
   for (int k = g0; k < g1; ++k) {
     recs += tile_bound(ps[order[k]], hp[k], chunk, 0);
@@ -1237,8 +1241,9 @@ size_t Engine::ring_work(const IntegrandShape& shape, const DevProfile* hp, cons
   W.per_job = (int)per_job;
   W.n_profiles = g1 - g0;
   W.chunk = chunk;
-  const size_t bytes = up((sizeof(RingRec) + sizeof(int4)) * ((size_t)recs + 1)) + up((size_t)W.elem_bytes * (size_t)list) +
-                       up(sizeof(int) * (size_t)per_job * (size_t)jobs) + (size_t)W.stride * (size_t)jobs;
+  const size_t bytes = up((sizeof(RingRec) + sizeof(int4)) * ((size_t)recs + 1)) +
+                       up((size_t)W.elem_bytes * (size_t)list) + up(sizeof(int) * (size_t)per_job * (size_t)jobs) +
+                       (size_t)W.stride * (size_t)jobs;
   // whole powers of two, so that the blocks of a sampler's next proposals fit the cached ones
   size_t cls = 1 << 20;
   while (cls < bytes) cls <<= 1;
@@ -1251,7 +1256,8 @@ size_t Engine::ring_work(const IntegrandShape& shape, const DevProfile* hp, cons
 //    loses between one round of its CTAs and four rings an SM where a ring's segments add to few nodes' sums: one
 //    energy, 213 to 492 rings of 78 to 188 elements, 32 nodes 128..260 -> 66..130 us, 64 nodes 134..276 -> 83..176,
 //    but 96 nodes 101..199 -> 94..225 and 128 nodes 90..188 -> 107..272; four energies, 96 nodes 249..486 ->
-//    130..389, 128 nodes 233 -> 151 but 426 -> 469.  With 16 elements a ring only several energies gain (one: 54 -> 69).
+//    130..389, 128 nodes 233 -> 151 but 426 -> 469.  With 16 elements a ring only several energies gain (one: 54 ->
+//    69).
 //  * Up to 64 energies a tile pays each energy with a reduction over the warp, a record with a lane: records win with
 //    the values (elements x energies) of a ring, however many rings there are: 192 values and 8 energies or more
 //    458 -> 229 us (32 energies, 546 rings) or 3052 -> 2472 (8 energies, 17298 rings); fewer values 1136 -> 875 (320)

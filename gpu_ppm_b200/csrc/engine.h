@@ -343,7 +343,8 @@ class Engine {
   // pinned areas of the synchronous calls, made at the first one, used under the lock: the batch build's uploads, the
   // outputs of small calls
   HostBuffer h_up, h_down;
-  std::atomic<long long> ring_held{0};  // device memory of the ring records of the batches that exist (serving's areas apart)
+  // device memory of the ring records of the batches that exist (serving's areas apart)
+  std::atomic<long long> ring_held{0};
   void pin_uploads(BatchImpl& B);
   std::map<int, double*> ring_tabs, fine_tabs;
   std::map<int, std::vector<double>> host_rings;

@@ -2,10 +2,12 @@
 // FP64/FP32 variants) and SIMT response folds.
 //
 // Two forms.  Batches whose rings fill the GPU run from tiles: a CTA per tile does
-// all of the steps below.  Small ones (a single profile, a served batch) run from
-// ring records: ring_kernel does steps 1 to 5 once a ring, the *_rec kernels do
-// step 6 for a ring's phase nodes, any CTA taking any node, and sum_parts_kernel
-// adds the stored node sums.  The results are the same bits.
+// all of the steps below.  Small ones (a single profile, a served batch) and
+// blackbody spectra run from ring records: ring_kernel does steps 1 to 5 once a
+// ring, the *_rec kernels do step 6 for a ring's phase nodes, any CTA taking any
+// node, and sum_parts_kernel adds the stored node sums.  NSX results are the same
+// bits in both forms; blackbody results agree to about 1e-16 (FP64 sums in another
+// order), FP32 blackbody ones to some units of 2^-23 times E / kT.
 //
 // Integrand structure (one CTA per tile = candidate elements of one ring of
 // one spot of one profile; CTAs pull tiles from a device queue, except in the
@@ -881,8 +883,8 @@ __device__ __forceinline__ void pair_slots(const Cubic2 (&Q)[C + 1], const float
 
 // Fills a context (one thread); MAXE slots a cell.
 template <int MAXE, int MOST>
-__device__ __forceinline__ void fill_ctx(ChunkCtx& c, const DevProfile& p, const DevSpot& sp, int ring, int n_act, bool mono,
-                                         bool held) {
+__device__ __forceinline__ void fill_ctx(ChunkCtx& c, const DevProfile& p, const DevSpot& sp, int ring, int n_act,
+                                         bool mono, bool held) {
   constexpr int NG = slot_groups(MAXE, MOST), MG = MAXE / NG;
   const RingPhi rp = sp.kind == 1 ? RingPhi{0.0, 0.0} : healpix_ring_phi(p.n_side, ring);
   c.dphi = rp.dphi;
@@ -928,7 +930,8 @@ struct Node {
 };
 
 // walk_bracket from a bracket that is right or at most two too low for almost every x (the table's: phase_o's widths
-// differ from 1 / n_fine by the delays' few per cent): two steps without a branch, the walk where a lane needs it.  All lanes of a warp call it.  lo, hi: xx at the bracket's ends.
+// differ from 1 / n_fine by the delays' few per cent): two steps without a branch, the walk where a lane needs it.
+// All lanes of a warp call it.  lo, hi: xx at the bracket's ends.
 __device__ __forceinline__ int near_bracket(const double* xx, int n, double x, int i, double& lo, double& hi) {
   i += x >= xx[i + 1] && i < n - 2 ? 1 : 0;
   i += x >= xx[i + 1] && i < n - 2 ? 1 : 0;
@@ -1310,8 +1313,8 @@ __device__ __forceinline__ int nsx_taps(const DevNsx& X, const DevProfile& p, co
 
 // Reduces the NSX table into S[E][mu] (row stride ldS, Sx = row 0, in shared or
 // global memory); all threads of the block, block barriers inside.
-__device__ __forceinline__ void build_slice(const DevNsx& X, int ldS, int C, const float* tapw, const int* tapo, int ntap,
-                                            float* Sx) {
+__device__ __forceinline__ void build_slice(const DevNsx& X, int ldS, int C, const float* tapw, const int* tapo,
+                                            int ntap, float* Sx) {
   const int tid = threadIdx.x, nt = blockDim.x, nE = X.nE, nmu = X.nmu;
   const int n_el = nE * nmu;
   if (ldS == nmu) {
@@ -1565,7 +1568,7 @@ __global__ void __launch_bounds__(256) ring_kernel(const KernelArgs a) {
 
 // Work of the home-cell NSX kernel: one node at a time.  Bound by the FMA pipe and the register file's ports, as over
 // tiles.  What a node is added to no longer shows: its sums are stored, not added atomically.  N_side 256, two spots,
-// 64 bins x 2 nodes, 300 energies: 1492 us from tiles, 937 with rings and sum from records.
+// 64 bins x 2 nodes, 300 energies: 1071 us with plan and sum from tiles, 973 with rings and sum from records.
 template <int MAXE, int C, int NTMAX>
 struct NsxWork : SetPlace<C> {
   const KernelArgs& a;
@@ -1621,9 +1624,8 @@ __global__ void __launch_bounds__(NTMAX, 1) integrand_nsx_rec_kernel(const Kerne
 // sums are FP64 in every arithmetic; a node's are combined over the lanes and
 // stored.  Bound by issue and latency (51 % of the issue slots, the FP64 pipe at
 // 16 %; 32 us for 48 rings, 64 energies, 32 x 2 nodes): the point's bracket walk
-// and the node's bookkeeping, not the Planck factor, whose exponential in another
-// form changed nothing.  That spectrum takes 425 us a call from tiles, 90 from
-// records.
+// and the node's bookkeeping.  That spectrum takes 458 us a call from tiles, 96
+// from records; where each form is used: Engine::bb_records.
 // FP32 arithmetic keeps the form of the tile kernel's path for the grid's size.
 template <typename Real>
 struct BbWork {
@@ -1647,7 +1649,8 @@ struct BbWork {
     c.n_nodes *= passes;  // as ring_kernel counted the chunk's tasks
     // nodes per take: about 2048 points, but takes for every warp several times over
     const long long tasks = (long long)min(*a.rings.n_recs, a.rings.rec_cap) * c.n_nodes;
-    c.take = (int)max(1ll, min(min((long long)c.u_mod / 8, 2048ll / max(q.n_act, 8)), tasks / (gridDim.x * (blockDim.x / 8))));
+    const long long per_take = min((long long)c.u_mod / 8, 2048ll / max(q.n_act, 8));
+    c.take = (int)max(1ll, min(per_take, tasks / (gridDim.x * (blockDim.x / 8))));
     int ll = 0;
     if (c.per_pass > kPhaseMajorMaxE)
       while (ll < 5 && (1 << ll) < c.per_pass) ++ll;
@@ -1674,7 +1677,8 @@ struct BbWork {
   }
   // The same of two points, in one block, so that the two evaluations overlap and share their constants; hidden points
   // have c = 0 and z = 1.  A point's value is its own: what the other lanes hold depends on the batch.
-  static __device__ __forceinline__ double planck_pair(double ca, double za, double cb, double zb, double E, double inv_kT) {
+  static __device__ __forceinline__ double planck_pair(double ca, double za, double cb, double zb, double E,
+                                                       double inv_kT) {
     const double ea = E * za, eb = E * zb;
     return ca * (ea * ea * ea / expm1(ea * inv_kT)) + cb * (eb * eb * eb / expm1(eb * inv_kT));
   }
@@ -1689,7 +1693,8 @@ struct BbWork {
     patch = patch < P0 ? patch + 1. : patch;
     if (!c.mono) return vhunt_call(b.P, c.n_fine + 1, patch, af);
     double lo, hi;
-    const int i = near_bracket(b.P, c.n_fine + 1, patch, b.hidx[clampi((int)((patch - P0) * c.n_fine), 0, c.n_fine)], lo, hi);
+    const int k = clampi((int)((patch - P0) * c.n_fine), 0, c.n_fine);
+    const int i = near_bracket(b.P, c.n_fine + 1, patch, b.hidx[k], lo, hi);
     af = divide ? (patch - lo) / (hi - lo) : (patch - lo) * b.MU[i];
     return i;
   }
@@ -1707,8 +1712,9 @@ struct BbWork {
     return on ? flux : 0.0;
   }
   // one point at the grid's few energies, in FP32 arithmetic: the phase-major walk's form (pm_walk)
-  static __device__ __forceinline__ void point_few32(const ChunkCtx& c, const ChunkBufs& b, int jj, bool on, double ppt, double wgl,
-                                                     const float* E, int n_e, float inv_kT, double* acc, unsigned& vis) {
+  static __device__ __forceinline__ void point_few32(const ChunkCtx& c, const ChunkBufs& b, int jj, bool on, double ppt,
+                                                     double wgl, const float* E, int n_e, float inv_kT, double* acc,
+                                                     unsigned& vis) {
     double afd;
     const int i = bracket(c, b, jj, ppt, false, afd);
     const float af = (float)afd;
@@ -2577,7 +2583,7 @@ __device__ __forceinline__ void dd_add(double& s, double& c, double x) {
 // Double-double sums: the exact sum to about 1e-32, in any order of the records, as the pool's compensated atomics
 // give it; what the atomics added is included.  Bound by the read of the node sums, from L2 for a single profile:
 // 125 MB in 69 us with 12 loads in flight a thread and 256-thread blocks (512 threads, 8 loads: 83 to 108; 1024
-// threads, one after the other: 177), of an 1080 us call that took 1640 with every node's compensated atomics.
+// threads, one after the other: 177), of an 1080 us call.
 template <typename T>
 __global__ void __launch_bounds__(kSumThreads) sum_parts_kernel(const KernelArgs a, int Q, int p0) {
   const RingWork& W = a.rings;
@@ -2606,7 +2612,8 @@ __global__ void __launch_bounds__(kSumThreads) sum_parts_kernel(const KernelArgs
     if (r < W.part_cap) {
       const int sp = entry & 1, at = atomicAdd(&s_n[sp], n_gl);
       for (int g = 0; g < n_gl; ++g)
-        s_ofs[sp ? kSumList - 1 - (at + g) : at + g] = (unsigned)(r * W.part_stride) + (unsigned)(g * n_e * (int)(sizeof(T) / 4));
+        s_ofs[sp ? kSumList - 1 - (at + g) : at + g] =
+            (unsigned)(r * W.part_stride) + (unsigned)(g * n_e * (int)(sizeof(T) / 4));
     }
     __syncthreads();
     const int n0 = s_n[0], n = n0 + s_n[1];

@@ -41,9 +41,9 @@ IntegrandShape make_shape(bool nsx, int nt, int ne_t, int pb, int max_cand, int 
 
 constexpr int kMaxRecSlots = 4;
 // Home-cell kernel over tiles: two CTAs of this many threads per SM.  The record loop is bound by the FMA pipe and the
-// register file's ports, not by the number of warps: 96 profiles of the batching prior took 64.4 ms with 24 warps per SM
-// at 80 registers, 59.5 ms with 20 at 96, 65.2 ms with 16 at 128 (with the
-// autotuned shape 52.4 now, 61.9 before pairs of records).
+// register file's ports, not by the number of warps: 96 profiles of the batching prior took 64.4 ms with 24 warps per
+// SM at 80 registers, 59.5 ms with 20 at 96, 65.2 ms with 16 at 128 (with the autotuned shape 52.4, 61.9 before pairs
+// of records).
 constexpr int kCellThreads = 320;
 constexpr int kCellSmallThreads = 192;  // three CTAs per SM of these where tiles are small (Engine::small_tiles)
 constexpr int kBbRecThreads = 768;  // integrand_bb_rec_kernel: 24 warps per SM at 80 registers

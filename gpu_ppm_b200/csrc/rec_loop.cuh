@@ -81,7 +81,8 @@ __device__ __forceinline__ void rec_loop(const KernelArgs& a, unsigned char* sm,
 
   // leader of a set: leaves slot sl; true if the set has become the loader of the drained slot
   auto leave = [&](int sl) {
-    return atomicSub(&s_word[sl], 1u) == (kSlotDrain | 1u) && atomicCAS(&s_word[sl], kSlotDrain, kSlotLoading) == kSlotDrain;
+    return atomicSub(&s_word[sl], 1u) == (kSlotDrain | 1u) &&
+           atomicCAS(&s_word[sl], kSlotDrain, kSlotLoading) == kSlotDrain;
   };
   constexpr int kExit = -1;  // s_got: a slot to work in, kExit, or -2 - slot to load
   int cur_rec = -1, cur_slot = -1, profile = -1, pref = w.set % NS;
@@ -142,7 +143,8 @@ __device__ __forceinline__ void rec_loop(const KernelArgs& a, unsigned char* sm,
         // chunks that nobody has yet, in order
         if (w.st == 0) {
           s_best[w.set] = 0;
-          const int nx = NS * (int)gridDim.x < n_recs ? NS * (int)gridDim.x + atomicAdd(&W.ctr[W.rec_cap].x, 1) : n_recs;
+          const int first = NS * (int)gridDim.x;  // chunks that are the slots' first ones
+          const int nx = first < n_recs ? first + atomicAdd(&W.ctr[W.rec_cap].x, 1) : n_recs;
           s_rec[w.set] = nx < n_recs ? nx : -1;
           if (nx < n_recs) atomicAdd(&W.ctr[nx].y, 1);
         }
@@ -186,7 +188,8 @@ __device__ __forceinline__ void rec_loop(const KernelArgs& a, unsigned char* sm,
       const int n16 = (W.off_slice + W.slice_bytes) >> 4;
       for (int k = w.st; k < n16; k += w.ST) cp_async16(dst + 16 * k, img + 16 * k);
       const int l16 = (q.n_act * W.elem_bytes + 15) >> 4;
-      for (int k = w.st; k < l16; k += w.ST) cp_async16(dst + 16 * (n16 + k), W.lists + (size_t)q.list * W.elem_bytes + 16 * k);
+      const unsigned char* const list = W.lists + (size_t)q.list * W.elem_bytes;
+      for (int k = w.st; k < l16; k += w.ST) cp_async16(dst + 16 * (n16 + k), list + 16 * k);
       if (w.st == 0) {
         const DevProfile& p = a.profiles[q.profile];
         ChunkCtx& c = s_ctx[sl];
@@ -219,8 +222,8 @@ __device__ __forceinline__ void rec_loop(const KernelArgs& a, unsigned char* sm,
     }
     const unsigned char* const base = sm + (size_t)got * S.rec_slot_bytes;
     const double* P = (const double*)base;
-    const ChunkBufs bufs{(const unsigned short*)(base + W.off_slice + W.slice_bytes), P, P + a16, P + 2 * a16, P + 3 * a16,
-                         (const unsigned short*)(base + W.off_hidx),
+    const ChunkBufs bufs{(const unsigned short*)(base + W.off_slice + W.slice_bytes),
+                         P, P + a16, P + 2 * a16, P + 3 * a16, (const unsigned short*)(base + W.off_hidx),
                          (const float*)(base + W.off_slice) + slice_row0(S.ldS, S.cpl)};
     w.nodes(c, bufs, s_u[w.set]);
     __threadfence_block();

@@ -55,8 +55,9 @@ constexpr size_t kStageBytes = size_t(32) << 20;
 // slot, allocated when the server starts (all of them at most an eighth of the
 // memory budget beside it) and used by the slot's batches one after the other.
 // Taken from the stream-ordered pool, the first batches grew it on the scheduler
-// thread while requests waited, up to 525 ms at once under overload (at most 0.7
-// now); 24 mixed requests take 24.9 ms, 31.7 from tiles.
+// thread while requests waited, up to 525 ms at once under overload.  24 mixed
+// requests up to N_side 512 take 24.9 ms with records, 25.3 from tiles; where each
+// batch is one request, that request gains what a single profile does.
 constexpr size_t kServeRingBytes = size_t(256) << 20;
 constexpr size_t kStageFixed = 64 + 256;  // control words and slack around the per-request arrays
 // a full batch's uploads (profiles, fold jobs, control words), each rounded up to 256 bytes
