@@ -90,6 +90,13 @@ void BlockCache::trim() {
 void* DeviceArena::alloc(size_t bytes) {
   void* p = nullptr;
   size_t sz = std::max<size_t>(bytes, 16);
+  const size_t in_area = (sz + 255) / 256 * 256;
+  if (area && in_area <= area_bytes - area_used) {
+    p = area + area_used;
+    area_used += in_area;
+    bytes_held += bytes;
+    return p;
+  }
   if (cache && !stream) {
     // 64 KiB granules, so that blocks of batches of similar size fit one another
     sz = (sz + 65535) / 65536 * 65536;

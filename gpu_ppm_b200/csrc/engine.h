@@ -124,6 +124,9 @@ struct DeviceArena {
   size_t bytes_held = 0;
   cudaStream_t stream = nullptr;  // set: stream-ordered allocations (no implicit device synchronisation)
   BlockCache* cache = nullptr;    // set (synchronous batches): blocks come from and return to the cache
+  // memory of the owner's to take from first (serving: the stream slot's, whose batches follow one another on its stream)
+  unsigned char* area = nullptr;
+  size_t area_bytes = 0, area_used = 0;
   void* alloc(size_t bytes);
   DeviceArena() = default;
   DeviceArena(const DeviceArena&) = delete;

@@ -51,14 +51,16 @@ HostBuffer take(HostBuffer& b) {
 // hundred MB) ever runs while requests wait; admission caps a batch by the
 // bytes it stages, and only a single request larger than a buffer gets its own.
 constexpr size_t kStageBytes = size_t(32) << 20;
-// Device memory of a served batch's ring records and node sums: an area per stream
-// slot, allocated when the server starts (all of them at most an eighth of the
-// memory budget beside it) and used by the slot's batches one after the other.
-// Taken from the stream-ordered pool, the first batches grew it on the scheduler
-// thread while requests waited, up to 525 ms at once under overload.  24 mixed
-// requests up to N_side 512 take 24.9 ms with records, 25.3 from tiles; where each
-// batch is one request, that request gains what a single profile does.
-constexpr size_t kServeRingBytes = size_t(256) << 20;
+// Device memory of a served batch: areas per stream slot for its ring records and
+// node sums, and for its outputs, queue and parameters, allocated when the server
+// starts (the record areas at most an eighth of the memory budget beside it, the
+// others a sixteenth) and used by the slot's batches one after the other; what does
+// not fit comes from the stream-ordered pool.  Taken from the pool, records grew it
+// on the scheduler thread while requests waited, up to 525 ms at once under
+// overload, and outputs alone still did for 40 to 116 ms, once in most runs.  24
+// mixed requests up to N_side 512 take 24.9 ms with records, 25.3 from tiles; where
+// each batch is one request, that request gains what a single profile does.
+constexpr size_t kServeRingBytes = size_t(256) << 20, kServeStateBytes = size_t(128) << 20;
 constexpr size_t kStageFixed = 64 + 256;  // control words and slack around the per-request arrays
 // a full batch's uploads (profiles, fold jobs, control words), each rounded up to 256 bytes
 constexpr size_t kUploadBytes = kMaxRequestsPerBatch * (sizeof(DevProfile) + sizeof(FoldJob)) + 4 * 256;
@@ -86,7 +88,7 @@ struct Server {
   struct Slot {
     cudaStream_t stream = nullptr;
     bool busy = false;
-    DeviceBuffer rings;  // memory of the batch's ring records (see kServeRingBytes)
+    DeviceBuffer rings, state;  // memory of the batch's ring records and of the rest (see kServeRingBytes)
     HostBuffer upload;  // pinned source of the batch build's uploads; reused once the slot's batch has finished
   };
   struct InFlight {
@@ -142,11 +144,13 @@ struct Server {
       stage_pool.resize(slots.size() + kMaxCompleting);
       for (auto& b : stage_pool) b.reserve(kStageBytes);
       for (auto& s : slots) s.upload.reserve(kUploadBytes);
-      const size_t area = std::min(kServeRingBytes, budget / (8 * slots.size())) / 256 * 256;
+      const size_t rings = std::min(kServeRingBytes, budget / (8 * slots.size())) / 256 * 256;
+      const size_t state = std::min(kServeStateBytes, budget / (16 * slots.size())) / 256 * 256;
       for (auto& s : slots) {
         try {
-          if (area) s.rings.reserve(area);
-        } catch (const Error&) {  // no room: its batches run from tiles
+          if (state) s.state.reserve(state);
+          if (rings) s.rings.reserve(rings);
+        } catch (const Error&) {  // no room: its batches run from the pool and from tiles
           cudaGetLastError();
         }
       }
@@ -156,6 +160,7 @@ struct Server {
         if (s.stream) cudaStreamDestroy(s.stream);
         s.upload.release();
         s.rings.release();
+        s.state.release();
       }
       throw;
     }
@@ -189,6 +194,7 @@ struct Server {
       }
       s.upload.release();
       s.rings.release();
+      s.state.release();
     }
     for (auto& b : stage_pool) b.release();
   }
@@ -372,6 +378,8 @@ struct Server {
     f.B.reset(new BatchImpl());
     BatchImpl& B = *f.B;
     B.mem.stream = slot.stream;
+    B.mem.area = (unsigned char*)slot.state.ptr;
+    B.mem.area_bytes = slot.state.cap;
     B.ring_area = (unsigned char*)slot.rings.ptr;
     B.ring_limit = std::max<size_t>(1, slot.rings.ptr ? slot.rings.cap / 256 * 256 : 0);
     B.h_upload = slot.upload.ptr;

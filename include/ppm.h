@@ -174,8 +174,10 @@ typedef struct ppm_engine_config {
                                  while the next is staged); the server also pins n_streams + 4 staging
                                  buffers of 32 MiB and, per stream, a small upload area for the batch
                                  build's host-to-device copies when it starts (first ppm_submit), and takes
-                                 256 MiB of device memory per stream for ring records, beside the budget
-                                 (all of them at most an eighth of it) */
+                                 384 MiB of device memory per stream for its batches, beside the budget (256
+                                 for ring records, all of them at most an eighth of it, and 128 for outputs
+                                 and queues, at most a sixteenth); a batch that needs more takes the rest
+                                 from the device's stream-ordered pool */
 } ppm_engine_config;
 
 /* ---- engine ---------------------------------------------------------------- */
