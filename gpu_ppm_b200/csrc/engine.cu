@@ -1262,9 +1262,10 @@ size_t Engine::ring_work(const IntegrandShape& shape, const DevProfile* hp, cons
 //  * Light curves (at most four energies): the tiles' phase-major walk evaluates a point in fewer instructions.  It
 //    loses between one round of its CTAs and four rings an SM where a ring's segments add to few nodes' sums: one
 //    energy, 213 to 492 rings of 78 to 188 elements, 32 nodes 128..260 -> 66..130 us, 64 nodes 134..276 -> 83..176,
-//    but 96 nodes 101..199 -> 94..225 and 128 nodes 90..188 -> 107..272; four energies, 96 nodes 249..486 ->
-//    130..389, 128 nodes 233 -> 151 but 426 -> 469.  With 16 elements a ring only several energies gain (one: 54 ->
-//    69).
+//    96 nodes 101..130 -> 94..121 up to 306 rings but 194..199 -> 205..225 from 467, 128 nodes 90..188 -> 107..272;
+//    four energies, 96 nodes 249..486 -> 130..389, 128 nodes 233..284 -> 151..230 up to 306 rings but 409..426 ->
+//    417..469.  With 16 elements a ring only several energies gain (one: 54 -> 69; four: 153 -> 107), with 5 none
+//    (four energies, 64 nodes, 237 rings: 61 -> 92).
 //  * Up to 64 energies a tile pays each energy with a reduction over the warp, a record with a lane: records win with
 //    the values (elements x energies) of a ring, however many rings there are: 192 values and 8 energies or more
 //    458 -> 229 us (32 energies, 546 rings) or 3052 -> 2472 (8 energies, 17298 rings); fewer values 1136 -> 875 (320)
@@ -1279,9 +1280,11 @@ bool Engine::bb_records(const GroupWork& w, int n_profiles, int bins_max) const 
   const int ne = w.ne_max;
   const double rings = (double)w.rings, per_ring = w.elements / std::max(1.0, rings), values = per_ring * ne;
   const double sum_blocks = (double)n_profiles * bins_max * ((ne + 31) / 32);
-  if (ne <= 4)
-    return rings > 1.35 * sm_count && rings < 4.0 * sm_count && w.nodes_max <= (ne == 1 ? 64 : 96) &&
-           (per_ring >= 32 || ne >= 3);
+  if (ne <= 4) {
+    const int most_nodes = (ne == 1 ? 64 : 96) + (rings <= 2.5 * sm_count ? 32 : 0);
+    return rings > 1.35 * sm_count && rings < 4.0 * sm_count && w.nodes_max <= most_nodes &&
+           per_ring >= (ne >= 3 ? 14 : 32);
+  }
   if (ne <= 64)
     return (values >= 192 && ne >= 8) ||
            (rings <= 1.5 * sm_count && sum_blocks <= 5.0 * sm_count && (ne >= 12 || values >= 150));
